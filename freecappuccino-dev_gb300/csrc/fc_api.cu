@@ -386,10 +386,11 @@ int solve_global(fc_ctx* ctx, const char* solver, double* x, const double* b, do
 }
 
 // Ordered sweep structure of the mesh system (which = 0) or of the cached
-// external pattern (which = 1): out[0..9] = tiles, levels, widest step of a
-// tile, ring depth, estimated forward sweep microseconds, ring-served
-// entries, pushed entries, cross-tile entries (both triangles), stage depth,
-// most steps of a tile.
+// external pattern (which = 1): out[0..10] = tiles, levels, most rows of a
+// tile in one level, ring depth, estimated forward sweep microseconds,
+// ring-served entries, pushed entries, cross-tile entries (both triangles),
+// steps staged ahead, most steps of a tile, most rows of a step where levels
+// are split into steps (else 0).
 extern "C" int fc_set_sweep_cap(fc_ctx* ctx, int rows) {
   if (!ctx || rows < 0) return FC_ERR_BAD_INPUT;
   ctx->sweep_cap = rows;
@@ -414,10 +415,10 @@ extern "C" int fc_sweep_stats(fc_ctx* ctx, int which, double* out) {
   CsrSystem* s = which ? ctx->sys_ext : ctx->sys_mesh;
   if (!s) return fc_fail_msg(ctx, FC_ERR_STATE, "no such system");
   const DevOrdered& D = s->ord;
-  out[0] = D.ntiles; out[1] = D.nlev; out[2] = D.maxW; out[3] = D.R;
+  out[0] = D.ntiles; out[1] = D.nlev; out[2] = D.max_level_rows; out[3] = D.R;
   out[4] = s->est_sweep_us; out[5] = (double)D.ring_entries; out[6] = (double)D.pushed_entries;
   out[7] = (double)D.cross_tile_entries; out[8] = D.K; out[9] = D.max_tile_steps;
-  out[10] = D.Wc;
+  out[10] = D.max_level_rows > D.maxW ? D.maxW : 0;
   return FC_OK;
 }
 

@@ -99,23 +99,31 @@ enum { FC_OUT_RES0 = 0, FC_OUT_RESL, FC_OUT_FACTOR, FC_OUT_RESOR, FC_OUT_ITR, FC
 
 // device copy of a schedule-ordered sweep structure (fc_schedule.hpp)
 struct DevOrdered {
-  int n = 0, nE = 0, ntiles = 0, nsteps = 0, nlev = 0, R = 4, K = 1, maxW = 0, max_tile_steps = 0;
+  int n = 0, nE = 0, ntiles = 0, nsteps = 0, nlev = 0, R = 4, K = 1, maxW = 0, max_tile_steps = 0, nc = 3, gen = 0;
   size_t stage_area = 0;             // shared memory of the sweeps' stage buffers; K: buffers of an application
-  int xmax = 4, pmax = 4;            // largest exchange / push block of a step
-  bool gs_ok = false;                // the Gauss-Seidel mode gets two stage buffers
-  int Wc = 0;                        // staged rows of a step (0: whole steps are staged)
+  // stage buffers of the applications (0) and of Gauss-Seidel (1, G = 0: it
+  // cannot run on this structure): steps of a buffer, its most rows, padded
+  // rows, push targets and exchanged values, the steps' descriptors
+  struct Groups {
+    int G = 0, rows = 0, padded = 0, push = 0, x = 0;
+    DVec<int> desc[2];
+  } grp[2];
+  int max_level_rows = 0;            // rows of a tile in its widest level
+  int rp_total = 0;                  // rows of all steps, each step padded to a multiple of 4
   int novf[2] = {0, 0}, nxv[2] = {0, 0};
-  DVec<int> tile_step_ptr, step_ptr, tile_W, perm;
-  DVec<int> srec[2], xv_ptr[2], push_ptr[2], push[2], slot[2], ucol;
+  DVec<int> tile_step_ptr, step_ptr, rp_ptr, tile_W, perm;
+  DVec<int> rec[2], xv_ptr[2], push_ptr[2], push[2];
   DVec<int> ovf_ptr[2], ovf_code[2], ovf_col[2], ovf_slot[2];
-  DVec<int> lo_tslot, lo_ovf_tslot, dslot, p_ptr, p_col, p_slot;
+  DVec<int> lo_tslot, lo_ovf_tslot, p_ptr, p_col, p_slot;
   long long ring_entries = 0, pushed_entries = 0, cross_tile_entries = 0;
 };
 
 // per-solve values of an ordered system in one precision (fc_sweep.cuh OrdVals)
 template <class T>
 struct OrdStore {
-  DVec<T> vrec0, vrec1, sx, aovf0, aovf1, tovf, adiag, ap, xv0, xv1, xo, bo;
+  DVec<unsigned char> blob0, blob1;
+  DVec<T> sx, tx, aovf0, aovf1, tovf, adiag, ap, xv0, xv1, xo, bo;
+  bool records = false;  // the blocks hold this structure's row records and push targets
 };
 
 struct LevelSchedule {
@@ -231,7 +239,7 @@ struct fc_ctx {
   int tracing = 0, trace_blocks = 0, trace_cap = 0;
   int sweep_cap = 0;   // rows per sweep step cap of the next pattern analyses (0: as wide as fits)
   int sweep_tiles = 0; // tile count of the next pattern analyses (0: the estimate's choice)
-  int stage_rows = 0;  // staged rows of a step in the next pattern analyses (0: as many as fit; tests)
+  int stage_rows = 0;  // rows of a step in the next pattern analyses (0: a set of compute warps' rows; tests)
   std::FILE* solve_log = nullptr;  // JSON line per solve (fc_set_solve_log)
   int grad_limiter = 0;            // FC_LIMITER_* applied by every gradient (fc_set_gradient_limiter)
   DVec<double> limiter_part;       // min/max partials of the limiters

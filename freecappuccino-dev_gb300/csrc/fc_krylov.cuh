@@ -14,8 +14,9 @@
 #include "fc_internal.hpp"
 
 #define FC_BLOCK 512
-// block of the kernels with ordered sweeps: 15 compute warps + 1 staging warp
-#define FC_SWEEP_BLOCK 512
+// block of the kernels with ordered sweeps: 16 compute, 3 import and 1 staging
+// warp (fc_sweep.cuh)
+#define FC_SWEEP_BLOCK 640
 #define FC_SPIN_LIMIT (1u << 24)
 
 namespace fcdev {
@@ -88,7 +89,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 // the previous reduction never sees slots of the next one being rewritten.
 template <int NV>
 __device__ __forceinline__ bool grid_reduce(const GridCtl& C, int& ph, double (&v)[NV]) {
-  __shared__ double sm[NV][FC_BLOCK / 32];
+  __shared__ double sm[NV][32];
   __shared__ double tot[NV];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int nb = vg_nb(C), bid = vg_bid(C);

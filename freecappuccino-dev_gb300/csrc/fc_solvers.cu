@@ -3,9 +3,9 @@
 // persistent kernel: the residual, the preconditioner setup, the Krylov loop
 // and its stopping test all run on the device, so the host never waits inside
 // an iteration.  Sequential recurrences of the reference (DIC/DILU setup,
-// triangular sweeps, Gauss-Seidel) run as level-scheduled sweeps with a grid
-// barrier per level and exact (non-contracted) FP64 arithmetic, so the
-// preconditioner is the reference's bit for bit.  Dots and norms use a
+// triangular sweeps, Gauss-Seidel) run as tiled sweeps over the levels
+// (fc_sweep.cuh); the factors and Gauss-Seidel in exact (non-contracted)
+// arithmetic, so that the preconditioner is the reference's bit for bit.  Dots and norms use a
 // deterministic tree and are accumulated in FP64 for every precision.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -94,16 +94,20 @@ struct Tracer {
     return out + (size_t)gridDim.x * FC_TRACE_N +
            (((size_t)(nsweep - 1) * gridDim.x + blockIdx.x) * tl_cap + k) * FC_TRACE_STAMPS;
   }
-  // stamp idx of step k, taken once dep is available (thread 0)
+  // the first thread of a set of compute warps, while stamps are kept
+  __device__ __forceinline__ bool stamps(int k) const {
+    return threadIdx.x % FC_SET_ROWS == 0 && threadIdx.x < FC_SETS * FC_SET_ROWS && nsweep <= 2 && k < tl_cap;
+  }
+  // stamp idx of step k, taken once dep is available
   template <class V>
   __device__ __forceinline__ void at(int k, int idx, V dep) {
-    if (threadIdx.x != 0 || nsweep > 2 || k >= tl_cap) return;
+    if (!stamps(k)) return;
     unsigned long long c;
     asm volatile("mov.u64 %0, %%clock64;" : "=l"(c) : "l"((unsigned long long)(long long)dep) : "memory");
     slot(k)[idx] = c;
   }
   __device__ __forceinline__ void step(int k) {
-    if (threadIdx.x != 0 || nsweep > 2 || k >= tl_cap) return;
+    if (!stamps(k)) return;
     unsigned long long gt;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(gt));
     unsigned long long* q = slot(k);
@@ -111,7 +115,7 @@ struct Tracer {
     q[3] = gt;
   }
   __device__ __forceinline__ void waited(int k) {
-    if (threadIdx.x != 0 || nsweep > 2 || k >= tl_cap) return;
+    if (!stamps(k)) return;
     slot(k)[1] = (unsigned long long)clock64();
   }
   // called by the staging thread only
@@ -159,11 +163,13 @@ __device__ bool residual_l1(const KArgs<T>& A, int& ph, double& l1out) {
   return true;
 }
 
-// First phase of the ordered kernels: matrix values into the new numbering,
-// exchange arrays to the sentinel, b (and x) gathered; ends with a barrier.
+// First phase of the ordered kernels: matrix values into the new numbering
+// (kept from the previous solve with skip_setup), exchange arrays to the
+// sentinel, b (and x) gathered; ends with a barrier.
 template <class T>
-__device__ bool ord_prologue(const KArgs<T>& A, bool dilu, bool with_x) {
-  ord_gather_values(A.C, A.O, A.V, A.S.a, A.nnz, dilu);
+__device__ bool ord_prologue(const KArgs<T>& A, bool dilu, bool with_x, bool gs = false) {
+  if (!A.skip_setup) ord_gather_values(A.C, A.O, A.V, A.S.a, A.nnz, dilu, gs);
+  ord_reset_exchange(A.C, A.O, A.V);
   ord_gather_vec(A.C, A.O, A.b, A.bo);
   if (with_x) ord_gather_vec(A.C, A.O, (const T*)A.x, A.xo);
   return grid_sync(A.C);
@@ -184,40 +190,43 @@ __device__ bool ord_residual_l1(const KArgs<T>& A, int& ph, double& l1out) {
   return true;
 }
 
-// z = M^-1 q with the DIC/DILU factors d: forward sweep into yf, barrier,
-// backward sweep into z (linear_solvers.f90:458-475); dot (optional) gets
-// sum e_i z_i of the rows this thread finished.  No barrier at the end.
-template <class T, bool WIDE, class TracerT>
+// z = M^-1 q with the DIC/DILU factors d: forward sweep into yf, backward
+// sweep into z (linear_solvers.f90:458-475); dot (optional) gets sum e_i z_i
+// of the rows this thread finished.  No barrier at the end, and none between
+// the sweeps: a tile turns round as soon as its own rows are done (the last
+// tile of the forward wavefront is the first of the backward one).
+template <class T, class TracerT>
 __device__ __forceinline__ bool precond_apply(const KArgs<T>& A, OsCtx& X, const T* q, T* yf, T* z, const T* e, double* dot,
                               TracerT* tr) {
   const OsIO<T> f{q, nullptr, yf};
-  if (!osweep<T, OS_FWD, WIDE>(A.C, A.O, A.V, f, X, nullptr, tr)) return false;
+  if (!osweep<T, OS_FWD>(A.C, A.O, A.V, f, X, nullptr, tr)) return false;
   tr->mark(TR_FWD);
-  if (!grid_sync(A.C)) return false;
-  tr->mark(TR_MID);
   const OsIO<T> g{yf, e, z};
   if (dot) {
-    if (!osweep<T, OS_BWD_DOT, WIDE>(A.C, A.O, A.V, g, X, dot, tr)) return false;
+    if (!osweep<T, OS_BWD_DOT>(A.C, A.O, A.V, g, X, dot, tr)) return false;
   } else {
-    if (!osweep<T, OS_BWD, WIDE>(A.C, A.O, A.V, g, X, nullptr, tr)) return false;
+    if (!osweep<T, OS_BWD>(A.C, A.O, A.V, g, X, nullptr, tr)) return false;
   }
   tr->mark(TR_BWD);
   return true;
 }
 
 // DIC (DILU) factors d_i, inverted as in the reference
-// (linear_solvers.f90:439-445, :613-624); ends with a barrier
-template <class T, bool DILU, bool WIDE>
+// (linear_solvers.f90:439-445, :613-624), and the applications' row values;
+// ends with a barrier
+template <class T, bool DILU>
 __device__ __forceinline__ bool precond_setup(const KArgs<T>& A, OsCtx& X) {
   const OsIO<T> io{nullptr, nullptr, A.d};
-  if (!osweep<T, DILU ? OS_SETUP_DILU : OS_SETUP_DIC, WIDE>(A.C, A.O, A.V, io, X, nullptr)) return false;
+  if (!osweep<T, DILU ? OS_SETUP_DILU : OS_SETUP_DIC>(A.C, A.O, A.V, io, X, nullptr)) return false;
+  if (!grid_sync(A.C)) return false;
+  ord_apply_values(A.C, A.O, A.V, (const T*)A.d);
   return grid_sync(A.C);
 }
 
 // ------------------------------------------------------------------ ICCG
 // iccg, linear_solvers.f90:364-545, in the schedule-ordered numbering
-template <class T, bool TRACE = false, bool WIDE = false>
-__global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_iccg(KArgs<T> A) {
+template <class T, bool TRACE = false>
+__global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_iccg(const __grid_constant__ KArgs<T> A) {
   const int gt = vg_gt(A.C), G = vg_G(A.C), n = A.O.n;
   int ph = 0;
   OsCtx X = osweep_ctx<T>(A.O, fc_smem, vg_bid(A.C));
@@ -229,13 +238,13 @@ __global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_iccg(KArgs<T> A) {
   if (!ord_residual_l1(A, ph, res0)) return;
   if (res0 < A.tol_abs) { write_out(A, res0, res0, 0.0, 0.0, 0, 1); return; }
   if (!A.skip_setup)
-    if (!precond_setup<T, false, WIDE>(A, X)) return;
+    if (!precond_setup<T, false>(A, X)) return;
   tr.mark(TR_SETUP);
   double s0 = FC_S0, resl = 0.0, factor = 0.0, resor = 0.0;
   int itr_used = 0;
   for (int l = 1; l <= A.itr_max; ++l) {
     double rz[1] = {0.0};
-    if (!precond_apply<T, WIDE>(A, X, (const T*)r, yf, z, (const T*)r, rz, &tr)) return;
+    if (!precond_apply<T>(A, X, (const T*)r, yf, z, (const T*)r, rz, &tr)) return;
     if (!grid_reduce<1>(A.C, ph, rz)) return;
     tr.mark(TR_DOT);
     const double sk = rz[0];
@@ -280,7 +289,7 @@ __global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_iccg(KArgs<T> A) {
 // bicgstab, linear_solvers.f90:548-786, in the schedule-ordered numbering.
 // Runs on the blocks A.C names (the launch grid, or one problem's group of a
 // batched launch).
-template <class T, bool WIDE>
+template <class T>
 __device__ __forceinline__ void bicgstab_body(const KArgs<T>& A) {
   const int gt = vg_gt(A.C), G = vg_G(A.C), n = A.O.n;
   int ph = 0;
@@ -292,7 +301,7 @@ __device__ __forceinline__ void bicgstab_body(const KArgs<T>& A) {
   if (!ord_residual_l1(A, ph, res0)) return;
   if (res0 < A.tol_abs) { write_out(A, res0, res0, 0.0, 0.0, 0, 1); return; }
   if (!A.skip_setup)
-    if (!precond_setup<T, true, WIDE>(A, X)) return;
+    if (!precond_setup<T, true>(A, X)) return;
   double bb[1] = {0.0};
   for (int i = gt; i < n; i += G) {
     T ri = ldcg(r + i);
@@ -312,7 +321,7 @@ __device__ __forceinline__ void bicgstab_body(const KArgs<T>& A) {
     const T omT = (T)om, alfT = (T)alf;
     for (int i = gt; i < n; i += G) p[i] = ldcg(r + i) + omT * (ldcg(p + i) - alfT * ldcg(u + i));
     if (!grid_sync(A.C)) return;
-    if (!precond_apply<T, WIDE>(A, X, (const T*)p, yf, z, (const T*)nullptr, nullptr, &tr)) return;
+    if (!precond_apply<T>(A, X, (const T*)p, yf, z, (const T*)nullptr, nullptr, &tr)) return;
     if (!grid_sync(A.C)) return;
     double ur[1] = {0.0};
     for (int i = gt; i < n; i += G) {
@@ -328,7 +337,7 @@ __device__ __forceinline__ void bicgstab_body(const KArgs<T>& A) {
       r[i] = ldcg(r + i) - gamT * ldcg(u + i);
     }
     if (!grid_sync(A.C)) return;
-    if (!precond_apply<T, WIDE>(A, X, (const T*)r, yf, z, (const T*)nullptr, nullptr, &tr)) return;
+    if (!precond_apply<T>(A, X, (const T*)r, yf, z, (const T*)nullptr, nullptr, &tr)) return;
     if (!grid_sync(A.C)) return;
     double vr[2] = {0.0, 0.0};
     for (int i = gt; i < n; i += G) {
@@ -367,9 +376,9 @@ __device__ __forceinline__ void bicgstab_body(const KArgs<T>& A) {
   write_out(A, res0, resl, factor, resor, itr_used, 0);
 }
 
-template <class T, bool WIDE = false>
-__global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_bicgstab(KArgs<T> A) {
-  bicgstab_body<T, WIDE>(A);
+template <class T>
+__global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_bicgstab(const __grid_constant__ KArgs<T> A) {
+  bicgstab_body<T>(A);
 }
 
 // ------------------------------------------------------------------ DPCG
@@ -432,12 +441,11 @@ __global__ void __launch_bounds__(FC_BLOCK, 1) k_dpcg(KArgs<T> A) {
 // GaussSeidel, linear_solvers.f90:96-201: the in-place sweep as an ordered
 // forward sweep; entries left of the diagonal take this sweep's values
 // (xb), the diagonal and the entries right of it the previous sweep's (xa).
-template <bool WIDE = false>
-__global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_gauss_seidel(KArgs<double> A) {
+__global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_gauss_seidel(const __grid_constant__ KArgs<double> A) {
   const int gt = vg_gt(A.C);
   int ph = 0;
   OsCtx X = osweep_ctx<double>(A.O, fc_smem, vg_bid(A.C));
-  if (!ord_prologue(A, false, true)) return;
+  if (!ord_prologue(A, false, true, true)) return;
   double* xa = A.xo;
   double* xb = A.w;
   double res0 = 0.0, resl = 0.0, factor = 0.0, resor = 0.0;
@@ -445,7 +453,7 @@ __global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_gauss_seidel(KArgs<double
   for (int l = 1; l <= A.itr_max; ++l) {
     double red[2] = {0.0, 0.0};
     const OsIO<double> io{A.bo, xa, xb};
-    if (!osweep<double, OS_GS, WIDE>(A.C, A.O, A.V, io, X, red)) return;
+    if (!osweep<double, OS_GS>(A.C, A.O, A.V, io, X, red)) return;
     if (!grid_reduce<2>(A.C, ph, red)) return;
     double* t = xa; xa = xb; xb = t;
     if (l == 1) {
@@ -465,15 +473,15 @@ __global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_gauss_seidel(KArgs<double
 
 // preconditioner only: d (DIC or DILU) and optionally z = M^-1 q, q = A.b;
 // results in the original numbering: d into A.v, z into A.z
-template <class T, bool DILU, bool WIDE = false>
-__global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_precond(KArgs<T> A, int apply) {
+template <class T, bool DILU>
+__global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_precond(const __grid_constant__ KArgs<T> A, int apply) {
   OsCtx X = osweep_ctx<T>(A.O, fc_smem, vg_bid(A.C));
   NoTracer tr(nullptr, 0);
   if (!ord_prologue(A, DILU, false)) return;
-  if (!precond_setup<T, DILU, WIDE>(A, X)) return;
+  if (!precond_setup<T, DILU>(A, X)) return;
   ord_scatter_vec(A.C, A.O, (const T*)A.d, A.v);
   if (!apply) return;
-  if (!precond_apply<T, WIDE>(A, X, (const T*)A.bo, A.u, A.w, (const T*)nullptr, nullptr, &tr)) return;
+  if (!precond_apply<T>(A, X, (const T*)A.bo, A.u, A.w, (const T*)nullptr, nullptr, &tr)) return;
   if (!grid_sync(A.C)) return;
   ord_scatter_vec(A.C, A.O, (const T*)A.w, A.z);
 }
@@ -540,7 +548,7 @@ __device__ __forceinline__ KArgs<T>& batch_args(const KArgs<T>* __restrict__ arg
   return *reinterpret_cast<KArgs<T>*>(raw);
 }
 
-template <class T, bool WIDE = false>
+template <class T>
 __global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1)
     k_bicgstab_batch(const KArgs<T>* __restrict__ args, const int* __restrict__ bprob, const BatchCtl* __restrict__ ctl) {
   __shared__ __align__(16) unsigned char raw[sizeof(KArgs<T>)];
@@ -551,7 +559,7 @@ __global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1)
   __syncthreads();
   if (threadIdx.x == 0) { A.skip_setup = ctl[p].skip_setup; A.itr_max = ctl[p].itr_max; }
   __syncthreads();
-  bicgstab_body<T, WIDE>(A);
+  bicgstab_body<T>(A);
   if (vg_bid(A.C) == 0 && threadIdx.x == 0) A.C.out[FC_OUT_GT] = (double)(globaltimer_ns() - t0);
 }
 
@@ -606,7 +614,7 @@ __global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1)
 #define FC_SWEEP_TAU0_US 0.15
 #define FC_SWEEP_ROW_US 0.001
 #define FC_SWEEP_HOP_US 1.5
-#define FC_RING 4                    // ring depth (steps) of the ordered sweeps
+#define FC_RING 4                    // ring depth (levels) of the ordered sweeps
 // FP32 inner BiCGStab of the mixed modes: iterations without halving the
 // residual after which the inner solve ends (the longest such run in the
 // converging solves of the batched convection-diffusion set is 22)
@@ -667,121 +675,89 @@ static cudaError_t upload_vec(cudaStream_t s, DVec<int>& d, const V& h) {
   return fc_h2d(s, d.p, h.data(), h.size() * sizeof(int));
 }
 
+// A structure's steps in groups of G, one stage buffer each: the
+// descriptors of the steps (OrdView::desc) and the largest group; false if
+// a descriptor's 16-bit fields do not hold it.
+static bool group_steps(const OrderedSweep& O, int G, OrdView& V, std::vector<int>* desc) {
+  V.G = G;
+  V.gen = O.max_entries > FC_ELL || O.maxW > FC_SET_ROWS;
+  V.nc = O.max_entries > 3 ? FC_ELL : 3;
+  V.g_rows = V.g_padded = V.g_push = V.g_x = 0;
+  if (desc)
+    for (int d = 0; d < 2; ++d) desc[d].assign((size_t)4 * O.nsteps, 0);
+  for (int d = 0; d < 2; ++d) {
+    const OrderedDir& H = O.dir[d];
+    for (int t = 0; t < O.ntiles; ++t) {
+      const int s0 = O.tile_step_ptr[t], ns = O.tile_step_ptr[t + 1] - s0;
+      for (int k0 = 0; k0 < ns; k0 += G) {
+        const int k1 = std::min(k0 + G, ns), lo = s0 + (d ? ns - k1 : k0), hi = s0 + (d ? ns - k0 : k1);
+        V.g_rows = std::max(V.g_rows, O.step_ptr[hi] - O.step_ptr[lo]);
+        V.g_padded = std::max(V.g_padded, O.rp_ptr[hi] - O.rp_ptr[lo]);
+        V.g_push = std::max(V.g_push, H.push_ptr[hi] - H.push_ptr[lo]);
+        V.g_x = std::max(V.g_x, H.xv_ptr[hi] - H.xv_ptr[lo]);
+        if (!desc) continue;
+        for (int s = lo; s < hi; ++s) {
+          int* q = desc[d].data() + 4 * (size_t)s;
+          q[0] = O.step_ptr[s];
+          q[1] = (O.step_ptr[s + 1] - O.step_ptr[s]) | ((H.push_ptr[s + 1] - H.push_ptr[s]) << 16);
+          q[2] = (O.rp_ptr[s] - O.rp_ptr[lo]) | ((H.push_ptr[s] - H.push_ptr[lo]) << 16);
+          q[3] = (O.step_ptr[s] - (O.step_ptr[lo] & ~3)) | ((H.xv_ptr[s] - H.xv_ptr[lo]) << 16);
+        }
+      }
+    }
+  }
+  return V.g_rows < 65530 && V.g_padded < 65536 && V.g_push < 65536 && V.g_x < 65536;
+}
+
 // the stage area of the ordered sweeps: the shared memory the fixed parts
 // leave (the sweep modes cut it into as many buffers as fit, at most
 // FC_MAX_STAGES); 0 when nothing is left
-static size_t ordered_stage_area(int R, int maxW, int max_tile_steps) {
-  const size_t fixed = osweep_fixed_bytes<double>(R, maxW, max_tile_steps);
+static size_t ordered_stage_area(int R, int maxW) {
+  const size_t fixed = osweep_fixed_bytes<double>(R, maxW);
   return fixed >= (size_t)FC_SWEEP_SMEM ? 0 : ((size_t)FC_SWEEP_SMEM - fixed) & ~(size_t)15;
 }
 
-// stage buffers of the sweep modes up to last_mode at width maxW (the widest
-// tile); the smallest over the modes is the depth the schedule is checked
-// against.  The Gauss-Seidel mode (OS_GS, the last) stages the most per row.
-static int ordered_min_stages(size_t area, int maxW, int xmax, int pmax, int last_mode = OS_GS) {
-  int kmin = FC_MAX_STAGES;
-  for (int m = OS_SETUP_DIC; m <= last_mode; ++m) {
-    StageLayout L;
-    L.init_for<double>(maxW, xmax, pmax, m);
-    kmin = std::min(kmin, (size_t)L.bytes <= area ? stages_in(area, L.bytes) : 0);
-  }
-  return kmin;
-}
-
-// largest exchange and push blocks of a step (both directions)
-static void ordered_blocks(const OrderedSweep& O, int& xmax, int& pmax) {
-  xmax = pmax = 4;
-  for (int d = 0; d < 2; ++d)
-    for (int gs = 0; gs < O.nsteps; ++gs) {
-      xmax = std::max(xmax, O.dir[d].xv_ptr[gs + 1] - O.dir[d].xv_ptr[gs]);
-      pmax = std::max(pmax, O.dir[d].push_ptr[gs + 1] - O.dir[d].push_ptr[gs]);
+// The most steps of a stage buffer with which every mode (gs: Gauss-Seidel,
+// else the setups and applications) gets the FC_SETS buffers the sweeps need
+// (see fc_sweep.cuh); 0 if none.
+static int steps_per_buffer(const OrderedSweep& O, bool gs) {
+  // Gauss-Seidel steps take one row per thread (their loads include the
+  // upper triangle's values)
+  if (gs && O.maxW > FC_SET_ROWS) return 0;
+  const size_t area = ordered_stage_area(O.R, O.maxW);
+  for (int G = FC_SETS; G >= 1; G /= 2) {
+    OrdView V;
+    bool ok = group_steps(O, G, V, nullptr);
+    for (int m = gs ? OS_GS : OS_SETUP_DIC; m <= (gs ? OS_GS : OS_BWD_DOT); ++m) {
+      const int bytes = StageLayout::of<double>(V, m).bytes;
+      ok = ok && (size_t)bytes <= area && stages_in(area, bytes) >= FC_SETS;
     }
-}
-
-// The staging a structure needs: two stage buffers for every sweep mode the
-// solves use (the factor setups, the applications, Gauss-Seidel when
-// with_gs) and FC_APPLY_STAGES for the applications, which run every
-// iteration: with fewer the staging thread cannot run far enough ahead to
-// hide its copies (measured on 6M tetrahedra: steps of 616 rows with two
-// application stages took 222 ms per SIMPLE iteration, steps of 364 rows
-// with four 179 ms, despite 2,512 levels against 4,088).
-#define FC_APPLY_STAGES 4
-// fewest staged rows of a step for which wide levels are kept whole (below,
-// they are split into narrower steps)
-#define FC_MIN_STAGED_ROWS 64
-static int last_mode_of(bool with_gs) { return with_gs ? OS_GS : OS_BWD_DOT; }
-static bool staging_ok(size_t area, int maxW, int xmax, int pmax, bool with_gs) {
-  if (ordered_min_stages(area, maxW, xmax, pmax, last_mode_of(with_gs)) < 2) return false;
-  for (int m = OS_FWD; m <= OS_BWD_DOT; ++m) {
-    StageLayout L;
-    L.init_for<double>(maxW, xmax, pmax, m);
-    if ((size_t)L.bytes > area || stages_in(area, L.bytes) < FC_APPLY_STAGES) return false;
-  }
-  return true;
-}
-static bool ordered_fits(const OrderedSweep& O, bool with_gs) {
-  int xmax, pmax;
-  ordered_blocks(O, xmax, pmax);
-  return staging_ok(ordered_stage_area(O.R, O.maxW, O.max_tile_steps), O.maxW, xmax, pmax, with_gs);
-}
-
-// The widest step (a multiple of 32 rows, at most maxW) whose staging
-// would be enough with exchange and push blocks of three entries per row, the
-// most a capped step of the meshes measured needed, and the tile step
-// tables grown in proportion to the split; 0 if none.  The first cap tried
-// when a schedule does not fit, instead of halving the width.
-static int estimated_step_cap(int R, int maxW, int max_tile_steps, bool with_gs) {
-  for (int w = maxW & ~31; w >= 32; w -= 32) {
-    const int steps = (int)std::min<long long>(1LL << 24, (long long)max_tile_steps * ((maxW + w - 1) / w));
-    if (staging_ok(ordered_stage_area(R, w, steps), w, 3 * w, 3 * w, with_gs)) return w;
+    if (ok) return G;
   }
   return 0;
 }
 
-// largest push block of the steps of at most w rows (the blocks that are staged)
-static int staged_push_max(const OrderedSweep& O, int w) {
-  int pmax = 4;
-  for (int d = 0; d < 2; ++d)
-    for (int gs = 0; gs < O.nsteps; ++gs)
-      if (O.step_ptr[gs + 1] - O.step_ptr[gs] <= w)
-        pmax = std::max(pmax, O.dir[d].push_ptr[gs + 1] - O.dir[d].push_ptr[gs]);
-  return pmax;
-}
-
-// The rows of a step the stage buffers hold when a wider step reads its
-// further rows, and its push block, from global memory: the largest multiple
-// of 32 (below maxW) whose staging is enough, with the ring at the full
-// width; 0 if none.
-static int staged_rows_fit(const OrderedSweep& O, bool with_gs) {
-  int xmax, pmax;
-  ordered_blocks(O, xmax, pmax);
-  const size_t area = ordered_stage_area(O.R, O.maxW, O.max_tile_steps);
-  for (int w = (O.maxW - 1) & ~31; w >= 32; w -= 32)
-    if (staging_ok(area, w, xmax, staged_push_max(O, w), with_gs)) return w;
-  return 0;
-}
-
-// Wc > 0: a step stages its first Wc rows (fewer than the widest step)
-static int upload_ordered(fc_ctx* ctx, const OrderedSweep& O, DevOrdered& D, bool with_gs, int Wc) {
+static int upload_ordered(fc_ctx* ctx, const OrderedSweep& O, DevOrdered& D) {
   D.n = O.n; D.nE = O.nE; D.ntiles = O.ntiles; D.nsteps = O.nsteps; D.nlev = O.nlev; D.R = O.R; D.maxW = O.maxW;
-  D.max_tile_steps = O.max_tile_steps;
-  ordered_blocks(O, D.xmax, D.pmax);
-  D.Wc = Wc > 0 && Wc < D.maxW ? Wc : 0;
-  const int Ws = D.Wc > 0 ? D.Wc : D.maxW;
-  if (D.Wc > 0) D.pmax = staged_push_max(O, D.Wc);  // the push blocks the stage buffers hold
-  D.stage_area = ordered_stage_area(D.R, D.maxW, D.max_tile_steps);
-  if (ordered_min_stages(D.stage_area, Ws, D.xmax, D.pmax, last_mode_of(with_gs)) < 2)
-    return fc_fail_msg(ctx, FC_ERR_UNSUPPORTED, "sweep tiles too wide for shared memory");
-  D.gs_ok = ordered_min_stages(D.stage_area, Ws, D.xmax, D.pmax, OS_GS) >= 2;
-  {
-    // stages of the preconditioner application (sweep statistics)
-    StageLayout L;
-    L.init_for<double>(Ws, D.xmax, D.pmax, OS_FWD);
-    D.K = stages_in(D.stage_area, L.bytes);
+  D.max_tile_steps = O.max_tile_steps; D.max_level_rows = O.max_level_rows; D.rp_total = O.rp_ptr.back();
+  D.stage_area = ordered_stage_area(D.R, D.maxW);
+  for (int gs = 0; gs < 2; ++gs) {
+    DevOrdered::Groups& P = D.grp[gs];
+    P.G = steps_per_buffer(O, gs != 0);
+    if (P.G == 0) continue;
+    OrdView V;
+    std::vector<int> desc[2];
+    group_steps(O, P.G, V, desc);
+    D.nc = V.nc; D.gen = V.gen;
+    P.rows = V.g_rows; P.padded = V.g_padded; P.push = V.g_push; P.x = V.g_x;
+    for (int d = 0; d < 2; ++d) FC_CUDA_TRY(ctx, upload_vec(ctx->stream, P.desc[d], desc[d]));
+    // steps staged ahead by the preconditioner application (sweep statistics)
+    if (!gs) D.K = stages_in(D.stage_area, StageLayout::of<double>(V, OS_FWD).bytes) * P.G;
   }
   D.ring_entries = D.pushed_entries = D.cross_tile_entries = 0;
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.tile_step_ptr, O.tile_step_ptr));
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.step_ptr, O.step_ptr));
+  FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.rp_ptr, O.rp_ptr));
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.tile_W, O.tile_W));
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.perm, O.perm));
   for (int d = 0; d < 2; ++d) {
@@ -791,24 +767,17 @@ static int upload_ordered(fc_ctx* ctx, const OrderedSweep& O, DevOrdered& D, boo
     D.ring_entries += H.ring_entries;
     D.pushed_entries += H.pushed_entries;
     D.cross_tile_entries += H.cross_tile_entries;
-    FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.srec[d], H.srec));
+    FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.rec[d], H.rec));
     FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.xv_ptr[d], H.xv_ptr));
     FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.push_ptr[d], H.push_ptr));
     FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.push[d], H.push));
-    FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.slot[d], H.slot));
     FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.ovf_ptr[d], H.ovf_ptr));
     FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.ovf_code[d], H.ovf_code));
     FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.ovf_col[d], H.ovf_col));
     FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.ovf_slot[d], H.ovf_slot));
   }
-  // columns of the upper entries, 4 per row (Gauss-Seidel)
-  std::vector<int> ucol((size_t)4 * O.nE, 0);
-  for (int q = 0; q < O.n; ++q)
-    for (int e = 0; e < FC_ELL; ++e) ucol[4 * (size_t)q + e] = O.dir[1].col[(size_t)e * O.nE + q];
-  FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.ucol, ucol));
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.lo_tslot, O.lo_tslot));
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.lo_ovf_tslot, O.lo_ovf_tslot));
-  FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.dslot, O.dslot));
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.p_ptr, O.p_ptr));
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.p_col, O.p_col));
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.p_slot, O.p_slot));
@@ -875,10 +844,6 @@ int sys_set_pattern(fc_ctx* ctx, CsrSystem* s, int n, int nnz, const int* ia1, c
   auto since = [](std::chrono::steady_clock::time_point a) {
     return std::chrono::duration<double>(std::chrono::steady_clock::now() - a).count();
   };
-  // systems whose tiles the caller plans (the batched solves) split wide
-  // levels into steps, as their tile planner assumes; the others keep them
-  // whole with staged rows (below)
-  const bool planned_tiles = tiles_req > 0;
   if (tiles_req <= 0 && ctx->sweep_tiles > 0) tiles_req = ctx->sweep_tiles;
   if (tiles_req > 0) {
     tiles = std::min(tiles_req, sms);
@@ -893,45 +858,26 @@ int sys_set_pattern(fc_ctx* ctx, CsrSystem* s, int n, int nnz, const int* ia1, c
   OrderedSweep O;
   SweepSchedule S;
   std::string err;
-  // the widest step must fit the shared-memory staging of the modes the
-  // solves use (Gauss-Seidel only when with_gs; a Gauss-Seidel solve on a
-  // structure without it analyses the pattern again): if it does not, wide
-  // levels are split into narrower steps (more, shorter steps), first at the
-  // estimated widest cap that fits, then at 7/8 of the previous cap, until
-  // it does
-  int wmax = ctx->sweep_cap > 0 ? ctx->sweep_cap : 0;
-  int wc = 0;  // rows a step stages when its further rows stay in global memory
+  // a level of a tile becomes steps of at most `chunk` rows: a set's compute
+  // threads, or the forced width (tests); fewer where the solves' modes do not
+  // get enough stage buffers
+  int chunk = FC_SET_ROWS;
+  if (ctx->stage_rows > 0 && !(with_gs && ctx->stage_rows > FC_SET_ROWS)) chunk = ctx->stage_rows;
   for (;;) {
-    if (!build_ordered_sweep(n, ia.data(), ja.data(), dg.data(), ts.data(), tiles, xyz, FC_RING, O, S, err, wmax))
+    if (!build_ordered_sweep(n, ia.data(), ja.data(), dg.data(), ts.data(), tiles, xyz, FC_RING, O, S, err,
+                             ctx->sweep_cap, chunk))
       return fc_fail_msg(ctx, FC_ERR_BAD_INPUT, err);
-    if (ctx->stage_rows > 0 && ctx->stage_rows < O.maxW) {
-      // forced (tuning, tests), where every mode the solves use still gets
-      // two stage buffers
-      int xmax, pmax;
-      ordered_blocks(O, xmax, pmax);
-      const int w = ctx->stage_rows;
-      if (ordered_min_stages(ordered_stage_area(O.R, O.maxW, O.max_tile_steps), w, xmax, staged_push_max(O, w),
-                             last_mode_of(with_gs)) >= 2) {
-        wc = w;
-        break;
-      }
-    }
-    if (ordered_fits(O, with_gs)) break;
-    if (wmax == 0 && !planned_tiles) {
-      // wide levels kept whole: the stage buffers hold the first rows of a
-      // step, the others are read from global memory
-      wc = staged_rows_fit(O, with_gs);
-      if (wc >= FC_MIN_STAGED_ROWS) break;
-      wc = 0;
-    }
-    const int est = wmax ? 0 : estimated_step_cap(FC_RING, O.maxW, O.max_tile_steps, with_gs);
-    wmax = est > 0 ? est : (wmax ? (wmax * 7 / 8) & ~7 : std::max(32, O.maxW / 2));
-    if (wmax < 32) return fc_fail_msg(ctx, FC_ERR_UNSUPPORTED, "sweep steps too wide for shared memory");
+    if (steps_per_buffer(O, false) > 0 && (!with_gs || steps_per_buffer(O, true) > 0)) break;
+    if (chunk > FC_SET_ROWS) chunk = std::max(FC_SET_ROWS, (3 * chunk / 4) & ~31);
+    else if (chunk > 32) chunk = 32;
+    else return fc_fail_msg(ctx, FC_ERR_UNSUPPORTED, "sweep tiles too large for shared memory");
   }
   s->t_schedule = since(t0);
   s->xyz_src = xyz;
-  int st2 = upload_ordered(ctx, O, s->ord, with_gs, wc);
+  int st2 = upload_ordered(ctx, O, s->ord);
+
   if (st2) return st2;
+  s->o64.records = s->o32.records = false;
   FC_CUDA_TRY(ctx, s->ia.alloc(n + 1));
   FC_CUDA_TRY(ctx, s->ja.alloc(nnz));
   FC_CUDA_TRY(ctx, s->diag.alloc(n));
@@ -954,13 +900,32 @@ int sys_set_pattern(fc_ctx* ctx, CsrSystem* s, int n, int nnz, const int* ia1, c
   return sys_alloc_work(ctx, s);
 }
 
+// the structure's row records and push targets into the blocks of a store
+template <class T>
+__global__ void k_blob_records(OrdView O, const int* __restrict__ push, int dirn, unsigned char* blob) {
+  const int lane = threadIdx.x & 31, gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  for (int s = gw; s < O.nsteps; s += (gridDim.x * blockDim.x) >> 5) {
+    const int base = O.step_ptr[s], cnt = O.step_ptr[s + 1] - base, cp = (cnt + 3) & ~3;
+    const int pp = O.push_ptr[dirn][s], np = O.push_ptr[dirn][s + 1] - pp;
+    unsigned char* B = blob + blob_offset<T>(O.rp_ptr[s], pp, blob_fields<T>(O.nc, dirn));
+    for (int sl = lane; sl < cnt; sl += 32) ((int4*)B)[sl] = O.rec[dirn][base + sl];
+    for (int m = lane; m < np; m += 32) ((int*)(B + 16 * cp))[m] = push[pp + m];
+  }
+}
+static OrdView ord_view_of(CsrSystem* s, bool gs = false);
+
 template <class T>
 static int alloc_ordered(fc_ctx* ctx, CsrSystem* s, OrdStore<T>& V) {
   const DevOrdered& D = s->ord;
-  const size_t nE = D.nE, rec = (size_t)Rec<T>::V * nE;
-  FC_CUDA_TRY(ctx, V.vrec0.alloc(rec));
-  FC_CUDA_TRY(ctx, V.vrec1.alloc(rec));
-  FC_CUDA_TRY(ctx, V.sx.alloc(rec));
+  const size_t nE = D.nE;
+  DVec<unsigned char>* blob[2] = {&V.blob0, &V.blob1};
+  for (int d = 0; d < 2; ++d) {
+    const size_t bytes = blob_offset<T>(D.rp_total, (int)D.push[d].n, blob_fields<T>(D.nc, d));
+    if (blob[d]->n != bytes) V.records = false;
+    FC_CUDA_TRY(ctx, blob[d]->alloc(bytes));
+  }
+  FC_CUDA_TRY(ctx, V.sx.alloc(D.rp_total));
+  FC_CUDA_TRY(ctx, V.tx.alloc((size_t)D.rp_total * D.nc));
   FC_CUDA_TRY(ctx, V.aovf0.alloc(std::max(1, D.novf[0])));
   FC_CUDA_TRY(ctx, V.aovf1.alloc(std::max(1, D.novf[1])));
   FC_CUDA_TRY(ctx, V.tovf.alloc(std::max(1, D.novf[0])));
@@ -970,10 +935,16 @@ static int alloc_ordered(fc_ctx* ctx, CsrSystem* s, OrdStore<T>& V) {
   FC_CUDA_TRY(ctx, V.ap.alloc(s->nnz));
   FC_CUDA_TRY(ctx, V.xo.alloc(nE));
   FC_CUDA_TRY(ctx, V.bo.alloc(nE));
-  // padding rows of the record arrays are read by the staging and never used
-  FC_CUDA_TRY(ctx, fc_zero(ctx->stream, V.vrec0.p, V.vrec0.bytes()));
-  FC_CUDA_TRY(ctx, fc_zero(ctx->stream, V.vrec1.p, V.vrec1.bytes()));
-  FC_CUDA_TRY(ctx, fc_zero(ctx->stream, V.sx.p, V.sx.bytes()));
+  if (!V.records) {
+    const OrdView O = ord_view_of(s);
+    for (int d = 0; d < 2; ++d) {
+      k_blob_records<T><<<std::max(1, std::min(2048, (D.nsteps + 7) / 8)), 256, 0, ctx->stream>>>(
+          O, D.push[d].p, d, blob[d]->p);
+      ctx->kernel_launches++;
+    }
+    FC_CUDA_TRY(ctx, cudaGetLastError());
+    V.records = true;
+  }
   return FC_OK;
 }
 
@@ -1017,21 +988,22 @@ static CsrView<T> view_of(CsrSystem* s, const T* a) {
   return v;
 }
 
-static OrdView ord_view_of(CsrSystem* s) {
+static OrdView ord_view_of(CsrSystem* s, bool gs) {
   DevOrdered& D = s->ord;
   OrdView O;
-  O.n = D.n; O.nE = D.nE; O.ntiles = D.ntiles; O.R = D.R; O.stage_area = (int)D.stage_area;
+  O.n = D.n; O.nE = D.nE; O.ntiles = D.ntiles; O.R = D.R; O.nc = D.nc; O.gen = D.gen; O.stage_area = (int)D.stage_area;
   O.novf0 = D.novf[0]; O.novf1 = D.novf[1];
-  O.nsteps = D.nsteps; O.maxW = D.maxW; O.xmax = D.xmax; O.pmax = D.pmax; O.Wc = D.Wc;
-  O.tile_step_ptr = D.tile_step_ptr.p; O.step_ptr = D.step_ptr.p; O.tile_W = D.tile_W.p; O.perm = D.perm.p;
+  O.nsteps = D.nsteps;
+  const DevOrdered::Groups& P = D.grp[gs ? 1 : 0];
+  O.G = P.G; O.g_rows = P.rows; O.g_padded = P.padded; O.g_push = P.push; O.g_x = P.x;
+  O.tile_step_ptr = D.tile_step_ptr.p; O.step_ptr = D.step_ptr.p; O.rp_ptr = D.rp_ptr.p; O.tile_W = D.tile_W.p;
+  O.perm = D.perm.p;
   for (int d = 0; d < 2; ++d) {
-    O.srec[d] = (const int4*)D.srec[d].p; O.xv_ptr[d] = D.xv_ptr[d].p; O.push_ptr[d] = D.push_ptr[d].p;
-    O.push[d] = D.push[d].p; O.slot[d] = D.slot[d].p;
+    O.rec[d] = (const int4*)D.rec[d].p; O.desc[d] = (const int4*)P.desc[d].p; O.xv_ptr[d] = D.xv_ptr[d].p; O.push_ptr[d] = D.push_ptr[d].p;
     O.ovf_ptr[d] = D.ovf_ptr[d].p; O.ovf_code[d] = D.ovf_code[d].p; O.ovf_col[d] = D.ovf_col[d].p;
     O.ovf_slot[d] = D.ovf_slot[d].p;
   }
-  O.ucol = (const int4*)D.ucol.p;
-  O.lo_tslot = D.lo_tslot.p; O.lo_ovf_tslot = D.lo_ovf_tslot.p; O.dslot = D.dslot.p;
+  O.lo_tslot = D.lo_tslot.p; O.lo_ovf_tslot = D.lo_ovf_tslot.p;
   O.p_ptr = D.p_ptr.p; O.p_col = D.p_col.p; O.p_slot = D.p_slot.p;
   return O;
 }
@@ -1039,7 +1011,7 @@ static OrdView ord_view_of(CsrSystem* s) {
 template <class T>
 static OrdVals<T> vals_of(OrdStore<T>& S) {
   OrdVals<T> V;
-  V.vrec[0] = S.vrec0.p; V.vrec[1] = S.vrec1.p; V.sx = S.sx.p; V.aovf[0] = S.aovf0.p; V.aovf[1] = S.aovf1.p;
+  V.blob[0] = S.blob0.p; V.blob[1] = S.blob1.p; V.sx = S.sx.p; V.tx = S.tx.p; V.aovf[0] = S.aovf0.p; V.aovf[1] = S.aovf1.p;
   V.tovf = S.tovf.p; V.adiag = S.adiag.p; V.ap = S.ap.p; V.xv[0] = S.xv0.p; V.xv[1] = S.xv1.p;
   return V;
 }
@@ -1050,7 +1022,7 @@ template <class T>
 static int launch_coop(fc_ctx* ctx, CsrSystem* s, const void* fn, KArgs<T>& A, void** extra, int nextra,
                        int block = FC_SWEEP_BLOCK) {
   const DevOrdered& D = s->ord;
-  const size_t smem = osweep_smem_bytes<T>(D.R, D.stage_area, D.maxW, D.max_tile_steps);
+  const size_t smem = osweep_smem_bytes<T>(D.R, D.stage_area, D.maxW);
   if (smem > 48 * 1024)
     FC_CUDA_TRY(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int nb = 0;
@@ -1121,14 +1093,14 @@ static int sys_reanalyse_for_gs(fc_ctx* ctx, CsrSystem* s) {
 
 static int solve_fp64(fc_ctx* ctx, CsrSystem* s, const std::string& solver, const double* a, double* x,
                       const double* b, int itr_max, double tol_abs, double tol_rel, SolveResult* res) {
-  if (solver == "gauss-seidel" && !s->ord.gs_ok) {
+  if (solver == "gauss-seidel" && !(s->ord.grp[1].G > 0)) {
     const int st = sys_reanalyse_for_gs(ctx, s);
     if (st) return st;
   }
   KArgs<double> A = make_args<double>(s, a, x, b, s->r.p, s->r0.p, s->p.p, s->u.p, s->z.p, s->v.p, s->d.p,
                                       s->w.p, itr_max, tol_abs, tol_rel);
+  if (solver == "gauss-seidel") A.O = ord_view_of(s, true);
   const bool traced = ctx->tracing && solver == "iccg";
-  const bool wide = s->ord.Wc > 0;  // steps wider than the stage buffers hold
   if (traced) {
     const int nb = std::max(1, ctx->num_sms);
     const int cap = s->ord.max_tile_steps + 1;
@@ -1142,19 +1114,12 @@ static int solve_fp64(fc_ctx* ctx, CsrSystem* s, const std::string& solver, cons
   FC_CUDA_TRY(ctx, cudaMemsetAsync(s->out.p, 0, FC_OUT_N * sizeof(double), ctx->stream));
   int st;
   if (solver == "iccg")
-    st = launch_coop(ctx, s,
-                     traced ? (wide ? (const void*)k_iccg<double, true, true> : (const void*)k_iccg<double, true>)
-                            : wide ? (const void*)k_iccg<double, false, true> : (const void*)k_iccg<double>,
-                     A, nullptr,
-                     0);
+    st = launch_coop(ctx, s, traced ? (const void*)k_iccg<double, true> : (const void*)k_iccg<double>, A, nullptr, 0);
   else if (solver == "bicgstab") {
     if (s->tslot_oob) return fc_fail_msg(ctx, FC_ERR_BAD_INPUT, "bicgstab: pattern is not structurally symmetric");
-    st = launch_coop(ctx, s, wide ? (const void*)k_bicgstab<double, true> : (const void*)k_bicgstab<double>, A,
-                     nullptr, 0);
+    st = launch_coop(ctx, s, (const void*)k_bicgstab<double>, A, nullptr, 0);
   } else if (solver == "dpcg") st = launch_coop(ctx, s, (const void*)k_dpcg<double>, A, nullptr, 0, FC_BLOCK);
-  else if (solver == "gauss-seidel")
-    st = launch_coop(ctx, s, wide ? (const void*)k_gauss_seidel<true> : (const void*)k_gauss_seidel<false>, A,
-                     nullptr, 0);
+  else if (solver == "gauss-seidel") st = launch_coop(ctx, s, (const void*)k_gauss_seidel, A, nullptr, 0);
   else return fc_fail_msg(ctx, FC_ERR_UNSUPPORTED, "unknown solver '" + solver + "'");
   if (st) return st;
   return fetch_out(ctx, s, res);
@@ -1234,9 +1199,8 @@ static int solve_mixed(fc_ctx* ctx, CsrSystem* s, const std::string& solver, con
                                       0.0, inner_tol);
     F.skip_setup = outer > 0 ? 1 : 0;
     if (solver == "bicgstab") F.stall_window = FC_INNER_STALL_WINDOW;
-    const bool wide = s->ord.Wc > 0;
-    const void* fn = solver == "iccg" ? (wide ? (const void*)k_iccg<float, false, true> : (const void*)k_iccg<float>)
-                     : solver == "bicgstab" ? (wide ? (const void*)k_bicgstab<float, true> : (const void*)k_bicgstab<float>)
+    const void* fn = solver == "iccg"       ? (const void*)k_iccg<float>
+                     : solver == "bicgstab" ? (const void*)k_bicgstab<float>
                                             : (const void*)k_dpcg<float>;
     if ((st = launch_coop(ctx, s, fn, F, nullptr, 0, solver == "dpcg" ? FC_BLOCK : FC_SWEEP_BLOCK))) return st;
     FC_CUDA_TRY(ctx, cudaMemcpyAsync(s->h_out, s->out.p, FC_OUT_N * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1387,16 +1351,9 @@ static size_t batch_smem(const std::vector<BatchItem>& items) {
   size_t m = 0;
   for (const BatchItem& it : items) {
     const DevOrdered& D = it.s->ord;
-    m = std::max(m, osweep_smem_bytes<T>(D.R, D.stage_area, D.maxW, D.max_tile_steps));
+    m = std::max(m, osweep_smem_bytes<T>(D.R, D.stage_area, D.maxW));
   }
   return m;
-}
-
-// some problem of the batch has steps wider than its stage buffers hold
-static bool batch_wide(const std::vector<BatchItem>& items) {
-  for (const BatchItem& it : items)
-    if (it.s->ord.Wc > 0) return true;
-  return false;
 }
 
 int batch_solve(fc_ctx* ctx, BatchDev*& dev, std::vector<BatchItem>& items, const char* solver_c, int itr_max,
@@ -1434,9 +1391,7 @@ int batch_solve(fc_ctx* ctx, BatchDev*& dev, std::vector<BatchItem>& items, cons
     int* pb = B.bprob.p;
     BatchCtl* pc = B.ctl.p;
     void* args[3] = {&pa, &pb, &pc};
-    const void* fn64 = batch_wide(items) ? (const void*)k_bicgstab_batch<double, true>
-                                         : (const void*)k_bicgstab_batch<double>;
-    if ((st = batch_launch(ctx, B, fn64, args, batch_smem<double>(items)))) return st;
+    if ((st = batch_launch(ctx, B, (const void*)k_bicgstab_batch<double>, args, batch_smem<double>(items)))) return st;
     if ((st = batch_fetch(ctx, B))) return st;
     for (int p = 0; p < np; ++p) {
       const double* o = B.h_out + (size_t)p * FC_OUT_N;
@@ -1530,9 +1485,7 @@ int batch_solve(fc_ctx* ctx, BatchDev*& dev, std::vector<BatchItem>& items, cons
       }
       if ((st = batch_put_ctl(ctx, B))) return st;
       void* fa[3] = {&pf, &pb, &pc};
-      const void* fn32 = batch_wide(items) ? (const void*)k_bicgstab_batch<float, true>
-                                           : (const void*)k_bicgstab_batch<float>;
-      if ((st = batch_launch(ctx, B, fn32, fa, smemf))) return st;
+      if ((st = batch_launch(ctx, B, (const void*)k_bicgstab_batch<float>, fa, smemf))) return st;
       if ((st = batch_fetch(ctx, B))) return st;
       for (int p = 0; p < np; ++p) {
         PState& q = ps[p];
@@ -1559,9 +1512,7 @@ int sys_precond(fc_ctx* ctx, CsrSystem* s, int dilu, const double* q, double* z_
   KArgs<double> A = make_args<double>(s, s->a.p, s->x.p, q, s->r.p, s->r0.p, s->p.p, s->u.p, s->z.p, s->v.p, s->d.p,
                                       s->w.p, 0, 0.0, 0.0);
   void* extra[1] = {&apply};
-  const bool wide = s->ord.Wc > 0;
-  const void* fn = dilu ? (wide ? (const void*)k_precond<double, true, true> : (const void*)k_precond<double, true>)
-                        : (wide ? (const void*)k_precond<double, false, true> : (const void*)k_precond<double, false>);
+  const void* fn = dilu ? (const void*)k_precond<double, true> : (const void*)k_precond<double, false>;
   int st = launch_coop(ctx, s, fn, A, extra, 1);
   if (st) return st;
   FC_CUDA_TRY(ctx, cudaMemcpyAsync(s->h_status, s->status.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));

@@ -2,136 +2,232 @@
 // (linear_solvers.f90:439-475, :613-683) and of Gauss-Seidel (:96-201).
 //
 // The system is renumbered in schedule order (fc_schedule.hpp): tile t is
-// block t, and every step of a tile is a contiguous range of new rows.  The
-// block is warp-specialised: the last warp stages, the others compute.
+// block t, and every step of a tile is a contiguous range of new rows.  What
+// bounds a sweep is the chain of its levels: on a 128^3 hex mesh 382 levels
+// follow each other, each with three dependent FP64 FMAs (64 cycles each on
+// this part).  Everything else a step needs is therefore taken off that
+// chain, by warps of three kinds:
 //
-//  - stager (one thread): for each step, a handful of bulk asynchronous
-//    copies (cp.async.bulk, the TMA engine) bring the step's packed row
-//    records (16 bytes per row: entry count, push count, offsets, ring
-//    codes), its coefficient records (coefficients, d_i, 1/(d_i + small)),
-//    the right-hand-side window and the step's exchange and push blocks into
-//    a K-deep shared-memory ring of stage buffers, up to K-1 steps ahead.
-//    Buffer b is handed over with two mbarriers: full[b] (copies landed) and
-//    empty[b] (the compute warps are done with it).
-//  - compute warps (one row per thread): wait full[b], read the step from
-//    shared memory, take dependencies from the value ring (produced in this
-//    tile within the last R-1 steps) or from the exchange block, run the
-//    short FMA chain, store the value (vector, ring, pushes to consumers in
-//    other tiles or far behind in this one), then a named barrier among the
-//    compute warps and release of buffer b.
+//  - stager (one warp): per group of steps (four, fewer where the rows are
+//    many) two or three bulk asynchronous copies (cp.async.bulk, the TMA
+//    engine): the packed records of the group's steps (see below), the
+//    right-hand-side window and, where the mode has one, the extra row
+//    value, into a ring of K stage buffers.  Copies step by step, issued by
+//    one thread, took longer than the steps themselves (520-580 cycles).
+//  - importers (FC_IMP_WARPS warps, group g by warp g mod FC_IMP_WARPS): poll
+//    the exchanged values of the group's steps in global memory until their
+//    producers have stored them, put them into the stage buffer and the
+//    sentinel back into the slots, and release each step once it has all of
+//    its values.  A poll takes an L2 round trip, three to four steps; with a
+//    whole group to a poll and three groups polled at once it delays a tile
+//    once and not at every step.
+//  - compute warps, FC_SETS sets of FC_SET_WARPS warps, one row per thread;
+//    set s runs the steps s, s + FC_SETS, ...  A set loads its next step
+//    (record, coefficients, right-hand side, where each dependency's value
+//    will be) into registers while the other sets run theirs.  What remains
+//    between two steps is: a named barrier (the set of step k-1 and the
+//    importer of step k arrive, the set of step k waits), the ring loads, the
+//    FMAs, the ring store.  The pushes to other tiles and the stores to memory
+//    follow after the next set has been released.
+//
+// A stage buffer is handed over with two mbarriers: full (copies landed) and
+// empty (the compute warps are done with its steps).  A wait names a phase by
+// its parity, so it must come after the phase before it has completed and
+// before the one after it does.  With at least FC_SETS buffers that holds: a
+// set looks for step k after its own step k - FC_SETS and nobody refills the
+// buffer without it; the stager waits for every group in order; an importer
+// looks for group g - ahead (ahead <= K) after it looked for group g - ahead -
+// FC_IMP_WARPS, and group g and what follows cannot pass before it.
+//
+// Measured on a GB300, FP64, per level of one tile: 350 cycles forward with 30
+// rows a level, 400 forward and 500 backward with 108 rows (the FP64 pipe
+// takes 16-19 cycles per warp instruction: 4 x 3 FMAs forward, 4 x 5
+// operations backward).  A one-role block that polled, staged and computed in
+// turn took 1,950 cycles a step at every width; the forward sweep at 128^3
+// went from 456 to 177 us on the same 152 tiles, ICCG to 1e-10 from 384 to
+// 201 ms.
 //
 // Exchange: a value a row needs from another tile (or from more than R-1
 // steps back) is pushed by its producer into the consumer's slot of the
-// exchange array xv, whose slots start every sweep at a sentinel NaN.  The
-// static data of a step is staged many steps ahead, but exchanged values
-// are not: a copy taken that early is stale, and every stale value costs
-// the consumer an L2 round trip on its critical path and, through the lag
-// it builds up, delays every tile downstream.  Instead each compute thread
-// loads the exchanged values of its row of the next step from global memory
-// while it works on the current one (relaxed loads through L2); a value
-// that still reads as the sentinel is polled (bounded) until the producer's
-// store arrives.  The consumer puts the sentinel back after use.  Bulk
-// copies read through L2, so staged data is never an SM's stale L1 line.
+// exchange array xv, whose slots start every sweep at a sentinel NaN.
+//
+// Arithmetic.  The setups (factors d_i, inverted as the reference does)
+// and Gauss-Seidel use the reference's operations in its order.  The FP64
+// applications solve the same triangular systems in scaled form: forward
+// t_i = q_i - sum (a_ij d_j) t_j, where the reference's y_i is t_i d_i, and
+// backward z_i = (d_i / (d_i + small)) d_i t_i - sum (a_ij d_i) z_j, with the
+// bracketed factors formed once per solve.  That leaves three FMAs (the
+// entries of a row) on a level's chain and no multiplication by d_i.  FP32
+// FMAs take 4 cycles, so the FP32 applications keep the plain form.
 #pragma once
 #include <type_traits>
 #include "fc_krylov.cuh"
 #include "fc_schedule.hpp"
 
+// Warp roles of a block: FC_SETS x FC_SET_WARPS compute warps, the importers,
+// the stager.  A set is one warp per SM sub-partition and covers a step of
+// FC_SET_ROWS rows with one row per thread: four warps issue their FMAs in
+// about the 64 cycles one FMA takes, so more rows per step would lengthen the
+// step in proportion.  20 warps leave 96 registers a thread (21 would leave 80).
+#define FC_SETS 4
+#define FC_SET_WARPS 4
+#define FC_IMP_WARPS 3
+#define FC_SET_ROWS (32 * FC_SET_WARPS)
+static_assert(FC_SWEEP_BLOCK == 32 * (FC_SETS * FC_SET_WARPS + FC_IMP_WARPS + 1), "warp roles fill the block");
+
 namespace fcdev {
 
 // ------------------------------------------------- bulk copies, mbarriers
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned long long* mb, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(mb)), "r"(count) : "memory");
+__device__ __forceinline__ void mbar_init(unsigned mb, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_tx(unsigned long long* mb, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(mb)), "r"(bytes) : "memory");
+__device__ __forceinline__ void mbar_arrive_tx(unsigned mb, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* mb, unsigned parity) {
+__device__ __forceinline__ bool mbar_try_wait(unsigned mb, unsigned parity) {
   unsigned ok;
   asm volatile(
       "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
       : "=r"(ok)
-      : "r"(smem_addr(mb)), "r"(parity)
+      : "r"(mb), "r"(parity)
       : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ void mbar_arrive(unsigned mb, unsigned count = 1) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(count) : "memory");
+}
 // global -> shared bulk copy of bytes (multiple of 16, both addresses
 // 16-byte aligned), completion reported to mbarrier mb
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, unsigned long long* mb) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(mb))
+__device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned mb) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(mb)
                : "memory");
 }
 #define FC_MAX_STAGES 16
 #define FC_SMEM_HDR (2 * FC_MAX_STAGES * 8)  // full and empty mbarriers at the start of the dynamic area
 #define FC_MBAR_SPIN_LIMIT (1u << 22)
-__device__ __forceinline__ void mbar_arrive(unsigned long long* mb) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(mb)) : "memory");
-}
-// bounded wait for the completion of phase `parity`; false if it ran out.
-// backoff_ns > 0 sleeps between polls (a thread that is expected to wait
-// long, so that it does not load the shared-memory pipe of the workers)
-__device__ __forceinline__ bool mbar_wait(unsigned long long* mb, unsigned parity, unsigned backoff_ns = 0) {
+// bounded wait for the completion of phase `parity`; false if it ran out or
+// the block is leaving.  backoff_ns > 0 sleeps between polls (a thread that
+// is expected to wait long, so that it does not load the shared-memory pipe
+// of the workers)
+__device__ __forceinline__ bool mbar_wait(unsigned mb, unsigned parity, volatile int* abort_flag,
+                                          unsigned backoff_ns = 0) {
   unsigned spins = 0;
   while (!mbar_try_wait(mb, parity)) {
-    if (++spins > FC_MBAR_SPIN_LIMIT) return false;
+    if (++spins > FC_MBAR_SPIN_LIMIT || ((spins & 15u) == 0 && abort_flag && *abort_flag)) return false;
     if (backoff_ns) __nanosleep(backoff_ns);
   }
   return true;
 }
-// a hint to bring the line holding p into L2 (prefetch.global.L2)
-__device__ __forceinline__ void l2_prefetch(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+// the same for a whole warp: one lane polls (32 lanes polling one word take
+// turns on it), the others wait for it
+__device__ __forceinline__ bool mbar_wait_warp(unsigned mb, unsigned parity, volatile int* abort_flag) {
+  bool ok = true;
+  if ((threadIdx.x & 31) == 0) ok = mbar_wait(mb, parity, abort_flag);
+  return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
 }
-
-// barrier among the first nthreads threads (the compute warps)
-__device__ __forceinline__ void bar_compute(int nthreads) {
-  asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
+// Named barriers 1..FC_STEP_BARS: the barrier of step k releases the set of
+// step k once the set of step k-1 and the importer of step k have arrived.  The
+// importers stay less than FC_STEP_BARS steps ahead, so that none arrives twice.
+#define FC_STEP_BARS (FC_IMP_WARPS * FC_SETS)
+__device__ __forceinline__ void bar_wait(int id, int nthreads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
-// record strides (elements of T) of the per-solve row records
-template <class T> struct Rec { static constexpr int V = sizeof(T) == 8 ? 6 : 8; };
+__device__ __forceinline__ void bar_release(int id, int nthreads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
+// Shared memory by 32-bit address.  Volatile, so that they keep their place
+// with respect to the barriers above.
+__device__ __forceinline__ double lds(unsigned a, double) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float lds(unsigned a, float) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ int lds(unsigned a, int) {
+  int v;
+  asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ int4 lds4(unsigned a) {
+  int4 v;
+  asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts(unsigned a, double v) {
+  asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void sts(unsigned a, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+// a value pushed to another tile: single-copy atomic, so that a poll sees the
+// sentinel or the value
+__device__ __forceinline__ void st_push(double* p, double v) {
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+__device__ __forceinline__ void st_push(float* p, float v) {
+  asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
 
 // ------------------------------------------------------------------ views
 // device copy of an OrderedSweep (fc_schedule.hpp)
 struct OrdView {
-  int n, nE, ntiles, R, novf0, novf1, nsteps, maxW, xmax, pmax;
+  int n, nE, ntiles, R, novf0, novf1, nsteps;
+  int nc;                                // coefficients of a record: 3, or FC_ELL where a row has more
+  int gen;                               // rows of more than FC_ELL entries, or steps wider than FC_SET_ROWS
+  int G;                                 // steps of a group (stage buffer): FC_SETS, 2 or 1
+  int g_rows, g_padded, g_push, g_x;     // a group's most rows, padded rows, push targets, exchanged values
+  // desc[d]: per step, where it lies in the stage buffer of its group (the
+  // groups run downwards from the tile's last step backward): first row;
+  // rows | push targets << 16; padded rows | push targets << 16 of the group's
+  // steps before it in memory; its row in the windows | its first exchanged
+  // value << 16
   int stage_area;                        // bytes of the stage area (multiple of 16)
-  // rows of a step that are staged in shared memory: the rows of a wider
-  // step past the first Wc read their records from global memory, and the
-  // step's push block is read from global memory too (0: every step fits)
-  int Wc;
   const int* __restrict__ tile_step_ptr;
   const int* __restrict__ step_ptr;
+  const int* __restrict__ rp_ptr;
   const int* __restrict__ tile_W;
   const int* __restrict__ perm;
-  const int4* __restrict__ srec[2];
+  const int4* __restrict__ rec[2];
+  const int4* __restrict__ desc[2];
   const int* __restrict__ xv_ptr[2];
   const int* __restrict__ push_ptr[2];
-  const int* __restrict__ push[2];
-  const int* __restrict__ slot[2];
-  const int4* __restrict__ ucol;      // columns of the upper entries, 4 per row (Gauss-Seidel)
   const int* __restrict__ ovf_ptr[2];
   const int* __restrict__ ovf_code[2];
   const int* __restrict__ ovf_col[2];
   const int* __restrict__ ovf_slot[2];
   const int* __restrict__ lo_tslot;
   const int* __restrict__ lo_ovf_tslot;
-  const int* __restrict__ dslot;
   const int* __restrict__ p_ptr;
   const int* __restrict__ p_col;
   const int* __restrict__ p_slot;
 };
 
-// per-solve values in the new numbering (gathered by the kernel from the
+// Per-solve values in the new numbering (gathered by the kernel from the
 // caller's CSR values) and the exchange arrays; every vector of n rows is
 // allocated with nE entries (the padding is read by the staging windows and
-// never used)
+// never used).
+//
+// blob[d]: one block per step, the blocks of a tile's steps one after the
+// other, so that a group of steps is copied in one piece.  A block holds the
+// row records (16 bytes a row), the push targets, then the row values field
+// by field (coefficients of entries 0..nc-1, then scaled: backward the factor
+// of the right-hand side; plain: d_i and, backward, 1/(d_i + small)), the rows
+// padded to a multiple of 4.  Records and targets are written when the array
+// is allocated, the values by every solve.  Field by field because a warp
+// then reads 32 consecutive values of a field without bank conflicts.
+// sx, tx: per step (rows padded as in the blocks) a_ii, and the DILU
+// transposes a_(j,i) of entries 0..nc-1.
 template <class T>
 struct OrdVals {
-  T* vrec[2];  // [nE][Rec::V]: a_0..a_3 of the triangle, d_i, 1/(d_i + small)
-  T* sx;       // [nE][Rec::V]: a_ii, then the DILU transposes a_(j,i) of entries 0..3
+  unsigned char* blob[2];
+  T* sx;
+  T* tx;
   T* aovf[2];  // coefficients of the overflow entries
   T* tovf;     // DILU transposes of the lower overflow entries
   T* adiag;    // [nE]
@@ -139,43 +235,41 @@ struct OrdVals {
   T* xv[2];    // exchange arrays (per-step blocks)
 };
 
+// the form of the applications (see the file header)
+template <class T> struct ScaledApply { static constexpr bool value = sizeof(T) == 8; };
+// values per row of a step's block
+template <class T>
+__host__ __device__ inline int blob_fields(int nc, int dirn) { return nc + dirn + (ScaledApply<T>::value ? 0 : 1); }
+// byte offset of the block of a step: rp padded rows and pp push targets precede it
+template <class T>
+__host__ __device__ inline size_t blob_offset(int rp, int pp, int fields) {
+  return (size_t)rp * (16 + sizeof(T) * fields) + 4 * (size_t)pp;
+}
 // ------------------------------------------------------------------ modes
 enum { OS_SETUP_DIC = 0, OS_SETUP_DILU, OS_FWD, OS_BWD, OS_BWD_DOT, OS_GS };
 
 // ----------------------------------------------------------- staging area
-// One stage buffer: the step's row records, coefficient records, setup
-// records (a_ii and transposes), the Gauss-Seidel upper columns and
-// coefficients, the q and e windows (rows widened to 16-byte bounds) and
-// the exchange and push blocks.  init() lays out every area (the size the
-// host reserves per stage); init_for() only the areas one sweep mode reads,
-// so that the preconditioner applications, which need about 40% of a full
-// buffer, fit more stages into the same shared memory.
+// One stage buffer of a sweep mode, for a group of steps: the blocks, the
+// a_ii and transposes of the setups, for Gauss-Seidel a_ii and the blocks of the upper triangle, the q and e windows (rows
+// widened to 16-byte bounds) and the exchanged values.
 struct StageLayout {
-  int W, Wp;
-  int oS, oV, oX2, oU, oV2, oQ, oE, oXV, oP, bytes;
+  int oX, oT, oU, oQ, oE, oI, bytes;
   template <class T>
-  __host__ __device__ void init(int w, int xmax, int pmax) { init_for<T>(w, xmax, pmax, -1); }
-  template <class T>
-  __host__ __device__ void init_for(int w, int xmax, int pmax, int mode) {
-    const bool all = mode < 0;
-    const bool setup = all || mode == OS_SETUP_DIC || mode == OS_SETUP_DILU;
-    const bool gs = all || mode == OS_GS;
-    const bool kq = all || !(mode == OS_SETUP_DIC || mode == OS_SETUP_DILU);
-    const bool ke = all || mode == OS_BWD_DOT || mode == OS_GS;
-    W = w;
-    Wp = ((w + 3) & ~3) + 8;
+  __host__ __device__ static StageLayout of(const OrdView& O, int mode) {
+    StageLayout L;
+    const int sz = (int)sizeof(T), dirn = mode == OS_BWD || mode == OS_BWD_DOT;
+    const bool setup = mode == OS_SETUP_DIC || mode == OS_SETUP_DILU, gs = mode == OS_GS;
     int o = 0;
     auto take = [&](bool used, int b) { const int r = o; if (used) o += (b + 15) & ~15; return r; };
-    oS = take(true, 16 * W);
-    oV = take(true, (int)sizeof(T) * Rec<T>::V * W);
-    oX2 = take(setup || gs, (int)sizeof(T) * Rec<T>::V * W);
-    oU = take(gs, 16 * W);
-    oV2 = take(gs, (int)sizeof(T) * Rec<T>::V * W);
-    oQ = take(kq, (int)sizeof(T) * Wp);
-    oE = take(ke, (int)sizeof(T) * Wp);
-    oXV = take(false, (int)sizeof(T) * xmax);  // exchanged values are not staged (see the file header)
-    oP = take(true, 4 * pmax);
-    bytes = o;
+    take(true, 4 * O.g_push + (16 + blob_fields<T>(O.nc, dirn) * sz) * O.g_padded);
+    L.oX = take(setup || gs, sz * O.g_padded);
+    L.oT = take(mode == OS_SETUP_DILU, sz * O.g_padded * O.nc);
+    L.oU = take(gs, 4 * O.g_push + (16 + blob_fields<T>(O.nc, 1) * sz) * O.g_padded);
+    L.oQ = take(!setup, sz * (O.g_rows + 8));
+    L.oE = take(mode == OS_BWD_DOT || gs, sz * (O.g_rows + 8));
+    L.oI = take(true, sz * O.g_x);
+    L.bytes = o;
+    return L;
   }
 };
 
@@ -187,90 +281,65 @@ __host__ __device__ inline int stages_in(size_t area, int buffer_bytes) {
   return K;
 }
 
-// dynamic shared memory of an ordered-sweep kernel: 2 FC_MAX_STAGES
-// mbarriers, ring, the stage area (cut by every sweep mode into its own
-// buffers), the tile's step tables (rows, exchange and push offsets of both
-// directions) and the abort flag
+// dynamic shared memory of an ordered-sweep kernel: mbarriers, ring (and the
+// zero past its end), the stage area (cut by every sweep mode into its own
+// buffers) and the abort flag
 template <class T>
-inline size_t osweep_fixed_bytes(int R, int maxW, int max_tile_steps) {
-  size_t ring = ((size_t)R * maxW * sizeof(T) + 15) & ~(size_t)15;
-  size_t tab = ((size_t)5 * (max_tile_steps + 1) * 4 + 15) & ~(size_t)15;
-  return FC_SMEM_HDR + ring + tab + 16;
+inline size_t osweep_fixed_bytes(int R, int maxW) {
+  size_t ring = (((size_t)R * maxW + 1) * sizeof(T) + 15) & ~(size_t)15;
+  return FC_SMEM_HDR + ring + 16;
 }
 template <class T>
-inline size_t osweep_smem_bytes(int R, size_t stage_area, int maxW, int max_tile_steps) {
-  return osweep_fixed_bytes<T>(R, maxW, max_tile_steps) + stage_area;
+inline size_t osweep_smem_bytes(int R, size_t stage_area, int maxW) {
+  return osweep_fixed_bytes<T>(R, maxW) + stage_area;
 }
 
 struct OsCtx {
-  unsigned long long* full;   // [FC_MAX_STAGES]
-  unsigned long long* empty;  // [FC_MAX_STAGES]
-  unsigned char* ring;
-  unsigned char* stage;       // the stage area, cut by each sweep mode into its buffers
-  size_t stage_area;
-  int* sp;                    // [ns+1] first row of each local step (ascending levels)
-  int* xp[2];                 // [ns+1] exchange block offsets per direction
-  int* pp[2];                 // [ns+1] push block offsets per direction
+  unsigned full, empty;       // shared addresses of the mbarriers, [FC_MAX_STAGES] each
+  unsigned ring, stage;       // shared addresses
+  int W, ncw;                 // the tile's widest step; compute warps of a set
+  int s0, ns;                 // the tile's first step, its steps
   int* abort_flag;
-  // stage buffer b: bit b of `parity` = parity of its next fill/completion,
-  // bit b of `used` = it has been filled before (registers, no runtime-
-  // indexed arrays, so the context never goes to local memory)
-  unsigned parity, used;
-  StageLayout L;
+  unsigned parity;            // bit b: parity of the next use of stage buffer b
 };
 
 template <class T>
 __device__ __forceinline__ OsCtx osweep_ctx(const OrdView& O, unsigned char* smem, int t) {
   OsCtx X;
-  const int W = t < O.ntiles ? __ldg(O.tile_W + t) : 1;
-  X.L.template init<T>(W, O.xmax, O.pmax);
+  X.W = 1;
+  X.s0 = X.ns = 0;
+  if (t < O.ntiles) {
+    X.W = __ldg(O.tile_W + t);
+    X.s0 = __ldg(O.tile_step_ptr + t);
+    X.ns = __ldg(O.tile_step_ptr + t + 1) - X.s0;
+  }
+  X.ncw = min(FC_SET_WARPS, (X.W + 31) >> 5);
+  X.full = smem_addr(smem);
+  X.empty = X.full + 8 * FC_MAX_STAGES;
   // carve with this tile's width; the host sized the area for the widest
-  X.full = (unsigned long long*)smem;
-  X.empty = X.full + FC_MAX_STAGES;
   size_t off = FC_SMEM_HDR;
-  X.ring = smem + off;
-  off += ((size_t)O.R * W * sizeof(T) + 15) & ~(size_t)15;
-  X.stage = smem + off;
-  X.stage_area = (size_t)O.stage_area;
-  off += X.stage_area;
-  const int ns = t < O.ntiles ? __ldg(O.tile_step_ptr + t + 1) - __ldg(O.tile_step_ptr + t) : 0;
-  int* tab = (int*)(smem + off);
-  X.sp = tab;
-  X.xp[0] = tab + (ns + 1);
-  X.xp[1] = tab + 2 * (ns + 1);
-  X.pp[0] = tab + 3 * (ns + 1);
-  X.pp[1] = tab + 4 * (ns + 1);
-  off += ((size_t)5 * (ns + 1) * 4 + 15) & ~(size_t)15;
+  X.ring = smem_addr(smem + off);
+  off += (((size_t)O.R * X.W + 1) * sizeof(T) + 15) & ~(size_t)15;
+  X.stage = smem_addr(smem + off);
+  off += (size_t)O.stage_area;
   X.abort_flag = (int*)(smem + off);
   X.parity = 0;
-  X.used = 0;
-  if (t < O.ntiles) {
-    const int s0 = __ldg(O.tile_step_ptr + t);
-    for (int k = threadIdx.x; k <= ns; k += blockDim.x) {
-      X.sp[k] = __ldg(O.step_ptr + s0 + k);
-      X.xp[0][k] = __ldg(O.xv_ptr[0] + s0 + k);
-      X.xp[1][k] = __ldg(O.xv_ptr[1] + s0 + k);
-      X.pp[0][k] = __ldg(O.push_ptr[0] + s0 + k);
-      X.pp[1][k] = __ldg(O.push_ptr[1] + s0 + k);
-    }
-  }
   if (threadIdx.x == 0) {
     *X.abort_flag = 0;
     for (int b = 0; b < FC_MAX_STAGES; ++b) {
-      mbar_init(X.full + b, 1);
-      mbar_init(X.empty + b, 1);
+      mbar_init(X.full + 8 * b, 1);
+      mbar_init(X.empty + 8 * b, O.G * X.ncw);  // every step's warps
     }
+    sts(X.ring + O.R * X.W * (unsigned)sizeof(T), T(0));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   return X;
 }
 
-
 // Row sources of a sweep.  q: the right-hand side (forward, backward,
 // Gauss-Seidel), e: an extra row value (the dot partner of OS_BWD_DOT, the
-// previous iterate of Gauss-Seidel), out: where the row values go (the
-// setups write d_i there and into the coefficient records).
+// previous iterate of Gauss-Seidel), out: where the row values go.
 template <class T>
 struct OsIO {
   const T* q;
@@ -278,401 +347,436 @@ struct OsIO {
   T* out;
 };
 
-// bounded poll of an exchange slot; on timeout the kernel's status becomes
-// FC_ERR_TIMEOUT and the block's abort flag is raised
+// One row of a step between its loads and its result
 template <class T>
-__device__ __noinline__ T xv_wait(const GridCtl& C, const T* p, int* abort_flag) {
-  unsigned spins = 0;
-  T v = Sentinel<T>::poll(p);
-  while (Sentinel<T>::is(v)) {
-    if (++spins > FC_SPIN_LIMIT || *((volatile int*)C.status) != 0) {
-      atomicCAS(C.status, 0, FC_ERR_TIMEOUT);
-      *((volatile int*)abort_flag) = 1;
-      return T(0);
-    }
-    v = Sentinel<T>::poll(p);
-  }
-  return v;
-}
+struct OsRow {
+  unsigned at[FC_ELL];  // shared address of each dependency's value
+  T c[FC_ELL];          // coefficients (DIC: their squares)
+  T x[FC_ELL];          // DILU: transposes; Gauss-Seidel: products of the upper entries
+  T acc;                // right-hand side (setups: a_ii)
+  T aii, xo;            // Gauss-Seidel: diagonal, previous iterate
+  T di;                 // plain applications: d_i
+  int push;             // push targets | place of the first << 8
+  int ovf;              // entries | exchanged ones among the first FC_ELL << 8 | exchange offset << 16
+};
 
-// One ordered sweep of tile vg_bid(C).  WIDE: the structure has steps wider
-// than the stage buffers hold (OrdView::Wc > 0), whose further rows read
-// their records from global memory; without it the staged path is all there is.  dirn 0: forward over the lower
-// triangle, 1: backward over the upper one.  red (MODE OS_BWD_DOT: red[0] +=
+// One ordered sweep of tile vg_bid(C).  Directions: forward over the lower
+// triangle, backward over the upper one.  red (MODE OS_BWD_DOT: red[0] +=
 // e*value; OS_GS: red[0] += |residual|, red[1] += |a_ii x_i|) accumulates
-// per thread.  Every thread of the block calls it; it ends with a block
-// barrier but no grid barrier, and returns false if a wait ran out.
-template <class T, int MODE, bool WIDE = false, class TracerT = NoTrace>
-__device__ __forceinline__ bool osweep(const GridCtl& C, const OrdView& O, const OrdVals<T>& V, const OsIO<T>& io, OsCtx& X,
-                       double* red, TracerT* tr = nullptr) {
+// per thread.  NC: values of a record's coefficients, GEN: the structure has
+// rows of more than FC_ELL entries or steps wider than a set's threads.  Both
+// are template parameters because every branch that is left on the chain
+// counts: with the entry count, the overflow loop and the wide rows decided
+// at run time a step took 490-560 cycles instead of 350-400 (a tile of 30 and
+// one of 108 chains, forward), and more with the overflow loop inside.
+// Every thread of the block calls it; it ends with a block barrier but no
+// grid barrier, and returns false if a wait ran out.  A backward sweep may
+// follow its forward sweep directly: it reads the forward values of its own
+// tile only.  Not inlined: the solvers keep more state across a sweep than
+// the sweep's own loop leaves registers for.
+template <class T, int MODE, int NC, bool GEN, class TracerT>
+__device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, const OrdVals<T>& V, const OsIO<T> io,
+                                         OsCtx& Xr, double* red_out, TracerT* tr) {
   constexpr int dirn = (MODE == OS_BWD || MODE == OS_BWD_DOT) ? 1 : 0;
   constexpr bool kSetup = MODE == OS_SETUP_DIC || MODE == OS_SETUP_DILU;
-  constexpr bool kQ = !kSetup;
   constexpr bool kE = MODE == OS_BWD_DOT || MODE == OS_GS;
   constexpr bool kGS = MODE == OS_GS;
-  constexpr int VR = Rec<T>::V;
-  if (tr) tr->sweep();
-  const int t = vg_bid(C);
-  if (t >= O.ntiles) return true;
-  const int ns = __ldg(O.tile_step_ptr + t + 1) - __ldg(O.tile_step_ptr + t);
-  // the areas this mode reads, as many stage buffers as the area holds
-  // W: the tile's widest step (ring stride, compute threads); Ws: the rows of
-  // a step the stage buffers hold
-  const int W = X.L.W, Ws = WIDE && O.Wc > 0 ? min(W, O.Wc) : W;
-  StageLayout L;
-  L.template init_for<T>(Ws, O.xmax, O.pmax, MODE);
-  const int K = stages_in(X.stage_area, L.bytes), R = O.R;
-  const int nct = (int)blockDim.x - 32;  // threads before the staging warp
-  // compute threads of this tile: whole warps covering its widest step
-  const int ncg = min(nct, (W + 31) & ~31);
-  T* ring = (T*)X.ring;
-  T* xv = V.xv[dirn];
-  const int* sp = X.sp;
-  const int* xp = X.xp[dirn];
-  const int* pp = X.pp[dirn];
+  constexpr bool kScaled = ScaledApply<T>::value;
+  constexpr int SZ = (int)sizeof(T);
+  const OsCtx X = Xr;
+  constexpr int nc = NC;
+  const int ns = X.ns, R = O.R, G = O.G;
+  const StageLayout L = StageLayout::of<T>(O, MODE);
+  const int K = stages_in((size_t)O.stage_area, L.bytes);
+  const int kshift = __ffs(K) - 1, gshift = __ffs(G) - 1;  // both powers of two
+  T* const xv = V.xv[dirn];
+  volatile int* const abort_flag = X.abort_flag;
+  const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5;
+  double red[2] = {0.0, 0.0};
   auto step_of = [&](int k) { return dirn ? ns - 1 - k : k; };
+  // parity of the use of its buffer by group g
+  auto use_parity = [&](int g) { return ((X.parity >> (g & (K - 1))) ^ (unsigned)(g >> kshift)) & 1u; };
+  const int nth = 32 * X.ncw;  // threads of a set
+  auto step_bar = [&](int k) { return 1 + k % FC_STEP_BARS; };
+  auto step_bar_threads = [&](int k) { return (k > 0 ? 2 : 1) * nth + 32; };
+  auto fail = [&]() {
+    atomicCAS(C.status, 0, FC_ERR_TIMEOUT);
+    *abort_flag = 1;
+  };
 
-  if ((int)threadIdx.x >= nct) {
-    // ------------------------------------------------------------ stager
-    if (threadIdx.x == (unsigned)nct) {
-      bool ok = true;
-      for (int k = 0; k < ns && ok; ++k) {
-        if (*((volatile int*)X.abort_flag)) break;
-        const int b = k & (K - 1);
-        // a timeout here only records the status: the compute warps then run
-        // out of their own bounded wait and raise the abort flag themselves,
-        // so that they all see it after the same named barrier
-        // release of the previous fill of b: its completion had parity
-        // (parity bit ^ 1)
-        if (((X.used >> b) & 1u) && !mbar_wait(X.empty + b, ((X.parity >> b) & 1u) ^ 1u, 64)) {
-          atomicCAS(C.status, 0, FC_ERR_TIMEOUT);
-          ok = false;
-          break;
-        }
-        if (tr) tr->staged(k);
-        const int ls = step_of(k);
-        const int base = sp[ls], cnt = WIDE ? min(sp[ls + 1] - base, Ws) : sp[ls + 1] - base;  // the staged rows
-        const int b0 = base & ~3, nw = ((base + cnt + 3) & ~3) - b0;
-        const int p0 = pp[ls], np = !WIDE || sp[ls + 1] - base <= Ws ? pp[ls + 1] - p0 : 0;
-        unsigned char* B = X.stage + (size_t)b * L.bytes;
-        unsigned long long* mb = X.full + b;
-        const unsigned vb = (unsigned)(sizeof(T) * VR) * cnt;
-        unsigned bytes = 16u * cnt + vb + 4u * np;
-        if (kSetup || kGS) bytes += vb;
-        if (kGS) bytes += 16u * cnt + vb;
-        if (kQ) bytes += (unsigned)sizeof(T) * nw;
-        if (kE) bytes += (unsigned)sizeof(T) * nw;
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive_tx(mb, bytes);
-        bulk_g2s(B + L.oS, O.srec[dirn] + base, 16u * cnt, mb);
-        bulk_g2s(B + L.oV, V.vrec[dirn] + (size_t)base * VR, vb, mb);
-        if (kSetup || kGS) bulk_g2s(B + L.oX2, V.sx + (size_t)base * VR, vb, mb);
-        if (kGS) {
-          bulk_g2s(B + L.oU, O.ucol + base, 16u * cnt, mb);
-          bulk_g2s(B + L.oV2, V.vrec[1] + (size_t)base * VR, vb, mb);
-        }
-        if (kQ) bulk_g2s(B + L.oQ, io.q + b0, (unsigned)sizeof(T) * nw, mb);
-        if (kE) bulk_g2s(B + L.oE, io.e + b0, (unsigned)sizeof(T) * nw, mb);
-        if (np) bulk_g2s(B + L.oP, O.push[dirn] + p0, 4u * np, mb);
-        X.parity ^= 1u << b;
-        X.used |= 1u << b;
-      }
-    }
-  } else if ((int)threadIdx.x < ncg) {
+  if (wid < FC_SETS * FC_SET_WARPS) {
     // ------------------------------------------------------------ compute
-    // Only the ceil(W/32) warps that a step of this tile can occupy take
-    // part; the others skip the sweep, so they add no shared-memory traffic
-    // and no barrier arrivals to the steps.
-    const int kmask = K - 1;  // K and R are powers of two
-    // the exchanged values of this thread's first row of step k, loaded
-    // during step k-1 (pf_ok), and whether step k's buffer was waited for then
-    T pf[FC_ELL];
-    bool pf_ok = false, pre_waited = false;
+    const int set = wid / FC_SET_WARPS, sw = wid % FC_SET_WARPS;
+    if (sw < X.ncw && set < ns) {
+      // only the warps that the tile's widest step needs take part
+      const int row0 = 32 * sw + lane;
+      const int4* const desc = O.desc[dirn] + X.s0;
+      const unsigned rw = (unsigned)(R * X.W);  // place of the zero
+      constexpr int kStride = 16;               // bytes of a record
+      const int rec_bytes = kStride + SZ * blob_fields<T>(nc, dirn);
+      int4 next = __ldg(desc + step_of(set));
+      int k = set;
+      for (; k < ns; k += FC_SETS) {
+        if (tr) tr->step(k);
+        const int4 d = next;
+        if (k + FC_SETS < ns) next = __ldg(desc + step_of(k + FC_SETS));
+        const int g = k >> gshift, b = g & (K - 1);
+        const int base = d.x, cnt = d.y & 0xFFFF, cp = (cnt + 3) & ~3, woff = d.w & 0xFFFF;
+        const int rpo = d.z & 0xFFFF, ppo = (int)((unsigned)d.z >> 16);
+        const unsigned S = X.stage + (unsigned)(b * L.bytes), B = S + (unsigned)(rpo * rec_bytes + 4 * ppo);
+        const unsigned PS = B + kStride * cp;
+        const unsigned CF = PS + 4 * ((unsigned)d.y >> 16);  // the step's values
+        const unsigned I = S + L.oI + ((unsigned)d.w >> 16) * SZ - (rw + 1) * SZ;
+        const unsigned ring_out = X.ring + (unsigned)((k & (R - 1)) * X.W * SZ);
+        if (!mbar_wait_warp(X.full + 8 * b, use_parity(g), abort_flag)) break;
+        if (tr) tr->waited(k);
+        auto load = [&](int sl, OsRow<T>& w) {
+          const int4 sr = lds4(B + kStride * sl);
+          const unsigned cf = CF + (unsigned)(sl * SZ), cs = (unsigned)(cp * SZ);
 #pragma unroll
-    for (int e = 0; e < FC_ELL; ++e) pf[e] = T(0);
-    // wait for step kk's buffer (warps with rows in it) and load the
-    // exchanged values of row threadIdx.x of that step into pf
-    auto prefetch = [&](int kk) {
-      const int lsk = step_of(kk);
-      const int bk = kk & kmask, basek = sp[lsk], cntk = sp[lsk + 1] - basek;
-      pf_ok = false;
-      pre_waited = false;
-      if ((int)(threadIdx.x & ~31u) >= cntk) return;
-      if (!mbar_wait(X.full + bk, (X.parity >> bk) & 1u)) {
-        atomicCAS(C.status, 0, FC_ERR_TIMEOUT);
-        *((volatile int*)X.abort_flag) = 1;
-      }
-      pre_waited = true;
-      if ((int)threadIdx.x >= cntk) return;
-      const int4 sr = !WIDE || (int)threadIdx.x < Ws
-                          ? ((const int4*)(X.stage + (size_t)bk * L.bytes + L.oS))[threadIdx.x]
-                          : __ldg(O.srec[dirn] + basek + threadIdx.x);
-      const int ne = sr.x & 255, xoff = (int)((unsigned)sr.x >> 16);
-      const unsigned cw[2] = {(unsigned)sr.z, (unsigned)sr.w};
-      const T* src = xv + xp[lsk] + xoff;
-      int m = 0;
+          for (int e = 0; e < NC; ++e) w.c[e] = lds(cf + e * cs, T());
+          w.push = sr.x;
+          w.ovf = sr.w;
+          const unsigned p01 = (unsigned)sr.y, p23 = (unsigned)sr.z;
+          const unsigned place[FC_ELL] = {p01 & 0xFFFFu, p01 >> 16, p23 & 0xFFFFu, p23 >> 16};
 #pragma unroll
-      for (int e = 0; e < FC_ELL; ++e) {
-        const bool ex = ((cw[e >> 1] >> (16 * (e & 1))) & 0xFFFFu) == 0 && e < ne;
-        pf[e] = ex ? Sentinel<T>::poll(src + m) : T(0);
-        m += ex ? 1 : 0;
-      }
-      pf_ok = true;
-    };
-    if (ns > 0) prefetch(0);
-    for (int k = 0; k < ns; ++k) {
-      if (tr) tr->step(k);
-      const int b = k & kmask;
-      const int ls = step_of(k);
-      const int base = sp[ls], cnt = sp[ls + 1] - base, woff = base - (base & ~3);
-      // only warps with rows in this step read the buffer, so only they wait
-      // for it (an mbarrier poll by every warp would serialise on its word)
-      if (!pre_waited && (int)(threadIdx.x & ~31u) < cnt && !mbar_wait(X.full + b, (X.parity >> b) & 1u)) {
-        atomicCAS(C.status, 0, FC_ERR_TIMEOUT);
-        *((volatile int*)X.abort_flag) = 1;
-      }
-      if (tr) tr->waited(k);
-      const bool have_pf = pf_ok;
-      T pfk[FC_ELL];
+          for (int e = 0; e < NC; ++e) w.at[e] = (place[e] <= rw ? X.ring : I) + place[e] * SZ;
+          if constexpr (kSetup) {
+            w.acc = lds(S + L.oX + (rpo + sl) * SZ, T());
 #pragma unroll
-      for (int e = 0; e < FC_ELL; ++e) pfk[e] = pf[e];
-      // the next step's exchanged values are loaded while this one runs
-      if (k + 1 < ns) prefetch(k + 1);
-      else { pf_ok = false; pre_waited = false; }
-      if constexpr (WIDE) {
-        // the records of this thread's unstaged rows of the next step are
-        // brought into L2 while this step runs (they are read through L2)
-        if (k + 1 < ns) {
-          const int lsn = step_of(k + 1), basen = sp[lsn], cntn = sp[lsn + 1] - basen;
-          for (int sl = threadIdx.x; sl < cntn; sl += ncg) {
-            if (sl < Ws) continue;
-            const int qn = basen + sl;
-            l2_prefetch(O.srec[dirn] + qn);
-            l2_prefetch(V.vrec[dirn] + (size_t)qn * VR);
-            l2_prefetch(V.vrec[dirn] + (size_t)qn * VR + VR - 1);
-            if (kQ) l2_prefetch(io.q + qn);
-            if (kE) l2_prefetch(io.e + qn);
-          }
-          // a wide step's push block, read from global memory, line by line
-          if (cntn > Ws) {
-            const int* pb = O.push[dirn] + pp[lsn];
-            const int npn = pp[lsn + 1] - pp[lsn];
-            for (int o = (int)threadIdx.x * 32; o < npn; o += ncg * 32) l2_prefetch(pb + o);
-          }
-        }
-      }
-      if (tr) tr->at(k, 4, (int)pf_ok);
-      const int xbase = xp[ls];
-      const unsigned char* B = X.stage + (size_t)b * L.bytes;
-      const int4* S4 = (const int4*)(B + L.oS);
-      const T* VRc = (const T*)(B + L.oV);
-      // the push block: staged for a step the stage buffer holds whole, else
-      // read from global memory
-      const int* PS = !WIDE || cnt <= Ws ? (const int*)(B + L.oP) : O.push[dirn] + pp[ls];
-      T* ring_out = ring + (k & (R - 1)) * W;
-      // one row of the step; STG: its records are in the stage buffer, else
-      // (the rows of a wider step past the staged ones) in global memory
-      auto row = [&](const int sl, auto stg_tag) {
-        constexpr bool STG = decltype(stg_tag)::value;
-        const int q = base + sl;
-        const int4 sr = STG ? S4[sl] : __ldg(O.srec[dirn] + q);
-        const int ne = sr.x & 255, np = (sr.x >> 8) & 255, xoff = (int)((unsigned)sr.x >> 16), poff = sr.y;
-        T vl[VR];  // an unstaged row's coefficient record
-        if constexpr (!STG)
-#pragma unroll
-          for (int e = 0; e < VR; ++e) vl[e] = ldcg(V.vrec[dirn] + (size_t)q * VR + e);
-        const T* vr = STG ? VRc + sl * VR : vl;
-        // dependency values of entries 0..3 without branches: entries past
-        // ne have code 0 and coefficient 0, so they contribute an exact
-        // zero; ring (code > 0) or exchanged value (code 0) by select.  The
-        // thread's first row takes its exchanged values from the loads of
-        // the previous step, every other row polls them below.
-        const unsigned cw[2] = {(unsigned)sr.z, (unsigned)sr.w};
-        const bool mine = have_pf && sl == (int)threadIdx.x;
-        T dv[FC_ELL];
-        unsigned xmask = 0;  // entries that come through the exchange array
-        int m = 0;
-#pragma unroll
-        for (int e = 0; e < FC_ELL; ++e) {
-          const int c1 = (int)((cw[e >> 1] >> (16 * (e & 1))) & 0xFFFFu);  // code + 1
-          const bool ex = c1 == 0 && e < ne;
-          const T rv = ring[c1 > 0 ? c1 - 1 : 0];
-          const T xv_ = mine ? pfk[e] : Sentinel<T>::value();
-          dv[e] = c1 > 0 ? rv : (ex ? xv_ : T(0));
-          xmask |= (ex ? 1u : 0u) << e;
-          m += ex ? 1 : 0;
-        }
-        if (xmask) {
-          // exchanged values: poll the slot if the early load came before
-          // the producer's store, and put the sentinel back
-          int mm = 0;
-#pragma unroll
-          for (int e = 0; e < FC_ELL; ++e)
-            if ((xmask >> e) & 1u) {
-              T v = dv[e];
-              if (Sentinel<T>::is(v)) v = xv_wait<T>(C, xv + xbase + xoff + mm, X.abort_flag);
-              xv[xbase + xoff + mm] = Sentinel<T>::value();
-              dv[e] = v;
-              ++mm;
+            for (int e = 0; e < NC; ++e) {
+              if (MODE == OS_SETUP_DILU) w.x[e] = lds(S + L.oT + (unsigned)((rpo * nc + e * cp + sl) * SZ), T());
+              else w.c[e] = mul_rn(w.c[e], w.c[e]);
             }
-        }
-        if (tr && sl == 0) tr->at(k, 5, __double_as_longlong((double)dv[0] + (double)dv[1] + (double)dv[2]));
-        // overflow entry e >= FC_ELL: its value and coefficient
-        auto dep_ovf = [&](int e, T& a) -> T {
-          const int o = __ldg(O.ovf_ptr[dirn] + q) + e - FC_ELL;
-          a = __ldg(V.aovf[dirn] + o);
-          const int c = __ldg(O.ovf_code[dirn] + o);
-          if (c >= 0) return ring[c];
-          const T v = xv_wait<T>(C, xv + xbase + xoff + m, X.abort_flag);
-          xv[xbase + xoff + m] = Sentinel<T>::value();
-          ++m;
-          return v;
+          } else if constexpr (kGS) {
+            w.acc = lds(S + L.oQ + (woff + sl) * SZ, T());
+            w.aii = lds(S + L.oX + (rpo + sl) * SZ, T());
+            w.xo = lds(S + L.oE + (woff + sl) * SZ, T());
+            // the upper triangle's block of the same step
+            const int s = X.s0 + k, p1 = __ldg(O.push_ptr[1] + s), p0 = __ldg(O.push_ptr[1] + X.s0 + (k & ~(G - 1)));
+            const unsigned U = S + L.oU + (unsigned)(rpo * (kStride + SZ * blob_fields<T>(nc, 1)) + 4 * (p1 - p0));
+            const unsigned UC = U + kStride * cp + 4 * (__ldg(O.push_ptr[1] + s + 1) - p1);
+            const int nu = lds(U + kStride * sl + 12, int()) & 255, k0 = __ldg(O.p_ptr + base + sl) + (w.ovf & 255) + 1;
+#pragma unroll
+            for (int e = 0; e < NC; ++e)
+              w.x[e] = e < nu ? mul_rn(lds(UC + (unsigned)((e * cp + sl) * SZ), T()), ldcg(io.e + __ldg(O.p_col + k0 + e)))
+                              : T(0);
+          } else {
+            w.acc = lds(S + L.oQ + (woff + sl) * SZ, T());
+            if constexpr (!kScaled) w.di = lds(cf + nc * cs, T());
+            if constexpr (dirn == 1) w.acc = w.acc * lds(cf + (nc + (kScaled ? 0 : 1)) * cs, T());
+          }
         };
-        T val;
-        if (kSetup) {
-          // d_i = a_ii - sum a_k^2 d_j (DIC) or a_k d_j a_(j,i) (DILU), then 1/d_i
-          // (the recurrence is exact, so entries past ne are skipped)
-          T sl_x[VR];
-          if constexpr (!STG)
+        // overflow entry e >= FC_ELL of a row: its value and coefficient; m
+        // counts the row's exchanged entries
+        auto dep_ovf = [&](const OsRow<T>& w, int q, int e, int& m, T& a) -> T {
+          const int o = __ldg(O.ovf_ptr[dirn] + q) + e - FC_ELL;
+          a = ldcg(V.aovf[dirn] + o);
+          const int c = __ldg(O.ovf_code[dirn] + o);
+          return lds(c >= 0 ? X.ring + c * SZ : I + (rw + 1 + ((unsigned)w.ovf >> 16) + m++) * SZ, T());
+        };
+        // the row's value from its dependencies
+        auto value = [&](int sl, OsRow<T>& w) {
+          T v[NC];
 #pragma unroll
-            for (int e = 0; e < VR; ++e) sl_x[e] = ldcg(V.sx + (size_t)q * VR + e);
-          const T* sx = STG ? (const T*)(B + L.oX2) + sl * VR : sl_x;
-          T di = sx[0];
+          for (int e = 0; e < NC; ++e) v[e] = lds(w.at[e], T());
+          int m = (w.ovf >> 8) & 255;
+          const int ne = GEN ? w.ovf & 255 : 0, q = base + sl;
+          T val = w.acc;
+          if constexpr (kSetup) {
+            // d_i = a_ii - sum a_k^2 d_j (DIC) or a_k d_j a_(j,i) (DILU), then
+            // 1/d_i; entries past the row's subtract an exact zero
 #pragma unroll
-          for (int e = 0; e < FC_ELL; ++e)
-            if (e < ne) {
-              const T a = vr[e];
-              di = MODE == OS_SETUP_DILU ? sub_rn(di, mul_rn(mul_rn(a, dv[e]), sx[1 + e]))
-                                         : sub_rn(di, mul_rn(mul_rn(a, a), dv[e]));
+            for (int e = 0; e < NC; ++e)
+              val = MODE == OS_SETUP_DILU ? sub_rn(val, mul_rn(mul_rn(w.c[e], v[e]), w.x[e]))
+                                          : sub_rn(val, mul_rn(w.c[e], v[e]));
+            for (int e = FC_ELL; e < ne; ++e) {
+              T a;
+              const T dj = dep_ovf(w, q, e, m, a);
+              const T at = MODE == OS_SETUP_DILU ? ldcg(V.tovf + __ldg(O.ovf_ptr[0] + q) + e - FC_ELL) : a;
+              val = MODE == OS_SETUP_DILU ? sub_rn(val, mul_rn(mul_rn(a, dj), at)) : sub_rn(val, mul_rn(mul_rn(a, a), dj));
             }
-          for (int e = FC_ELL; e < ne; ++e) {
-            T a;
-            const T dj = dep_ovf(e, a);
-            const T at = MODE == OS_SETUP_DILU ? __ldg(V.tovf + __ldg(O.ovf_ptr[0] + q) + e - FC_ELL) : a;
-            di = MODE == OS_SETUP_DILU ? sub_rn(di, mul_rn(mul_rn(a, dj), at)) : sub_rn(di, mul_rn(mul_rn(a, a), dj));
+            val = div_rn(T(1), val);
           }
-          val = div_rn(T(1), di);
-          const T f = T(1) / (val + (T)FC_SMALL);
-          V.vrec[0][(size_t)q * VR + 4] = val;
-          V.vrec[0][(size_t)q * VR + 5] = f;
-          V.vrec[1][(size_t)q * VR + 4] = val;
-          V.vrec[1][(size_t)q * VR + 5] = f;
-        } else if (kGS) {
-          // s = b - sum_{k<kd} a x_new - a_ii x_old_i - sum_{k>kd} a x_old;
-          // x_i = x_old_i + s / (a_ii + small)   (exact arithmetic)
-          T s = STG ? ((const T*)(B + L.oQ))[woff + sl] : ldcg(io.q + q);
+          if constexpr (kGS) {
+            // s = b - sum_{k<kd} a x_new - a_ii x_old_i - sum_{k>kd} a x_old;
+            // x_i = x_old_i + s / (a_ii + small)   (exact arithmetic)
 #pragma unroll
-          for (int e = 0; e < FC_ELL; ++e)
-            if (e < ne) s = sub_rn(s, mul_rn(vr[e], dv[e]));
-          for (int e = FC_ELL; e < ne; ++e) {
-            T a;
-            const T xj = dep_ovf(e, a);
-            s = sub_rn(s, mul_rn(a, xj));
-          }
-          const T aii = STG ? ((const T*)(B + L.oX2))[sl * VR] : ldcg(V.sx + (size_t)q * VR);
-          const T xo = STG ? ((const T*)(B + L.oE))[woff + sl] : ldcg(io.e + q);
-          s = sub_rn(s, mul_rn(aii, xo));
-          const int nu = __ldg(&O.srec[1][q].x) & 255;
-          T v2l[VR];
-          if constexpr (!STG)
-#pragma unroll
-            for (int e = 0; e < VR; ++e) v2l[e] = ldcg(V.vrec[1] + (size_t)q * VR + e);
-          const T* v2 = STG ? (const T*)(B + L.oV2) + sl * VR : v2l;
-          const int4 uc = STG ? ((const int4*)(B + L.oU))[sl] : __ldg(O.ucol + q);
-#pragma unroll
-          for (int e = 0; e < FC_ELL; ++e)
-            if (e < nu) {
-              const int cj = e == 0 ? uc.x : e == 1 ? uc.y : e == 2 ? uc.z : uc.w;
-              s = sub_rn(s, mul_rn(v2[e], ldcg(io.e + cj)));
+            for (int e = 0; e < NC; ++e) val = sub_rn(val, mul_rn(w.c[e], v[e]));
+            for (int e = FC_ELL; e < ne; ++e) {
+              T a;
+              const T xj = dep_ovf(w, q, e, m, a);
+              val = sub_rn(val, mul_rn(a, xj));
             }
-          for (int e = FC_ELL; e < nu; ++e) {
-            const int o = __ldg(O.ovf_ptr[1] + q) + e - FC_ELL;
-            s = sub_rn(s, mul_rn(__ldg(V.aovf[1] + o), ldcg(io.e + __ldg(O.ovf_col[1] + o))));
+            val = sub_rn(val, mul_rn(w.aii, w.xo));
+#pragma unroll
+            for (int e = 0; e < NC; ++e) val = sub_rn(val, w.x[e]);
+            const int nu = GEN ? __ldg(&O.rec[1][q].w) & 255 : 0;
+            for (int e = FC_ELL; e < nu; ++e) {
+              const int o = __ldg(O.ovf_ptr[1] + q) + e - FC_ELL;
+              val = sub_rn(val, mul_rn(ldcg(V.aovf[1] + o), ldcg(io.e + __ldg(O.ovf_col[1] + o))));
+            }
+            w.acc = val;
+            val = add_rn(w.xo, div_rn(val, add_rn(w.aii, (T)FC_SMALL)));
           }
-          val = add_rn(xo, div_rn(s, add_rn(aii, (T)FC_SMALL)));
-          red[0] += fabs((double)s);
-          red[1] += fabs((double)aii * (double)val);
-        } else {
-          // forward: y_i = (q_i - sum a y_j) d_i;
-          // backward: z_i = (y_i / (d_i + small) - sum a z_j) d_i, the division
-          // taken as a product with 1/(d_i + small) from the setup.  Entries
-          // 0..2 unconditionally (padding adds exactly zero), entry 3 when
-          // present.
-          const T di = vr[4];
-          T acc = STG ? ((const T*)(B + L.oQ))[woff + sl] : ldcg(io.q + q);
-          if (dirn) acc = acc * vr[5];
-          acc = fma(-vr[0], dv[0], acc);
-          acc = fma(-vr[1], dv[1], acc);
-          acc = fma(-vr[2], dv[2], acc);
-          if (ne > 3) acc = fma(-vr[3], dv[3], acc);
-          for (int e = FC_ELL; e < ne; ++e) {
-            T a;
-            const T v = dep_ovf(e, a);
-            acc = fma(-a, v, acc);
+          if constexpr (!kSetup && !kGS) {
+            // scaled: the nearest row's entry last (the last one forward, the
+            // first one backward); plain: in the row's order
+            if constexpr (dirn == 0 || !kScaled) {
+#pragma unroll
+              for (int e = 0; e < NC; ++e) val = fma(-w.c[e], v[e], val);
+            }
+            for (int e = FC_ELL; e < ne; ++e) {
+              T a;
+              const T x = dep_ovf(w, q, e, m, a);
+              val = fma(-a, x, val);
+            }
+            if constexpr (dirn == 1 && kScaled) {
+#pragma unroll
+              for (int e = NC - 1; e >= 0; --e) val = fma(-w.c[e], v[e], val);
+            }
+            if constexpr (!kScaled) val = val * w.di;
           }
-          val = acc * di;
-          if (MODE == OS_BWD_DOT)
-            red[0] += (double)(STG ? ((const T*)(B + L.oE))[woff + sl] : ldcg(io.e + q)) * (double)val;
+          return val;
+        };
+        // pushes, the result vector, the reductions
+        auto store = [&](int sl, const OsRow<T>& w, T val) {
+          const int np = w.push & 255;
+          const unsigned ps = PS + 4 * ((unsigned)w.push >> 8);
+          for (int m = 0; m < np; ++m) st_push(xv + lds(ps + 4 * m, int()), val);
+          io.out[base + sl] = val;
+          if constexpr (MODE == OS_BWD_DOT) red[0] += (double)lds(S + L.oE + (woff + sl) * SZ, T()) * (double)val;
+          if constexpr (kGS) {
+            red[0] += fabs((double)w.acc);
+            red[1] += fabs((double)w.aii * (double)val);
+          }
+        };
+        // threads past the step's rows repeat its last row up to the ring
+        // store, so that nothing on the chain branches
+        const int sl = min(row0, cnt - 1);
+        OsRow<T> w;
+        load(sl, w);
+        if (tr) tr->at(k, 4, 0);
+        const int bar = step_bar(k), bar1 = bar == FC_STEP_BARS ? 1 : bar + 1;
+        __syncwarp();
+        bar_wait(bar, step_bar_threads(k));
+        if (tr) tr->at(k, 5, 0);
+        T val = value(sl, w);
+        if (row0 < cnt) sts(ring_out + row0 * SZ, val);
+        if constexpr (GEN && !kGS) {
+          if (cnt > nth)  // a step wider than a set's threads (forced widths only)
+            for (int s2 = row0 + nth; s2 < cnt; s2 += nth) {
+              OsRow<T> w2;
+              load(s2, w2);
+              const T v2 = value(s2, w2);
+              sts(ring_out + s2 * SZ, v2);
+              store(s2, w2, v2);
+            }
         }
-        if (tr && sl == 0) tr->at(k, 6, __double_as_longlong((double)val));
-        io.out[q] = val;
-        ring_out[sl] = val;
-        // plain stores: an aligned 8-byte (4-byte) store is single-copy
-        // atomic, so a consumer polling the slot sees the sentinel or the value
-        for (int mm = 0; mm < np; ++mm) xv[PS[poff + mm]] = val;
-        if (tr && sl == 0) tr->at(k, 7, np);
-      };
-      for (int sl = threadIdx.x; sl < cnt; sl += ncg) {
-        if constexpr (WIDE) {
-          if (sl < Ws) row(sl, std::true_type{});
-          else row(sl, std::false_type{});
-        } else {
-          row(sl, std::true_type{});
+        if (tr) tr->at(k, 6, __double_as_longlong((double)val));
+        __syncwarp();
+        if (k + 1 < ns) bar_release(bar1, step_bar_threads(k + 1));
+        if (row0 < cnt) store(row0, w, val);
+        if (tr) tr->at(k, 7, 0);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(X.empty + 8 * b);
+      }
+      if (k < ns) {
+        // a wait for records ran out: only the barriers are kept up
+        if (lane == 0) fail();
+        for (; k < ns; k += FC_SETS) {
+          __syncwarp();
+          bar_wait(step_bar(k), step_bar_threads(k));
+          if (k + 1 < ns) bar_release(step_bar(k + 1), step_bar_threads(k + 1));
         }
       }
-      bar_compute(ncg);
-      if (threadIdx.x == 0) mbar_arrive(X.empty + b);
-      X.parity ^= 1u << b;
-      X.used |= 1u << b;
-      if (*((volatile int*)X.abort_flag)) break;
     }
+  } else if (wid < FC_SETS * FC_SET_WARPS + FC_IMP_WARPS) {
+    // ----------------------------------------------------------- importers
+    constexpr int U = 4;  // polls in flight per lane
+    const int* const xp = O.xv_ptr[dirn] + X.s0;
+    const int ng = (ns + G - 1) >> gshift, ahead = min(K, FC_STEP_BARS >> gshift);  // groups
+    bool ok = true;   // false: only the barriers are kept up
+    for (int g = wid - FC_SETS * FC_SET_WARPS; g < ng; g += FC_IMP_WARPS) {
+      const int k0 = g << gshift, k1 = min(k0 + G, ns), b = g & (K - 1);
+      const int lo = dirn ? ns - k1 : k0, hi = dirn ? ns - k0 : k1;
+      const int x0 = __ldg(xp + lo), nx = __ldg(xp + hi) - x0;
+      const unsigned I = X.stage + (unsigned)(b * L.bytes + L.oI);
+      // the values in the order of the steps: value i lies at place(i)
+      auto place = [&](int i) { return dirn ? nx - 1 - i : i; };
+      int rel = k0;  // next step to release
+      // lane j: the values of step k0 + j end before value my_end
+      int my_end = 0x7FFFFFFF;
+      if (k0 + lane < k1) my_end = dirn ? nx - (__ldg(xp + ns - 1 - k0 - lane) - x0) : __ldg(xp + k0 + lane + 1) - x0;
+      auto release = [&](int have) {  // the steps whose values are all among the first `have`
+        while (rel < k1 && __shfl_sync(0xffffffffu, my_end, rel - k0) <= have) {
+          bar_release(step_bar(rel), step_bar_threads(rel));
+          ++rel;
+        }
+      };
+      // the place of the values, and the barriers of the steps, are free once
+      // group g - ahead is done
+      if (ok && g >= ahead) ok = mbar_wait_warp(X.empty + 8 * ((g - ahead) & (K - 1)), use_parity(g - ahead), abort_flag);
+      if (ok) release(0);
+      for (int c0 = 0; c0 < nx && ok; c0 += 32 * U) {
+        unsigned pending = 0, spins = 0;
+#pragma unroll
+        for (int j = 0; j < U; ++j) pending |= (c0 + 32 * j + lane < nx ? 1u : 0u) << j;
+        for (;;) {
+          T v[U];
+#pragma unroll
+          for (int j = 0; j < U; ++j)
+            v[j] = (pending >> j) & 1u ? Sentinel<T>::poll(xv + x0 + place(c0 + 32 * j + lane)) : Sentinel<T>::value();
+#pragma unroll
+          for (int j = 0; j < U; ++j) {
+            if (Sentinel<T>::is(v[j])) continue;
+            const int at = place(c0 + 32 * j + lane);
+            sts(I + at * SZ, v[j]);
+            st_push(xv + x0 + at, Sentinel<T>::value());
+            pending &= ~(1u << j);
+          }
+          const unsigned first = pending ? (unsigned)(c0 + 32 * (__ffs(pending) - 1) + lane) : 0xFFFFFFFFu;
+          const unsigned have = __reduce_min_sync(0xffffffffu, first);
+          release(have == 0xFFFFFFFFu ? min(c0 + 32 * U, nx) : (int)have);
+          if (have == 0xFFFFFFFFu) break;
+          // the status word is in global memory: another block's failure is
+          // looked for every 256 polls only
+          if (++spins > FC_SPIN_LIMIT || *abort_flag || ((spins & 255u) == 0 && *((volatile int*)C.status) != 0)) ok = false;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+        }
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        // missing values only spoil numbers that an error status goes with
+        if (lane == 0) fail();
+        for (; rel < k1; ++rel) {
+          __syncwarp();
+          bar_wait(step_bar(rel), step_bar_threads(rel));
+        }
+      }
+    }
+  } else {
+    // -------------------------------------------------------------- stager
+    // each lane works out the copies of one group of the next 32 and issues
+    // them in its turn.  The vectors were written by ordinary stores, the
+    // copies are not ordinary loads.
+    asm volatile("fence.proxy.async;" ::: "memory");
+    const int ng = (ns + G - 1) >> gshift;
+    int issued = 0;
+    bool ok = true;
+    for (int g0 = 0; g0 < ng && ok; g0 += 32) {
+      const int g = min(g0 + lane, ng - 1), k0 = g << gshift, k1 = min(k0 + G, ns);  // steps k0 .. k1-1
+      const int lo = X.s0 + (dirn ? ns - k1 : k0), hi = X.s0 + (dirn ? ns - k0 : k1);
+      const int r0 = __ldg(O.step_ptr + lo), r1 = __ldg(O.step_ptr + hi), b0 = r0 & ~3, nw = ((r1 + 3) & ~3) - b0;
+      const int rp0 = __ldg(O.rp_ptr + lo), nr = __ldg(O.rp_ptr + hi) - rp0;
+      const int p0 = __ldg(O.push_ptr[dirn] + lo), np = __ldg(O.push_ptr[dirn] + hi) - p0;
+      const int nf = blob_fields<T>(nc, dirn);
+      const unsigned S = X.stage + (unsigned)((g & (K - 1)) * L.bytes), mb = X.full + 8 * (g & (K - 1));
+      const unsigned nB = (16 + SZ * nf) * nr + 4 * np, nX = SZ * nr, nT = SZ * nc * nr, nQ = SZ * nw;
+      const unsigned char* const from = V.blob[dirn] + blob_offset<T>(rp0, p0, nf);
+      unsigned bytes = nB;
+      if (kSetup || kGS) bytes += nX;
+      if (MODE == OS_SETUP_DILU) bytes += nT;
+      if (!kSetup) bytes += nQ;
+      if (kE) bytes += nQ;
+      unsigned nU = 0;
+      const unsigned char* fromU = nullptr;
+      if constexpr (kGS) {
+        const int u0 = __ldg(O.push_ptr[1] + lo), nu = __ldg(O.push_ptr[1] + hi) - u0;
+        nU = (16 + SZ * blob_fields<T>(nc, 1)) * nr + 4 * nu;
+        fromU = V.blob[1] + blob_offset<T>(rp0, u0, blob_fields<T>(nc, 1));
+        bytes += nU;
+      }
+      const int turns = min(32, ng - g0);
+      for (int j = 0; j < turns && ok; ++j) {
+        if (lane == j) {
+          if (g >= K && !mbar_wait(X.empty + 8 * (g & (K - 1)), use_parity(g) ^ 1u, abort_flag)) {
+            fail();
+            ok = false;
+          } else {
+            if (tr) tr->staged(k0);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mbar_arrive_tx(mb, bytes);
+            bulk_g2s(S, from, nB, mb);
+            if (kSetup || kGS) bulk_g2s(S + L.oX, V.sx + rp0, nX, mb);
+            if (MODE == OS_SETUP_DILU) bulk_g2s(S + L.oT, V.tx + (size_t)rp0 * nc, nT, mb);
+            if constexpr (kGS) bulk_g2s(S + L.oU, fromU, nU, mb);
+            if (!kSetup) bulk_g2s(S + L.oQ, io.q + b0, nQ, mb);
+            if (kE) bulk_g2s(S + L.oE, io.e + b0, nQ, mb);
+            // the arrivals of the steps that the last group lacks
+            if (k1 - k0 < G) mbar_arrive(X.empty + 8 * (g & (K - 1)), (G - (k1 - k0)) * X.ncw);
+          }
+        }
+        ok = __shfl_sync(0xffffffffu, (int)ok, j) != 0;
+        issued += ok ? 1 : 0;
+      }
+    }
+    // after a failure, let the copies that nobody waits for land (bounded)
+    // before the block leaves
+    if (lane == 0 && *abort_flag)
+      for (int g = max(0, issued - K); g < issued; ++g) mbar_wait(X.full + 8 * (g & (K - 1)), use_parity(g), nullptr);
   }
+  __syncwarp();
+  // the values written here may be read by the next sweep's copies
+  asm volatile("fence.proxy.async;" ::: "memory");
   __syncthreads();
-  if (*((volatile int*)X.abort_flag)) {
-    // after an abort, let the copies of fills that were never consumed land
-    // (bounded) before the block leaves
-    if (threadIdx.x == (unsigned)nct)
-      for (int b = 0; b < K; ++b)
-        if ((X.used >> b) & 1u) mbar_wait(X.full + b, ((X.parity >> b) & 1u) ^ 1u);
-    __syncthreads();
-    return false;
+  // every group used its buffer once
+  {
+    const int ng = (ns + G - 1) >> gshift, rounds = ng >> kshift, rest = ng & (K - 1);
+    const unsigned all = (1u << K) - 1u, first = (1u << rest) - 1u;
+    Xr.parity = X.parity ^ first ^ (rounds & 1 ? all : 0u);
   }
+  if (MODE == OS_BWD_DOT || kGS) red_out[0] += red[0];
+  if (kGS) red_out[1] += red[1];
+  if (*abort_flag) return false;
   if (tr) tr->step(ns);
   return true;
 }
 
+template <class T, int MODE, class TracerT = NoTrace>
+__device__ __forceinline__ bool osweep(const GridCtl& C, const OrdView& O, const OrdVals<T>& V, const OsIO<T>& io,
+                                       OsCtx& X, double* red, TracerT* tr = nullptr) {
+  if (tr) tr->sweep();
+  if (vg_bid(C) >= O.ntiles) return true;
+  if (O.gen && O.nc == FC_ELL) return osweep_tile<T, MODE, FC_ELL, true, TracerT>(C, O, V, io, X, red, tr);
+  if (O.gen) return osweep_tile<T, MODE, 3, true, TracerT>(C, O, V, io, X, red, tr);
+  if (O.nc == FC_ELL) return osweep_tile<T, MODE, FC_ELL, false, TracerT>(C, O, V, io, X, red, tr);
+  return osweep_tile<T, MODE, 3, false, TracerT>(C, O, V, io, X, red, tr);
+}
+
 // ------------------------------------------------------ gather / scatter
 // Per-solve values in the new numbering from the caller's CSR values a
-// (original entry slots), exchange arrays filled with the sentinel.  Grid-
-// stride; the caller ends the phase with a grid barrier.
+// (original entry slots), exchange arrays filled with the sentinel.  The
+// blocks of the sweeps hold the plain coefficients of the lower triangle
+// afterwards (gs: of both triangles).  A warp per step, so that a field of
+// the step's rows is written in one piece; the caller ends the phase with a
+// grid barrier.
 template <class T>
 __device__ void ord_gather_values(const GridCtl& C, const OrdView& O, const OrdVals<T>& V, const T* __restrict__ a,
-                                  int nnz, bool dilu) {
-  const int gt = vg_gt(C), G = vg_G(C), n = O.n, nE = O.nE;
-  constexpr int VR = Rec<T>::V;
-  const T SENT = Sentinel<T>::value();
-  for (int q = gt; q < n; q += G) {
-    const T aii = __ldg(a + __ldg(O.dslot + q));
-    V.adiag[q] = aii;
-    T* sx = V.sx + (size_t)q * VR;
-    sx[0] = aii;
+                                  int nnz, bool dilu, bool gs) {
+  const int gt = vg_gt(C), G = vg_G(C), nc = O.nc, lane = threadIdx.x & 31;
+  for (int s = gt >> 5; s < O.nsteps; s += G >> 5) {
+    const int base = __ldg(O.step_ptr + s), cnt = __ldg(O.step_ptr + s + 1) - base, cp = (cnt + 3) & ~3;
+    const int rp = __ldg(O.rp_ptr + s);
+    T* cf[2];
     for (int d = 0; d < 2; ++d) {
-      T* vr = V.vrec[d] + (size_t)q * VR;
-#pragma unroll
-      for (int e = 0; e < FC_ELL; ++e) {
-        const int s = __ldg(O.slot[d] + (size_t)e * nE + q);
-        vr[e] = s >= 0 ? __ldg(a + s) : T(0);
-        if (d == 0) sx[1 + e] = (dilu && s >= 0) ? __ldg(a + __ldg(O.lo_tslot + (size_t)e * nE + q)) : T(0);
+      const int pp = __ldg(O.push_ptr[d] + s), np = __ldg(O.push_ptr[d] + s + 1) - pp;
+      cf[d] = (T*)(V.blob[d] + blob_offset<T>(rp, pp, blob_fields<T>(nc, d)) + 16 * cp + 4 * np);
+    }
+    T *sx = V.sx + rp, *tx = V.tx + (size_t)rp * nc;
+    for (int sl = lane; sl < cnt; sl += 32) {
+      const int q = base + sl, k0 = __ldg(O.p_ptr + q), ne = __ldg(&O.rec[0][q].w) & 255;
+      const T aii = __ldg(a + __ldg(O.p_slot + k0 + ne));
+      V.adiag[q] = aii;
+      sx[sl] = aii;
+      for (int e = 0; e < nc; ++e) {
+        cf[0][e * cp + sl] = e < ne ? __ldg(a + __ldg(O.p_slot + k0 + e)) : T(0);
+        if (dilu) tx[e * cp + sl] = e < ne ? __ldg(a + __ldg(O.lo_tslot + (size_t)e * O.nE + q)) : T(0);
+      }
+      if (gs) {
+        const int nu = __ldg(&O.rec[1][q].w) & 255;
+        for (int e = 0; e < nc; ++e) cf[1][e * cp + sl] = e < nu ? __ldg(a + __ldg(O.p_slot + k0 + ne + 1 + e)) : T(0);
       }
     }
   }
@@ -682,10 +786,57 @@ __device__ void ord_gather_values(const GridCtl& C, const OrdView& O, const OrdV
       V.aovf[d][o] = __ldg(a + __ldg(O.ovf_slot[d] + o));
       if (d == 0 && dilu) V.tovf[o] = __ldg(a + __ldg(O.lo_ovf_tslot + o));
     }
-    const int nx = __ldg(O.xv_ptr[d] + O.nsteps);
-    for (int p = gt; p < nx; p += G) V.xv[d][p] = SENT;
   }
   for (int k = gt; k < nnz; k += G) V.ap[k] = __ldg(a + __ldg(O.p_slot + k));
+}
+
+// exchange slots to the sentinel (every solve: an earlier one may have been cut short)
+template <class T>
+__device__ __forceinline__ void ord_reset_exchange(const GridCtl& C, const OrdView& O, const OrdVals<T>& V) {
+  for (int d = 0; d < 2; ++d) {
+    const int nx = __ldg(O.xv_ptr[d] + O.nsteps);
+    for (int p = vg_gt(C); p < nx; p += vg_G(C)) V.xv[d][p] = Sentinel<T>::value();
+  }
+}
+
+// The row values of the applications from the factors d (see the file
+// header).  Scaled: forward a_ij d_j, backward a_ij d_i and the factor
+// (d_i / (d_i + small)) d_i of the right-hand side.  Plain: d_i in both
+// directions, backward a_ij and 1/(d_i + small).  Once per setup; the caller
+// ends the phase with a grid barrier.
+template <class T>
+__device__ void ord_apply_values(const GridCtl& C, const OrdView& O, const OrdVals<T>& V, const T* d) {
+  const int gt = vg_gt(C), G = vg_G(C), nc = O.nc, lane = threadIdx.x & 31;
+  for (int s = gt >> 5; s < O.nsteps; s += G >> 5) {
+    const int base = __ldg(O.step_ptr + s), cnt = __ldg(O.step_ptr + s + 1) - base, cp = (cnt + 3) & ~3;
+    const int rp = __ldg(O.rp_ptr + s);
+    T* cf[2];
+    for (int r = 0; r < 2; ++r) {
+      const int pp = __ldg(O.push_ptr[r] + s), np = __ldg(O.push_ptr[r] + s + 1) - pp;
+      cf[r] = (T*)(V.blob[r] + blob_offset<T>(rp, pp, blob_fields<T>(nc, r)) + 16 * cp + 4 * np);
+    }
+    for (int sl = lane; sl < cnt; sl += 32) {
+      const int q = base + sl, k0 = __ldg(O.p_ptr + q);
+      const int ne = __ldg(&O.rec[0][q].w) & 255, nu = __ldg(&O.rec[1][q].w) & 255;
+      const T di = ldcg(d + q);
+      if constexpr (ScaledApply<T>::value) {
+        for (int e = 0; e < nc; ++e) {
+          cf[0][e * cp + sl] = e < ne ? ldcg(V.ap + k0 + e) * ldcg(d + __ldg(O.p_col + k0 + e)) : T(0);
+          cf[1][e * cp + sl] = e < nu ? ldcg(V.ap + k0 + ne + 1 + e) * di : T(0);
+        }
+        cf[1][nc * cp + sl] = di / (di + (T)FC_SMALL) * di;
+        for (int e = FC_ELL; e < ne; ++e)
+          V.aovf[0][__ldg(O.ovf_ptr[0] + q) + e - FC_ELL] = ldcg(V.ap + k0 + e) * ldcg(d + __ldg(O.p_col + k0 + e));
+        for (int e = FC_ELL; e < nu; ++e)
+          V.aovf[1][__ldg(O.ovf_ptr[1] + q) + e - FC_ELL] = ldcg(V.ap + k0 + ne + 1 + e) * di;
+      } else {
+        cf[0][nc * cp + sl] = di;
+        for (int e = 0; e < nc; ++e) cf[1][e * cp + sl] = e < nu ? ldcg(V.ap + k0 + ne + 1 + e) : T(0);
+        cf[1][nc * cp + sl] = di;
+        cf[1][(nc + 1) * cp + sl] = T(1) / (di + (T)FC_SMALL);
+      }
+    }
+  }
 }
 
 // y[q] = src[perm[q]] (into the new numbering) / dst[perm[q]] = y[q]

@@ -676,7 +676,7 @@ class Context:
         return dict(zip(keys, [float(v) for v in out]))
 
     def set_sweep_stage_rows(self, rows):
-        """Rows of a step held in the stage buffers in the pattern analyses that follow (0: the default)."""
+        """Most rows of a sweep step in the pattern analyses that follow (0: the default)."""
         self._check(self.L.fc_set_sweep_stage_rows(self.h, int(rows)), "fc_set_sweep_stage_rows")
 
     def set_sweep_tiles(self, tiles):
@@ -699,10 +699,11 @@ class Context:
     def trace(self, timeline=False):
         """Phase cycles of the last traced ICCG solve: (dict phase -> cycles
         summed over blocks, blocks); with timeline=True also the step stamps
-        as a uint64 array [sweep(fwd, bwd)][tile][step][8]: step start,
-        stage buffer landed, staging started (clock64), step start
-        (globaltimer), then thread 0's next-step loads issued, dependency
-        values ready, value computed, stores issued (clock64)."""
+        as a uint64 array [sweep(fwd, bwd)][tile][step][8]: start of the
+        step's loads, stage buffer landed, staging of the group started
+        (clock64), start of the loads (globaltimer), then the loads issued,
+        released by the previous step, value computed, stores issued
+        (clock64)."""
         out = np.zeros(11)
         self._check(self.L.fc_trace_get(self.h, _ptr(out), None), "fc_trace_get")
         keys = ("setup", "fwd_sweep", "sweep_barrier", "bwd_sweep", "dot", "p_update", "spmv", "xr_update")

@@ -508,7 +508,8 @@ static int split_wide_levels(int n, const int* ia, const int* ja, const int* dg,
 }
 
 bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, const int* ts, int ntiles,
-                         const double* xyz, int R, OrderedSweep& O, SweepSchedule& S, std::string& err, int wmax) {
+                         const double* xyz, int R, OrderedSweep& O, SweepSchedule& S, std::string& err, int wmax,
+                         int chunk) {
   O = OrderedSweep();
   O.n = n;
   O.R = std::max(2, R);
@@ -518,12 +519,12 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
   O.nlev = nlev;
   std::vector<int> code_tmp((size_t)ia[n], 0);
   build_sweep_schedule(n, ia, ja, dg, lev, nlev, true, ntiles, xyz, S, code_tmp);
-  // ---- new numbering: tile, step, slot order, empty slots dropped
+  // ---- new numbering: tile, step, slot order, empty slots dropped; a level
+  // wider than chunk rows takes several steps
   const int T = S.ntiles;
   O.ntiles = T;
-  O.nsteps = S.tile_step_ptr[T];
-  O.tile_step_ptr = S.tile_step_ptr;
-  O.step_ptr.assign(O.nsteps + 1, 0);
+  O.tile_step_ptr.assign(T + 1, 0);
+  O.step_ptr.reserve(S.tile_step_ptr[T] + 1);
   O.tile_W.assign(T, 1);
   O.perm.reserve(n);
   O.iperm.assign(n, -1);
@@ -533,25 +534,43 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
   std::vector<RowInfo> rinfo(n);
   std::vector<int> row_tile(n), row_ls(n);
   for (int t = 0; t < T; ++t) {
-    O.max_tile_steps = std::max(O.max_tile_steps, S.tile_step_ptr[t + 1] - S.tile_step_ptr[t]);
+    const int first = (int)O.step_ptr.size();
     for (int gs = S.tile_step_ptr[t]; gs < S.tile_step_ptr[t + 1]; ++gs) {
-      O.step_ptr[gs] = (int)O.perm.size();
-      int pos = 0;
+      O.step_ptr.push_back((int)O.perm.size());
+      int pos = 0, rows = 0;
       for (int q = S.step_row_ptr[gs]; q < S.step_row_ptr[gs + 1]; ++q) {
         const int i = S.rows[q];
         if (i < 0) continue;
+        if (chunk > 0 && pos == chunk) {
+          O.step_ptr.push_back((int)O.perm.size());
+          pos = 0;
+        }
         O.iperm[i] = (int)O.perm.size();
         O.perm.push_back(i);
         row_tile[i] = t;
-        row_ls[i] = gs - S.tile_step_ptr[t];
+        row_ls[i] = (int)O.step_ptr.size() - 1 - first;
         rinfo[i] = {O.iperm[i], t, row_ls[i], pos++};
+        ++rows;
+        O.tile_W[t] = std::max(O.tile_W[t], pos);
       }
-      O.tile_W[t] = std::max(O.tile_W[t], pos);
+      O.max_level_rows = std::max(O.max_level_rows, rows);
     }
+    O.tile_step_ptr[t + 1] = (int)O.step_ptr.size();
+    O.max_tile_steps = std::max(O.max_tile_steps, O.tile_step_ptr[t + 1] - O.tile_step_ptr[t]);
   }
-  O.step_ptr[O.nsteps] = (int)O.perm.size();
+  O.nsteps = (int)O.step_ptr.size();
+  O.step_ptr.push_back((int)O.perm.size());
+  O.rp_ptr.assign(O.nsteps + 1, 0);
+  for (int gs = 0; gs < O.nsteps; ++gs)
+    O.rp_ptr[gs + 1] = O.rp_ptr[gs] + ((O.step_ptr[gs + 1] - O.step_ptr[gs] + 3) & ~3);
   if ((int)O.perm.size() != n) { err = "ordered sweep: schedule does not cover every row once"; return false; }
   for (int t = 0; t < T; ++t) O.maxW = std::max(O.maxW, O.tile_W[t]);
+  if (chunk > 0) {
+    int per_level = 1;  // steps of the widest level, rounded up to a power of two
+    while (per_level * chunk < O.max_level_rows) per_level *= 2;
+    while (per_level > 1 && (long long)O.R * per_level * O.maxW * 8 > FC_RING_BYTES) per_level /= 2;
+    O.R *= per_level;
+  }
   const int nE = (n + 3) & ~3;
   O.nE = nE;
   const size_t E = (size_t)FC_ELL * nE;
@@ -566,6 +585,7 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
     D.slot.assign(E, -1);
     D.col.assign(E, 0);
     D.srec.assign((size_t)4 * nE, 0);
+    D.rec.assign((size_t)4 * nE, 0);
     D.ovf_ptr.assign(n + 1, 0);
     for (int q = 0; q < n; ++q) {
       const int i = O.perm[q];
@@ -584,7 +604,7 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
     std::vector<int> push_src, push_dst, push_m;
     for (int q = 0; q < n; ++q) {
       const int i = O.perm[q], t = row_tile[i];
-      const int nst = S.tile_step_ptr[t + 1] - S.tile_step_ptr[t];
+      const int nst = O.tile_step_ptr[t + 1] - O.tile_step_ptr[t];
       const int W = O.tile_W[t];
       const int my = dirn == 0 ? row_ls[i] : nst - 1 - row_ls[i];
       const int k0 = dirn == 0 ? ia[i] : dg[i] + 1;
@@ -640,8 +660,8 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
     std::vector<int>().swap(push_src);
     std::vector<int>().swap(push_dst);
     std::vector<int>().swap(push_m);
-    // exchange blocks (consumer side) and push blocks (producer side), one
-    // per step, each starting on a multiple of 4 elements
+    // exchange blocks (consumer side) and push blocks (producer side, copied
+    // in bulk: each starts on a multiple of 4 elements), one per step
     D.xv_ptr.assign(O.nsteps + 1, 0);
     D.push_ptr.assign(O.nsteps + 1, 0);
     std::vector<int> xoff(n, 0), poff(n, 0);
@@ -653,8 +673,8 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
         xs += nx[q];
         ps += cons_ptr[q + 1] - cons_ptr[q];
       }
-      if (xs > 65535 || ps > (1 << 30)) { derr = "ordered sweep: exchange block of a step too large"; return false; }
-      D.xv_ptr[gs + 1] = D.xv_ptr[gs] + ((xs + 3) & ~3);
+      if (xs > 65534 - O.R * O.maxW || ps > 65535) { derr = "ordered sweep: exchange block of a step too large"; return false; }
+      D.xv_ptr[gs + 1] = D.xv_ptr[gs] + xs;
       D.push_ptr[gs + 1] = D.push_ptr[gs] + ((ps + 3) & ~3);
     }
     D.push.assign(D.push_ptr[O.nsteps], 0);
@@ -663,6 +683,22 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
       if (nx[q] > 255 || np > 255) { derr = "ordered sweep: more than 255 exchanged entries in a row"; return false; }
       D.srec[4 * (size_t)q] = D.ne[q] | (np << 8) | (xoff[q] << 16);
       D.srec[4 * (size_t)q + 1] = poff[q];
+      {
+        const int rw = O.R * O.tile_W[row_tile[O.perm[q]]];
+        unsigned place[FC_ELL];
+        int mx = 0;
+        for (int e = 0; e < FC_ELL; ++e) {
+          const unsigned c1 = ((unsigned)D.srec[4 * (size_t)q + 2 + e / 2] >> (16 * (e & 1))) & 0xFFFFu;
+          if (c1 > 0) place[e] = c1 - 1;
+          else if (e < D.ne[q]) place[e] = rw + 1 + xoff[q] + mx++;
+          else place[e] = rw;
+        }
+        int* r = D.rec.data() + 4 * (size_t)q;
+        r[0] = np | (poff[q] << 8);
+        r[1] = (int)(place[0] | (place[1] << 16));
+        r[2] = (int)(place[2] | (place[3] << 16));
+        r[3] = D.ne[q] | (mx << 8) | (xoff[q] << 16);
+      }
       for (int m = 0; m < np; ++m) {
         const int qc = cons_q[cons_ptr[q] + m], mc = cons_m[cons_ptr[q] + m];
         D.push[D.push_ptr[row_step[q]] + poff[q] + m] = D.xv_ptr[row_step[qc]] + xoff[qc] + mc;
@@ -677,6 +713,8 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
   th1.join();
   if (!ok0) return false;
   if (!ok1) { err = err1; return false; }
+  for (int d = 0; d < 2; ++d)
+    for (int q = 0; q < n; ++q) O.max_entries = std::max(O.max_entries, O.dir[d].ne[q]);
   // ---- DILU transpose slots of the lower entries, diagonal slots, matrix
   O.lo_tslot.assign(E, 0);
   O.lo_ovf_tslot.assign(O.dir[0].ovf_ptr[n], 0);

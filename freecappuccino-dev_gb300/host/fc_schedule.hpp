@@ -69,10 +69,16 @@ double estimate_sweep_us(const SweepSchedule& S, double tau0, double per_row, do
 // index (local step % R) * W + position); every other dependency is pushed:
 // its producer stores the value into the consumer's own slot of an exchange
 // array xv.  The slots of a step's rows form one contiguous block of xv (in
-// row order, entries in CSR order), so the consumer fetches all values the
-// step needs with one copy; the producer's targets likewise form one block
-// per producing step.
+// row order, entries in CSR order); the producer's targets likewise form one
+// block per producing step.
+//
+// With chunk > 0 a level of a tile wider than chunk rows becomes several
+// consecutive steps of at most chunk rows (their rows are independent, so
+// the tiling, the levels and the values stay the same).  The dependencies of
+// a level then lie up to two levels' worth of steps back, so the ring gets
+// that many times its depth (as far as FC_RING_BYTES allows).
 #define FC_ELL 4
+#define FC_RING_BYTES (64 * 1024)  // most shared memory of a value ring deepened for chunked levels
 
 struct OrderedDir {
   std::vector<int> ne;        // [nE] entries of this triangle in the row
@@ -85,7 +91,14 @@ struct OrderedDir {
   //   [2], [3] codes of entries 0..3, 16 bits each, stored as code + 1
   //       (0: the value arrives through the exchange block)
   std::vector<int> srec;
-  std::vector<int> xv_ptr;    // [nsteps+1] exchange block of each step (multiples of 4)
+  // [4*nE] the same record as the kernels read it:
+  //   [0] np | poff << 8
+  //   [1], [2] places of the values of entries 0..3, 16 bits each: a ring
+  //       index (below R * W of the tile), R * W: a zero (past the row's
+  //       entries), R * W + 1 + j: value j of the step's exchange block
+  //   [3] ne | exchanged entries among 0..3 << 8 | xoff << 16
+  std::vector<int> rec;
+  std::vector<int> xv_ptr;    // [nsteps+1] exchange block of each step
   std::vector<int> push_ptr;  // [nsteps+1] push block of each step (multiples of 4)
   std::vector<int> push;      // absolute exchange positions the values are pushed to
   std::vector<int> ovf_ptr;   // [n+1] entries e >= FC_ELL
@@ -95,9 +108,12 @@ struct OrderedDir {
 
 struct OrderedSweep {
   int n = 0, nE = 0, ntiles = 0, nsteps = 0, nlev = 0, R = 4, maxW = 0, max_tile_steps = 0;
+  int max_level_rows = 0;          // rows of a tile in its widest level (maxW: in its widest step)
+  int max_entries = 0;             // entries of the fullest row of a triangle
   std::vector<int> perm, iperm;    // new -> old, old -> new
   std::vector<int> tile_step_ptr;  // [ntiles+1]
   std::vector<int> step_ptr;       // [nsteps+1] first new row of each step
+  std::vector<int> rp_ptr;         // [nsteps+1] the same with every step's rows padded to a multiple of 4
   std::vector<int> tile_W;         // widest step of each tile (ring / staging width)
   OrderedDir dir[2];               // 0: left of the diagonal (forward), 1: right (backward)
   std::vector<int> lo_tslot;       // [FC_ELL*nE] transpose slot of each lower entry (DILU)
@@ -119,10 +135,11 @@ int pick_sweep_tiles(int n, const int* ia, const int* ja, const int* dg, const d
 
 // ia, ja, dg 0-based; ts (optional) the transpose slot of every entry;
 // ntiles the tile target; xyz (optional) row coordinates for the tiling; R
-// the ring depth; wmax > 0 caps the rows of a step (a wider level of a tile
-// is split into consecutive steps, whose rows are independent).  S receives
-// the underlying tiled schedule (for the critical-path estimate).  Returns
-// false with a message if a consistency check fails.
+// the ring depth; wmax > 0 caps the rows of a level in a tile by splitting
+// levels (and cutting the tiles again); chunk > 0 caps the rows of a step as
+// described above.  S receives the underlying tiled schedule (for the
+// critical-path estimate).  Returns false with a message if a consistency
+// check fails.
 bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, const int* ts, int ntiles,
                          const double* xyz, int R, OrderedSweep& O, SweepSchedule& S, std::string& err,
-                         int wmax = 0);
+                         int wmax = 0, int chunk = 0);

@@ -195,20 +195,15 @@ int fc_spmv(fc_ctx* ctx, int n, int nnz, const int* ia, const int* ja, const dou
             const double* x, double* y, int transpose);
 /* Statistics of the schedule-ordered sweep structure of the mesh system
  * (which=0) or of the cached fc_csrsolve pattern (which=1): out[11] = tiles,
- * levels, widest step of a tile, ring depth, estimated forward-sweep us,
- * ring-served entries, pushed entries, cross-tile entries (both triangles),
- * stage depth, most steps of a tile, rows of a step held in the stage
- * buffers (0: whole steps; the further rows of a wider step are read from
- * global memory). */
+ * levels, most rows of a tile in one level, ring depth, estimated
+ * forward-sweep us, ring-served entries, pushed entries, cross-tile entries
+ * (both triangles), steps staged ahead, most steps of a tile, most rows of a
+ * step where a level of a tile has more (0: every level is one step). */
 int fc_sweep_stats(fc_ctx* ctx, int which, double* out);
-/* Caps the rows of a sweep step in the pattern analyses that follow (rows
- * >= 1; 0 restores the default).  A level of a tile wider than the cap is
- * split into consecutive steps; the preconditioner is unchanged.  By default
- * a level too wide for the shared-memory staging (e.g. on 6 million
- * tetrahedra) stays one step whose first rows are staged (see
- * fc_set_sweep_stage_rows), and the analysis splits levels by itself only
- * for batched systems or when too few rows would be staged.  Tuning and
- * testing only: no counterpart in the reference. */
+/* Caps the rows of a level in a tile in the pattern analyses that follow (rows
+ * >= 1; 0 restores the default, no cap).  A wider level is split into
+ * consecutive levels and the tiles are cut again; the preconditioner is
+ * unchanged.  Tuning and testing only: no counterpart in the reference. */
 int fc_set_sweep_cap(fc_ctx* ctx, int rows);
 /* Sets the tile count (thread blocks of the ordered sweeps, at most one per
  * SM) of the pattern analyses that follow; 0 restores the default, the
@@ -216,11 +211,11 @@ int fc_set_sweep_cap(fc_ctx* ctx, int rows);
  * preconditioner and the iterates do not depend on it.  Tuning and testing
  * only: no counterpart in the reference. */
 int fc_set_sweep_tiles(fc_ctx* ctx, int tiles);
-/* Sets the rows of a step that the stage buffers hold in the pattern
- * analyses that follow (0 restores the default: whole steps where they fit,
- * else as many rows as fit); the further rows of a wider step read their
- * records from global memory.  Results do not depend on it.  Tuning and
- * testing only: no counterpart in the reference. */
+/* Sets the most rows of a sweep step in the pattern analyses that follow, as
+ * far as that many fit the shared-memory staging (0 restores the default, one
+ * row per compute thread); a level of a tile with more rows takes several
+ * consecutive steps.  Results do not depend on it.  Tuning and testing only:
+ * no counterpart in the reference. */
 int fc_set_sweep_stage_rows(fc_ctx* ctx, int rows);
 /* Appends one JSON line per solve to the file at path (NULL or "": stop):
  * the entry point, solver, variable, rows, precision mode, status,
@@ -278,11 +273,12 @@ int fc_batch_tune(fc_batch* b, const char* solver, const double* const* a, const
  * barrier, backward sweep, dot product, p update, SpMV, x/r update; then the
  * blocks that ran, the blocks of the launch (B) and the stamps per tile (K);
  * timeline (optional, 2*B*K*8 entries) receives the stamps as
- * [sweep][tile][step][8]: the compute warps' start of the step, the moment
- * its staged data had landed, the staging thread's start of its copies
- * (clock64 of the tile's SM), the step start on the global timer, then
- * thread 0's next-step loads issued, its row's dependencies ready, its value
- * computed and its stores issued (clock64).  With
+ * [sweep][tile][step][8]: the start of the step's loads by its set of compute
+ * warps, the moment its staged data had landed, the staging thread's start of
+ * the copies of the step's group (first step of a group only; clock64 of the
+ * tile's SM), the start of the loads on the global timer, then the set's first
+ * thread's loads issued, its release by the previous step, its value computed
+ * and its stores issued (clock64).  With
  * tracing on, the multicolour inner solve of FC_PREC_MIXED_COLOURED launches
  * its kernels from the host instead of its CUDA graph, so that a profiler
  * sees each launch. */
