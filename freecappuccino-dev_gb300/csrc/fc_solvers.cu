@@ -609,11 +609,13 @@ __global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1)
 
 // ======================================================================== host
 // Critical-path model of a sweep schedule used to pick the tile count:
-// per step cost, per row cost and the delay of a value pushed to another
-// tile (its transfer plus the stage lead of the consumer), microseconds.
+// cost per step and per row and the delay of a value pushed to another tile,
+// microseconds.  Fitted to sweeps measured on 1 to 150 tiles of 1.3k to 2.1M
+// rows (forward and backward averaged): 35 rows a step take 0.17 us, 117 rows
+// 0.22 us, and every tile a dependency passes through adds 1.1 to 1.9 us.
 #define FC_SWEEP_TAU0_US 0.15
-#define FC_SWEEP_ROW_US 0.001
-#define FC_SWEEP_HOP_US 1.5
+#define FC_SWEEP_ROW_US 0.0006
+#define FC_SWEEP_HOP_US 1.2
 #define FC_RING 4                    // ring depth (levels) of the ordered sweeps
 // FP32 inner BiCGStab of the mixed modes: iterations without halving the
 // residual after which the inner solve ends (the longest such run in the
@@ -737,13 +739,13 @@ static int steps_per_buffer(const OrderedSweep& O, bool gs) {
   return 0;
 }
 
-static int upload_ordered(fc_ctx* ctx, const OrderedSweep& O, DevOrdered& D) {
+static int upload_ordered(fc_ctx* ctx, const OrderedSweep& O, DevOrdered& D, bool for_gs) {
   D.n = O.n; D.nE = O.nE; D.ntiles = O.ntiles; D.nsteps = O.nsteps; D.nlev = O.nlev; D.R = O.R; D.maxW = O.maxW;
   D.max_tile_steps = O.max_tile_steps; D.max_level_rows = O.max_level_rows; D.rp_total = O.rp_ptr.back();
   D.stage_area = ordered_stage_area(D.R, D.maxW);
   for (int gs = 0; gs < 2; ++gs) {
     DevOrdered::Groups& P = D.grp[gs];
-    P.G = steps_per_buffer(O, gs != 0);
+    P.G = gs && !for_gs ? 0 : steps_per_buffer(O, gs != 0);
     if (P.G == 0) continue;
     OrdView V;
     std::vector<int> desc[2];
@@ -845,13 +847,31 @@ int sys_set_pattern(fc_ctx* ctx, CsrSystem* s, int n, int nnz, const int* ia1, c
     return std::chrono::duration<double>(std::chrono::steady_clock::now() - a).count();
   };
   if (tiles_req <= 0 && ctx->sweep_tiles > 0) tiles_req = ctx->sweep_tiles;
+  int nocut = -1;  // axis the tiles are not cut along
   if (tiles_req > 0) {
     tiles = std::min(tiles_req, sms);
     s->est_sweep_us = 0.0;
   } else {
-    const std::vector<int> cand = {sms, (3 * sms) / 4, sms / 2, sms / 4};
+    // Candidates: counts p x p or p x (p+1), whose slabs are cut at the same
+    // places, from every SM downwards.  A tile of more than 40,000 rows takes
+    // at least 60 us, longer than the whole sweep on more tiles, and fewer than
+    // four rows of a level in a tile only add tiles to pass through: such
+    // counts are not tried.
+    std::vector<int> cand;
+    auto add = [&](int t) {
+      int p = 1;
+      while ((p + 1) * (p + 1) <= t) ++p;
+      const int c = p * (p + 1) <= t ? p * (p + 1) : p * p;
+      const bool large = (long long)n > 40000LL * c, narrow = (long long)n < 4LL * c * s->lf.nlev;
+      if (t >= 1 && !narrow && (!large || 2 * t > sms) && (cand.empty() || c < cand.back())) cand.push_back(c);
+    };
+    for (int t = sms; t >= 1; t /= 2) {
+      add(t);
+      add(3 * t / 4);
+    }
+    if (cand.empty()) cand.push_back(1);
     tiles = pick_sweep_tiles(n, ia.data(), ja.data(), dg.data(), xyz, cand, FC_SWEEP_TAU0_US, FC_SWEEP_ROW_US,
-                             FC_SWEEP_HOP_US, &s->est_sweep_us);
+                             FC_SWEEP_HOP_US, &s->est_sweep_us, &nocut);
   }
   s->t_tiling = since(t0);
   t0 = std::chrono::steady_clock::now();
@@ -862,11 +882,21 @@ int sys_set_pattern(fc_ctx* ctx, CsrSystem* s, int n, int nnz, const int* ia1, c
   // threads, or the forced width (tests); fewer where the solves' modes do not
   // get enough stage buffers
   int chunk = FC_SET_ROWS;
-  if (ctx->stage_rows > 0 && !(with_gs && ctx->stage_rows > FC_SET_ROWS)) chunk = ctx->stage_rows;
+  // A forced width of more rows than a set has threads leaves Gauss-Seidel
+  // out, whose first solve then analyses the pattern again (with_gs) with steps
+  // of half a set's threads.
+  const bool wide = ctx->stage_rows > FC_SET_ROWS;
+  if (ctx->stage_rows > 0) chunk = wide && with_gs ? FC_SET_ROWS / 2 : ctx->stage_rows;
   for (;;) {
     if (!build_ordered_sweep(n, ia.data(), ja.data(), dg.data(), ts.data(), tiles, xyz, FC_RING, O, S, err,
-                             ctx->sweep_cap, chunk))
+                             ctx->sweep_cap, chunk, nocut))
       return fc_fail_msg(ctx, FC_ERR_BAD_INPUT, err);
+    if (tiles_req > 0 && nocut < 0 && S.cut_axes == 3) {
+      // a given tile count: the axis to leave out is still chosen
+      pick_sweep_tiles(n, ia.data(), ja.data(), dg.data(), xyz, {tiles}, FC_SWEEP_TAU0_US, FC_SWEEP_ROW_US,
+                       FC_SWEEP_HOP_US, nullptr, &nocut);
+      if (nocut >= 0) continue;
+    }
     if (steps_per_buffer(O, false) > 0 && (!with_gs || steps_per_buffer(O, true) > 0)) break;
     if (chunk > FC_SET_ROWS) chunk = std::max(FC_SET_ROWS, (3 * chunk / 4) & ~31);
     else if (chunk > 32) chunk = 32;
@@ -874,7 +904,7 @@ int sys_set_pattern(fc_ctx* ctx, CsrSystem* s, int n, int nnz, const int* ia1, c
   }
   s->t_schedule = since(t0);
   s->xyz_src = xyz;
-  int st2 = upload_ordered(ctx, O, s->ord);
+  int st2 = upload_ordered(ctx, O, s->ord, with_gs || !wide);
 
   if (st2) return st2;
   s->o64.records = s->o32.records = false;

@@ -73,6 +73,7 @@
 #define FC_SET_WARPS 4
 #define FC_IMP_WARPS 3
 #define FC_SET_ROWS (32 * FC_SET_WARPS)
+static_assert(FC_SET_ROWS == FC_STEP_ROWS, "the schedule's cost model counts these steps");
 static_assert(FC_SWEEP_BLOCK == 32 * (FC_SETS * FC_SET_WARPS + FC_IMP_WARPS + 1), "warp roles fill the block");
 
 namespace fcdev {

@@ -3,6 +3,7 @@
 #include "fc_schedule.hpp"
 
 #include <algorithm>
+#include <cmath>
 #include <deque>
 #include <limits>
 #include <numeric>
@@ -21,64 +22,98 @@ struct Deps {
 
 }  // namespace
 
-// recursive coordinate bisection of items (chains) weighted by rows into
-// nparts parts; split along the axis of largest extent at the weighted
-// median.  The two halves of the first levels are cut concurrently (they
-// write disjoint entries of part_of).
-static void rcb(std::vector<int>& items, const std::vector<double>& cx, const std::vector<double>& cy,
-                const std::vector<double>& cz, const std::vector<int>& w, int nparts, int first_part,
-                std::vector<int>& part_of, int depth = 0) {
-  if (nparts <= 1 || items.size() <= 1) {
-    for (int c : items) part_of[c] = first_part;
+// Slabs along the axes for T nearly cubic cells.  ext: extents of the chain
+// centroids; an axis along which they hardly spread (the direction of the grid
+// lines) and axis nocut (>= 0) are not cut.  Returns the axes that are.
+static int cut_counts(int T, const double (&ext)[3], int nocut, int (&slabs)[3]) {
+  const double emax = std::max(ext[0], std::max(ext[1], ext[2]));
+  int axes[3], dims = 0;
+  double vol = 1.0;
+  for (int a = 0; a < 3; ++a) {
+    slabs[a] = 1;
+    if (a == nocut || !(ext[a] > 0.05 * emax)) continue;
+    vol *= ext[a];
+    axes[dims++] = a;
+  }
+  // the longest axes first; the last one takes what is left of T
+  std::stable_sort(axes, axes + dims, [&](int p, int q) { return ext[p] > ext[q]; });
+  int left = T, used = 0;
+  for (int l = 0; l < dims; ++l) {
+    const double side = std::pow(vol / left, 1.0 / (dims - l));  // of a cubic cell of what is left
+    const int want = l + 1 == dims ? left : (int)std::lround(ext[axes[l]] / side);
+    slabs[axes[l]] = std::max(1, std::min(left, want));
+    left = (left + slabs[axes[l]] - 1) / slabs[axes[l]];
+    vol /= ext[axes[l]];
+    used += slabs[axes[l]] > 1;
+  }
+  return used;
+}
+
+// Cuts items (chains) weighted by rows into T parts: slabs along axis ax[0],
+// each of them along ax[1], each of those along ax[2].  The parts are shared
+// out evenly over the slabs, whose weights follow.  A cut goes to the
+// position nearest to the balanced one, within half a slab, where the gap in
+// the coordinate is at least half the widest gap there, so that grid lines
+// sharing a coordinate stay on one side.  Slabs of a structured mesh with as
+// many parts are then cut at the same places: a dependency passes through as
+// few tiles one after the other as the counts allow, and the tiles have the
+// same number of lines to within one in each direction (bisecting the chains
+// over and over left tiles of 6,400 to 25,088 rows at 128^3, 37 of them one
+// after the other, where this leaves 12,288 to 14,976 rows and 23 tiles).
+// The slabs of the first axis are cut concurrently (they write disjoint
+// entries of part_of).
+static void axis_cuts(std::vector<int>& items, const std::vector<double>* const (&c)[3], const std::vector<int>& w,
+                      const int (&ax)[3], const int (&slabs)[3], int level, int T, int first_part,
+                      std::vector<int>& part_of) {
+  while (level < 3 && slabs[ax[level]] == 1) ++level;
+  if (level == 3 || T == 1) {
+    for (int i : items) part_of[i] = first_part;
     return;
   }
-  double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-  for (int c : items) {
-    const double p[3] = {cx[c], cy[c], cz[c]};
-    for (int a = 0; a < 3; ++a) { lo[a] = std::min(lo[a], p[a]); hi[a] = std::max(hi[a], p[a]); }
-  }
-  int ax = 0;
-  for (int a = 1; a < 3; ++a)
-    if (hi[a] - lo[a] > hi[ax] - lo[ax]) ax = a;
-  const std::vector<double>& key = ax == 0 ? cx : ax == 1 ? cy : cz;
-  // stable sort by the coordinate, on (key, item) pairs kept together
+  bool last = true;
+  for (int l = level + 1; l < 3; ++l) last = last && slabs[ax[l]] == 1;
+  const int np = last ? T : std::min(T, slabs[ax[level]]);
+  const std::vector<double>& key = *c[ax[level]];
   std::vector<std::pair<double, int>> kv(items.size());
   for (size_t q = 0; q < items.size(); ++q) kv[q] = {key[items[q]], items[q]};
   std::stable_sort(kv.begin(), kv.end(),
                    [](const std::pair<double, int>& a, const std::pair<double, int>& b) { return a.first < b.first; });
-  for (size_t q = 0; q < kv.size(); ++q) items[q] = kv[q].second;
-  const int nl = nparts / 2;
-  long long tot = 0;
-  for (int c : items) tot += w[c];
-  const long long want = tot * nl / nparts;
-  // cut at the widest coordinate gap among the positions whose left weight is
-  // within half a part of the balanced cut, so that grid lines sharing a
-  // coordinate stay on one side and the tile boundaries follow the mesh
-  const long long tol = std::max<long long>(1, tot / nparts / 2);
-  size_t cut = 0, best_near = 1;
-  double best_gap = -1.0;
-  long long acc = 0, best_dist = -1;
-  for (size_t q = 1; q < items.size(); ++q) {
-    acc += w[items[q - 1]];
-    const long long dist = acc > want ? acc - want : want - acc;
-    if (best_dist < 0 || dist < best_dist) { best_dist = dist; best_near = q; }
-    if (dist <= tol) {
-      const double gap = kv[q].first - kv[q - 1].first;
-      if (gap > best_gap) { best_gap = gap; cut = q; }
+  std::vector<long long> before(kv.size() + 1, 0);  // weight of the first q items
+  for (size_t q = 0; q < kv.size(); ++q) before[q + 1] = before[q] + w[kv[q].second];
+  const long long tot = before.back();
+  auto parts_before = [&](int s) { return (int)((long long)T * s / np); };  // parts of the first s slabs
+  std::vector<size_t> cut(np + 1, 0);
+  cut[np] = kv.size();
+  for (int s = 1; s < np; ++s) {
+    const long long want = tot * parts_before(s) / T, tol = std::max<long long>(1, tot / np / 2);
+    auto at = [&](long long x) { return (size_t)(std::lower_bound(before.begin(), before.end(), x) - before.begin()); };
+    const size_t lo = std::max(at(want - tol), cut[s - 1]), hi = std::min(at(want + tol), kv.size());
+    double widest = 0.0;
+    for (size_t q = std::max<size_t>(1, lo); q < hi; ++q) widest = std::max(widest, kv[q].first - kv[q - 1].first);
+    size_t best = std::max(at(want), cut[s - 1]);
+    long long best_dist = -1;
+    for (size_t q = std::max<size_t>(1, lo); q < hi; ++q) {
+      if (kv[q].first - kv[q - 1].first < 0.5 * widest) continue;
+      const long long dist = before[q] > want ? before[q] - want : want - before[q];
+      if (best_dist < 0 || dist < best_dist) { best_dist = dist; best = q; }
     }
+    cut[s] = best;
   }
-  if (cut == 0) cut = best_near;
-  cut = std::max<size_t>(1, std::min(cut, items.size() - 1));
-  std::vector<int> left(items.begin(), items.begin() + cut), right(items.begin() + cut, items.end());
+  std::vector<std::vector<int>> slab(np);
+  for (int s = 0; s < np; ++s)
+    for (size_t q = cut[s]; q < cut[s + 1]; ++q) slab[s].push_back(kv[q].second);
   kv.clear();
   kv.shrink_to_fit();
-  if (depth < 3 && items.size() > 4096) {
-    std::thread th([&]() { rcb(left, cx, cy, cz, w, nl, first_part, part_of, depth + 1); });
-    rcb(right, cx, cy, cz, w, nparts - nl, first_part + nl, part_of, depth + 1);
-    th.join();
+  auto run = [&](int s) {
+    const int p0 = parts_before(s);
+    axis_cuts(slab[s], c, w, ax, slabs, level + 1, parts_before(s + 1) - p0, first_part + p0, part_of);
+  };
+  if (!last && items.size() > 4096) {
+    std::vector<std::thread> th;
+    for (int s = 0; s < np; ++s) th.emplace_back(run, s);
+    for (std::thread& t : th) t.join();
   } else {
-    rcb(left, cx, cy, cz, w, nl, first_part, part_of, depth + 1);
-    rcb(right, cx, cy, cz, w, nparts - nl, first_part + nl, part_of, depth + 1);
+    for (int s = 0; s < np; ++s) run(s);
   }
 }
 
@@ -101,7 +136,7 @@ static void parallel_chunks(int n, F body) {
 
 void build_sweep_schedule(int n, const int* ia, const int* ja, const int* dg, const std::vector<int>& lev, int nlev,
                           bool forward, int ntiles_target, const double* xyz, SweepSchedule& S,
-                          std::vector<int>& code, bool with_waits) {
+                          std::vector<int>& code, bool with_waits, int nocut) {
   S = SweepSchedule();
   S.n = n;
   S.nlev = nlev;
@@ -163,7 +198,18 @@ void build_sweep_schedule(int n, const int* ia, const int* ja, const int* dg, co
     for (int c = 0; c < nch; ++c) { cx[c] /= chain_rows[c]; cy[c] /= chain_rows[c]; cz[c] /= chain_rows[c]; }
     std::vector<int> items(nch);
     std::iota(items.begin(), items.end(), 0);
-    rcb(items, cx, cy, cz, chain_rows, T, 0, tile_of_chain);
+    const std::vector<double>* const cen[3] = {&cx, &cy, &cz};
+    double ext[3];
+    for (int a = 0; a < 3; ++a) {
+      const auto mm = std::minmax_element(cen[a]->begin(), cen[a]->end());
+      ext[a] = *mm.second - *mm.first;
+    }
+    int slabs[3];
+    S.cut_axes = cut_counts(T, ext, nocut, slabs);
+    if (nocut == FC_CUT_UNLESS_3 && S.cut_axes == 3) return;
+    int ax[3] = {0, 1, 2};  // the longest axes first
+    std::stable_sort(ax, ax + 3, [&](int p, int q) { return ext[p] > ext[q]; });
+    axis_cuts(items, cen, chain_rows, ax, slabs, 0, T, 0, tile_of_chain);
     // drop empty parts
     std::vector<int> used(T, 0);
     for (int c = 0; c < nch; ++c) used[tile_of_chain[c]] = 1;
@@ -376,10 +422,10 @@ void build_sweep_schedule(int n, const int* ia, const int* ja, const int* dg, co
   }
 }
 
-// Critical-path estimate of a sweep: every step of a tile costs
-// tau0 + per_row * (rows in the step); a step starts when the tile's previous
-// step is done and, for each producer it waits on, hop microseconds after the
-// producer published the needed progress.  Returns microseconds.
+// Critical-path estimate of a sweep: every level of a tile costs tau0 per
+// FC_STEP_ROWS rows begun and per_row * rows; it starts when the tile's
+// previous level is done and, for each producer it waits on, hop microseconds
+// after the producer published the needed progress.  Returns microseconds.
 double estimate_sweep_us(const SweepSchedule& S, double tau0, double per_row, double hop) {
   std::vector<std::vector<double>> pub(S.ntiles);
   std::vector<int> cur(S.ntiles, 0);
@@ -409,7 +455,7 @@ double estimate_sweep_us(const SweepSchedule& S, double tau0, double per_row, do
     }
     int rowsn = 0;
     for (int sl = 0; sl < S.tile_slots[t]; ++sl) rowsn += S.rows[S.step_row_ptr[gs] + sl] >= 0;
-    const double end = st + tau0 + per_row * rowsn;
+    const double end = st + tau0 * ((rowsn + FC_STEP_ROWS - 1) / FC_STEP_ROWS) + per_row * rowsn;
     pub[t].push_back(end);
     tmax = std::max(tmax, end);
   }
@@ -418,31 +464,44 @@ double estimate_sweep_us(const SweepSchedule& S, double tau0, double per_row, do
 
 // ---------------------------------------------------------------------------
 int pick_sweep_tiles(int n, const int* ia, const int* ja, const int* dg, const double* xyz, const std::vector<int>& cand,
-                     double tau0, double per_row, double hop, double* best_est) {
+                     double tau0, double per_row, double hop, double* best_est, int* nocut) {
   std::vector<int> lev;
   const int nls = symmetric_levels(n, ia, ja, dg, lev);
   const int nc = (int)cand.size();
-  std::vector<double> est(nc, 1e300);
-  auto trial = [&](int c) {
-    std::vector<int> code(ia[n], 0);
-    SweepSchedule S;
-    build_sweep_schedule(n, ia, ja, dg, lev, nls, true, cand[c], xyz, S, code);
-    est[c] = estimate_sweep_us(S, tau0, per_row, hop);
+  struct Trial { int c, out; double est; bool cut3; };
+  auto run = [&](std::vector<Trial>& tr) {
+    auto one = [&](Trial& t) {
+      std::vector<int> code(ia[n], 0);
+      SweepSchedule S;
+      build_sweep_schedule(n, ia, ja, dg, lev, nls, true, cand[t.c], xyz, S, code, true, t.out);
+      t.cut3 = S.cut_axes == 3;
+      if (S.ntiles > 0) t.est = estimate_sweep_us(S, tau0, per_row, hop);
+    };
+    std::vector<std::thread> th;
+    for (Trial& t : tr) th.emplace_back([&one, &t]() { one(t); });
+    for (std::thread& t : th) t.join();
   };
-  std::vector<std::thread> th;
-  for (int c = 0; c < nc; ++c) {
-    if (cand[c] < 1) continue;
-    bool dup = false;
-    for (int d = 0; d < c; ++d) dup = dup || cand[d] == cand[c];
-    if (dup) continue;
-    th.emplace_back(trial, c);
-  }
-  for (std::thread& t : th) t.join();
-  int best = -1;
+  std::vector<int> counts;  // candidates to try, without duplicates
   for (int c = 0; c < nc; ++c)
-    if (best < 0 || est[c] < est[best]) best = c;
-  if (best_est) *best_est = best >= 0 ? est[best] : 0.0;
-  return best >= 0 && est[best] < 1e300 ? cand[best] : (nc ? std::max(1, cand[0]) : 1);
+    if (cand[c] >= 1 && std::find(cand.begin(), cand.begin() + c, cand[c]) == cand.begin() + c) counts.push_back(c);
+  std::vector<Trial> tr;
+  for (int c : counts) tr.push_back({c, nocut ? FC_CUT_UNLESS_3 : -1, 1e300, false});
+  run(tr);
+  if (nocut && std::any_of(tr.begin(), tr.end(), [](const Trial& t) { return t.cut3; })) {
+    // the trials that would have cut all three axes stopped there
+    std::vector<Trial> more;
+    for (size_t k = 0; k < counts.size(); k += 2)
+      for (int out = 0; out < 3; ++out) more.push_back({counts[k], out, 1e300, false});
+    for (size_t k = 0; k < counts.size() && k < 2; ++k) more.push_back({counts[k], -1, 1e300, false});
+    run(more);
+    tr.insert(tr.end(), more.begin(), more.end());
+  }
+  const Trial* best = nullptr;
+  for (const Trial& t : tr)
+    if (!best || t.est < best->est) best = &t;
+  if (nocut) *nocut = best && best->out >= 0 ? best->out : -1;
+  if (best_est) *best_est = best ? best->est : 0.0;
+  return best && best->est < 1e300 ? cand[best->c] : (nc ? std::max(1, cand[0]) : 1);
 }
 
 int symmetric_levels(int n, const int* ia, const int* ja, const int* dg, std::vector<int>& lev) {
@@ -466,11 +525,11 @@ int symmetric_levels(int n, const int* ia, const int* ja, const int* dg, std::ve
 // tiles), so the split is repeated until no step is wider than wmax (a few
 // passes).  Returns the number of levels.
 static int split_wide_levels(int n, const int* ia, const int* ja, const int* dg, int ntiles, const double* xyz,
-                             int wmax, std::vector<int>& lev, int nlev) {
+                             int wmax, std::vector<int>& lev, int nlev, int nocut) {
   std::vector<int> code_tmp;  // not written by a layout-only build
   for (int pass = 0; pass < 8; ++pass) {
     SweepSchedule T;
-    build_sweep_schedule(n, ia, ja, dg, lev, nlev, true, ntiles, xyz, T, code_tmp, false);
+    build_sweep_schedule(n, ia, ja, dg, lev, nlev, true, ntiles, xyz, T, code_tmp, false, nocut);
     std::vector<int> chunk(n, 0);
     int maxc = 0;
     const int nsteps = T.tile_step_ptr[T.ntiles];
@@ -509,16 +568,16 @@ static int split_wide_levels(int n, const int* ia, const int* ja, const int* dg,
 
 bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, const int* ts, int ntiles,
                          const double* xyz, int R, OrderedSweep& O, SweepSchedule& S, std::string& err, int wmax,
-                         int chunk) {
+                         int chunk, int nocut) {
   O = OrderedSweep();
   O.n = n;
   O.R = std::max(2, R);
   std::vector<int> lev;
   int nlev = symmetric_levels(n, ia, ja, dg, lev);
-  if (wmax > 0) nlev = split_wide_levels(n, ia, ja, dg, ntiles, xyz, wmax, lev, nlev);
+  if (wmax > 0) nlev = split_wide_levels(n, ia, ja, dg, ntiles, xyz, wmax, lev, nlev, nocut);
   O.nlev = nlev;
   std::vector<int> code_tmp((size_t)ia[n], 0);
-  build_sweep_schedule(n, ia, ja, dg, lev, nlev, true, ntiles, xyz, S, code_tmp);
+  build_sweep_schedule(n, ia, ja, dg, lev, nlev, true, ntiles, xyz, S, code_tmp, true, nocut);
   // ---- new numbering: tile, step, slot order, empty slots dropped; a level
   // wider than chunk rows takes several steps
   const int T = S.ntiles;

@@ -4,8 +4,9 @@
 // The rows are cut into dependency chains (each row continues the chain of
 // its most recent dependency, so on a naturally ordered structured mesh the
 // chains are the grid lines along the fastest index), the chains are grouped
-// into tiles of about n/T rows by growing regions over the chain graph, and
-// every tile is given to one thread block.  A block walks its rows level by
+// into tiles of about n/T rows by cuts along the axes (or, without
+// coordinates, by growing regions over the chain graph), and every tile is
+// given to one thread block.  A block walks its rows level by
 // level: rows of one level are independent, values produced inside the tile
 // in the last R steps are read from a shared-memory ring, everything else
 // from global memory after the producing tile has published enough progress.
@@ -19,6 +20,7 @@ struct SweepSchedule {
   int nlev = 0;                    // levels of the sweep (0..nlev-1)
   int R = 4;                       // shared-memory ring depth in steps
   int max_slots = 0;               // widest tile (rows of one tile in one level)
+  int cut_axes = 0;                // axes that the tiles were cut along
   std::vector<int> tile_step_ptr;  // tile t owns global steps [ptr[t], ptr[t+1])
   std::vector<int> step_level;     // level of each global step
   std::vector<int> tile_slots;     // rows per step (padded width) of each tile
@@ -37,18 +39,23 @@ struct SweepSchedule {
 // every row for the direction (forward: from the lower part, backward: from
 // the upper part); code must have nnz entries (shared between directions).
 // xyz (optional, 3*n: x,y,z of every row, e.g. the cell centroids) lets the
-// tiles be cut by recursive coordinate bisection of the chain centroids:
-// dependencies along the mesh then run one way between tiles, so tiles
-// pipeline instead of waiting on each other at every level.  Without
+// tiles be cut along the axes by the chain centroids: dependencies along the
+// mesh then run one way between tiles, so tiles pipeline instead of waiting
+// on each other at every level.  Without
 // coordinates the tiles are grown over the chain graph.  with_waits false
 // stops after the layout (tiles, steps, rows): code, the waits and the entry
-// counts are left empty.
+// counts are left empty.  nocut: an axis (0, 1, 2) not to cut along, -1: none,
+// FC_CUT_UNLESS_3: none, and where all three axes would be cut S.cut_axes alone
+// is filled in.
+#define FC_CUT_UNLESS_3 (-2)
 void build_sweep_schedule(int n, const int* ia, const int* ja, const int* dg, const std::vector<int>& lev, int nlev,
                           bool forward, int ntiles, const double* xyz, SweepSchedule& S, std::vector<int>& code,
-                          bool with_waits = true);
+                          bool with_waits = true, int nocut = -1);
 
-// Critical-path estimate (microseconds) of a schedule: per step tau0 +
-// per_row * rows, cross-tile waits delayed by hop after publication.
+// Critical-path estimate (microseconds) of a schedule: per level of a tile
+// tau0 per FC_STEP_ROWS rows begun + per_row * rows, cross-tile waits delayed
+// by hop after publication.
+#define FC_STEP_ROWS 128  // rows of a step of the sweeps (fc_sweep.cuh)
 double estimate_sweep_us(const SweepSchedule& S, double tau0, double per_row, double hop);
 
 // ---------------------------------------------------------------------------
@@ -129,17 +136,23 @@ int symmetric_levels(int n, const int* ia, const int* ja, const int* dg, std::ve
 // The tile count among cand whose forward schedule has the smallest
 // critical-path estimate (the trials are built concurrently, one thread
 // each; ties go to the earlier candidate, duplicates and counts < 1 are
-// skipped).  best_est (optional) receives that estimate.
+// skipped).  best_est (optional) receives that estimate.  With nocut, and
+// where the chains spread along all three axes, every second count is tried
+// with each axis left out of the cuts (and the first two with all of them), and *nocut
+// receives the best one (-1: none): on tetrahedra a cut along one of the axes can separate chains that
+// depend on each other both ways, which makes the tiles wait for each other
+// at every level (750k tetrahedra, 150 tiles: 250 such pairs of tiles and an
+// estimate of 152 us with all axes cut, none and 55 us without one of them).
 int pick_sweep_tiles(int n, const int* ia, const int* ja, const int* dg, const double* xyz, const std::vector<int>& cand,
-                     double tau0, double per_row, double hop, double* best_est);
+                     double tau0, double per_row, double hop, double* best_est, int* nocut = nullptr);
 
 // ia, ja, dg 0-based; ts (optional) the transpose slot of every entry;
 // ntiles the tile target; xyz (optional) row coordinates for the tiling; R
 // the ring depth; wmax > 0 caps the rows of a level in a tile by splitting
 // levels (and cutting the tiles again); chunk > 0 caps the rows of a step as
-// described above.  S receives the underlying tiled schedule (for the
+// described above; nocut as above.  S receives the underlying tiled schedule (for the
 // critical-path estimate).  Returns false with a message if a consistency
 // check fails.
 bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, const int* ts, int ntiles,
                          const double* xyz, int R, OrderedSweep& O, SweepSchedule& S, std::string& err,
-                         int wmax = 0, int chunk = 0);
+                         int wmax = 0, int chunk = 0, int nocut = -1);
