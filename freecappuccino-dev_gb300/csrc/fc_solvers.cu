@@ -884,9 +884,9 @@ int sys_set_pattern(fc_ctx* ctx, CsrSystem* s, int n, int nnz, const int* ia1, c
   int chunk = FC_SET_ROWS;
   // A forced width of more rows than a set has threads leaves Gauss-Seidel
   // out, whose first solve then analyses the pattern again (with_gs) with steps
-  // of half a set's threads.
+  // of one warp's rows.
   const bool wide = ctx->stage_rows > FC_SET_ROWS;
-  if (ctx->stage_rows > 0) chunk = wide && with_gs ? FC_SET_ROWS / 2 : ctx->stage_rows;
+  if (ctx->stage_rows > 0) chunk = wide && with_gs ? 32 : ctx->stage_rows;
   for (;;) {
     if (!build_ordered_sweep(n, ia.data(), ja.data(), dg.data(), ts.data(), tiles, xyz, FC_RING, O, S, err,
                              ctx->sweep_cap, chunk, nocut))
