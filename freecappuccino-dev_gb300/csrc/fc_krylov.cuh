@@ -29,9 +29,10 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
 __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ unsigned atom_add_acqrel_u32(unsigned* p, unsigned v) {
+// p = p >= limit ? 0 : p + 1; returns the old value
+__device__ __forceinline__ unsigned atom_inc_acqrel_u32(unsigned* p, unsigned limit) {
   unsigned old;
-  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(limit) : "memory");
   return old;
 }
 
@@ -44,32 +45,31 @@ __device__ __forceinline__ int vg_nb(const GridCtl& C) { return C.nb > 0 ? C.nb 
 __device__ __forceinline__ int vg_gt(const GridCtl& C) { return vg_bid(C) * (int)blockDim.x + (int)threadIdx.x; }
 __device__ __forceinline__ int vg_G(const GridCtl& C) { return vg_nb(C) * (int)blockDim.x; }
 
-// Generation barrier over all blocks of the (cooperative) grid or group.  Returns
-// false if the wait ran out or another block already failed; the caller then
-// leaves the kernel.
+// Barrier over all blocks of the (cooperative) grid or group.  Returns false
+// if the wait ran out or another block already failed; the caller then leaves
+// the kernel.  One counter: the arrivals of a round take it from a multiple of
+// nb to the next (it wraps at a multiple, so the difference to the round's
+// start tells).  A block arrives and polls with one atomic and then loads of
+// one word; a separate generation word, read before the arrival, and fences
+// around the acquire-release operations cost another round trip each
+// (2.8 us a barrier with 152 blocks, now 1.3).  The counter is zeroed before
+// the launch.
 __device__ __forceinline__ bool grid_sync(const GridCtl& C) {
   __shared__ int s_ok;
   __syncthreads();
+  const unsigned nb = (unsigned)vg_nb(C);
+  if (nb == 1) return true;
   if (threadIdx.x == 0) {
     int ok = 1;
-    __threadfence();
-    unsigned gen = ld_acquire_u32(C.bar + 1);
-    unsigned arrived = atom_add_acqrel_u32(C.bar, 1u);
-    if (arrived == (unsigned)vg_nb(C) - 1u) {
-      atomicExch(C.bar, 0u);
-      st_release_u32(C.bar + 1, gen + 1u);
-    } else {
-      unsigned spins = 0;
-      while (ld_acquire_u32(C.bar + 1) == gen) {
-        if (++spins > FC_SPIN_LIMIT || *((volatile int*)C.status) != 0) {
-          atomicCAS(C.status, 0, FC_ERR_TIMEOUT);
-          ok = 0;
-          break;
-        }
-        __nanosleep(32);
+    const unsigned old = atom_inc_acqrel_u32(C.bar, nb * (1u << 16) - 1u), start = old - old % nb;
+    unsigned spins = 0;
+    while (ld_acquire_u32(C.bar) - start < nb) {
+      if (++spins > FC_SPIN_LIMIT || ((spins & 63u) == 0 && *((volatile int*)C.status) != 0)) {
+        atomicCAS(C.status, 0, FC_ERR_TIMEOUT);
+        ok = 0;
+        break;
       }
     }
-    __threadfence();
     s_ok = ok;
   }
   __syncthreads();
@@ -82,46 +82,60 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Sum NV values over the grid.  Deterministic: each block reduces in a fixed
-// tree and writes one partial per value; after the barrier every block sums
+// Sum NV values over the grid.  Deterministic: each block sums in a fixed
+// order and writes one partial per value; after the barrier every block sums
 // the partials in the same fixed order, so all blocks hold identical totals.
 // Partials alternate between two slot sets (ph), so a block still reading
 // the previous reduction never sees slots of the next one being rewritten.
+//
+// A block's threads leave their values in shared memory and one warp per value
+// sums them, four chains a lane, then a tree: the FP64 pipe takes a warp's
+// addition each ~17 cycles, and a shuffle tree in each of 20 warps was 100
+// of them per value (2 values on 152 blocks: 5.8 us with the trees, now 3.4;
+// the barrier alone 1.3).
+__device__ __forceinline__ double* red_buf() {
+  __shared__ double sm[FC_NPART * FC_SWEEP_BLOCK];
+  return sm;
+}
 template <int NV>
 __device__ __forceinline__ bool grid_reduce(const GridCtl& C, int& ph, double (&v)[NV]) {
-  __shared__ double sm[NV][32];
+  static_assert(NV <= FC_NPART, "partial slots");
   __shared__ double tot[NV];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, j = tid >> 5, bd = blockDim.x;
   const int nb = vg_nb(C), bid = vg_bid(C);
+  double* sm = red_buf();
   double* part = C.part + (size_t)(ph & 1) * FC_NPART * nb;
   ++ph;
 #pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    double s = warp_sum(v[j]);
-    if (lane == 0) sm[j][wid] = s;
-  }
+  for (int k = 0; k < NV; ++k) sm[k * bd + tid] = v[k];
   __syncthreads();
-  if (wid == 0) {
+  if (j < NV) {
+    double e[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int t = lane; t < bd; t += 128)
 #pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      double s = lane < nw ? sm[j][lane] : 0.0;
-      s = warp_sum(s);
-      if (lane == 0) part[j * nb + bid] = s;
+      for (int k = 0; k < 4; ++k)
+        if (t + 32 * k < bd) e[k] += sm[j * bd + t + 32 * k];
+    const double s = warp_sum((e[0] + e[1]) + (e[2] + e[3]));
+    if (lane == 0) {
+      if (nb == 1) tot[j] = s;
+      else part[j * nb + bid] = s;
     }
   }
-  if (!grid_sync(C)) return false;
-  if (wid == 0) {
+  if (nb > 1) {
+    if (!grid_sync(C)) return false;
+    if (j < NV) {
+      double e[5];
 #pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      double s = 0.0;
-      for (int b = lane; b < nb; b += 32) s += __ldcg(part + j * nb + b);
+      for (int k = 0; k < 5; ++k) e[k] = lane + 32 * k < nb ? __ldcg(part + j * nb + lane + 32 * k) : 0.0;
+      double s = ((e[0] + e[1]) + (e[2] + e[3])) + e[4];
+      for (int b = lane + 160; b < nb; b += 32) s += __ldcg(part + j * nb + b);
       s = warp_sum(s);
       if (lane == 0) tot[j] = s;
     }
   }
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < NV; ++j) v[j] = tot[j];
+  for (int k = 0; k < NV; ++k) v[k] = tot[k];
   return true;
 }
 

@@ -204,10 +204,17 @@ struct OrdView {
   const int* __restrict__ ovf_slot[2];
   const int* __restrict__ lo_tslot;
   const int* __restrict__ lo_ovf_tslot;
-  const int* __restrict__ p_ptr;
-  const int* __restrict__ p_col;
-  const int* __restrict__ p_slot;
+  // the matrix in slices of FC_SLICE rows: entry k (in the row's original
+  // order) of row q at sell_ptr[q / FC_SLICE] + k FC_SLICE + q % FC_SLICE,
+  // column and original slot -1 past the row's entries
+  const int* __restrict__ sell_ptr;
+  const int* __restrict__ sell_col;
+  const int* __restrict__ sell_slot;
 };
+#define FC_SLICE 32
+__device__ __forceinline__ int sell_at(const OrdView& O, int q, int k) {
+  return __ldg(O.sell_ptr + q / FC_SLICE) + k * FC_SLICE + q % FC_SLICE;
+}
 
 // Per-solve values in the new numbering (gathered by the kernel from the
 // caller's CSR values) and the exchange arrays; every vector of n rows is
@@ -232,7 +239,7 @@ struct OrdVals {
   T* aovf[2];  // coefficients of the overflow entries
   T* tovf;     // DILU transposes of the lower overflow entries
   T* adiag;    // [nE]
-  T* ap;       // [nnz] matrix values in new row order (original entry order)
+  T* ap;       // matrix values in the slices of OrdView (0 past a row's entries)
   T* xv[2];    // exchange arrays (per-step blocks)
 };
 
@@ -457,10 +464,10 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
             const int s = X.s0 + k, p1 = __ldg(O.push_ptr[1] + s), p0 = __ldg(O.push_ptr[1] + X.s0 + (k & ~(G - 1)));
             const unsigned U = S + L.oU + (unsigned)(rpo * (kStride + SZ * blob_fields<T>(nc, 1)) + 4 * (p1 - p0));
             const unsigned UC = U + kStride * cp + 4 * (__ldg(O.push_ptr[1] + s + 1) - p1);
-            const int nu = lds(U + kStride * sl + 12, int()) & 255, k0 = __ldg(O.p_ptr + base + sl) + (w.ovf & 255) + 1;
+            const int nu = lds(U + kStride * sl + 12, int()) & 255, k0 = sell_at(O, base + sl, (w.ovf & 255) + 1);
 #pragma unroll
             for (int e = 0; e < NC; ++e)
-              w.x[e] = e < nu ? mul_rn(lds(UC + (unsigned)((e * cp + sl) * SZ), T()), ldcg(io.e + __ldg(O.p_col + k0 + e)))
+              w.x[e] = e < nu ? mul_rn(lds(UC + (unsigned)((e * cp + sl) * SZ), T()), ldcg(io.e + __ldg(O.sell_col + k0 + FC_SLICE * e)))
                               : T(0);
           } else {
             w.acc = lds(S + L.oQ + (woff + sl) * SZ, T());
@@ -755,7 +762,7 @@ __device__ __forceinline__ bool osweep(const GridCtl& C, const OrdView& O, const
 // grid barrier.
 template <class T>
 __device__ void ord_gather_values(const GridCtl& C, const OrdView& O, const OrdVals<T>& V, const T* __restrict__ a,
-                                  int nnz, bool dilu, bool gs) {
+                                  bool dilu, bool gs) {
   const int gt = vg_gt(C), G = vg_G(C), nc = O.nc, lane = threadIdx.x & 31;
   for (int s = gt >> 5; s < O.nsteps; s += G >> 5) {
     const int base = __ldg(O.step_ptr + s), cnt = __ldg(O.step_ptr + s + 1) - base, cp = (cnt + 3) & ~3;
@@ -767,17 +774,18 @@ __device__ void ord_gather_values(const GridCtl& C, const OrdView& O, const OrdV
     }
     T *sx = V.sx + rp, *tx = V.tx + (size_t)rp * nc;
     for (int sl = lane; sl < cnt; sl += 32) {
-      const int q = base + sl, k0 = __ldg(O.p_ptr + q), ne = __ldg(&O.rec[0][q].w) & 255;
-      const T aii = __ldg(a + __ldg(O.p_slot + k0 + ne));
+      const int q = base + sl, k0 = sell_at(O, q, 0), ne = __ldg(&O.rec[0][q].w) & 255;
+      auto entry = [&](int k) { return __ldg(a + __ldg(O.sell_slot + k0 + FC_SLICE * k)); };
+      const T aii = entry(ne);
       V.adiag[q] = aii;
       sx[sl] = aii;
       for (int e = 0; e < nc; ++e) {
-        cf[0][e * cp + sl] = e < ne ? __ldg(a + __ldg(O.p_slot + k0 + e)) : T(0);
+        cf[0][e * cp + sl] = e < ne ? entry(e) : T(0);
         if (dilu) tx[e * cp + sl] = e < ne ? __ldg(a + __ldg(O.lo_tslot + (size_t)e * O.nE + q)) : T(0);
       }
       if (gs) {
         const int nu = __ldg(&O.rec[1][q].w) & 255;
-        for (int e = 0; e < nc; ++e) cf[1][e * cp + sl] = e < nu ? __ldg(a + __ldg(O.p_slot + k0 + ne + 1 + e)) : T(0);
+        for (int e = 0; e < nc; ++e) cf[1][e * cp + sl] = e < nu ? entry(ne + 1 + e) : T(0);
       }
     }
   }
@@ -788,7 +796,11 @@ __device__ void ord_gather_values(const GridCtl& C, const OrdView& O, const OrdV
       if (d == 0 && dilu) V.tovf[o] = __ldg(a + __ldg(O.lo_ovf_tslot + o));
     }
   }
-  for (int k = gt; k < nnz; k += G) V.ap[k] = __ldg(a + __ldg(O.p_slot + k));
+  const int nsell = __ldg(O.sell_ptr + (O.n + FC_SLICE - 1) / FC_SLICE);
+  for (int k = gt; k < nsell; k += G) {
+    const int slot = __ldg(O.sell_slot + k);
+    V.ap[k] = slot >= 0 ? __ldg(a + slot) : T(0);
+  }
 }
 
 // exchange slots to the sentinel (every solve: an earlier one may have been cut short)
@@ -817,22 +829,24 @@ __device__ void ord_apply_values(const GridCtl& C, const OrdView& O, const OrdVa
       cf[r] = (T*)(V.blob[r] + blob_offset<T>(rp, pp, blob_fields<T>(nc, r)) + 16 * cp + 4 * np);
     }
     for (int sl = lane; sl < cnt; sl += 32) {
-      const int q = base + sl, k0 = __ldg(O.p_ptr + q);
+      const int q = base + sl, k0 = sell_at(O, q, 0);
+      auto entry = [&](int k) { return ldcg(V.ap + k0 + FC_SLICE * k); };
+      auto column = [&](int k) { return __ldg(O.sell_col + k0 + FC_SLICE * k); };
       const int ne = __ldg(&O.rec[0][q].w) & 255, nu = __ldg(&O.rec[1][q].w) & 255;
       const T di = ldcg(d + q);
       if constexpr (ScaledApply<T>::value) {
         for (int e = 0; e < nc; ++e) {
-          cf[0][e * cp + sl] = e < ne ? ldcg(V.ap + k0 + e) * ldcg(d + __ldg(O.p_col + k0 + e)) : T(0);
-          cf[1][e * cp + sl] = e < nu ? ldcg(V.ap + k0 + ne + 1 + e) * di : T(0);
+          cf[0][e * cp + sl] = e < ne ? entry(e) * ldcg(d + column(e)) : T(0);
+          cf[1][e * cp + sl] = e < nu ? entry(ne + 1 + e) * di : T(0);
         }
         cf[1][nc * cp + sl] = di / (di + (T)FC_SMALL) * di;
         for (int e = FC_ELL; e < ne; ++e)
-          V.aovf[0][__ldg(O.ovf_ptr[0] + q) + e - FC_ELL] = ldcg(V.ap + k0 + e) * ldcg(d + __ldg(O.p_col + k0 + e));
+          V.aovf[0][__ldg(O.ovf_ptr[0] + q) + e - FC_ELL] = entry(e) * ldcg(d + column(e));
         for (int e = FC_ELL; e < nu; ++e)
-          V.aovf[1][__ldg(O.ovf_ptr[1] + q) + e - FC_ELL] = ldcg(V.ap + k0 + ne + 1 + e) * di;
+          V.aovf[1][__ldg(O.ovf_ptr[1] + q) + e - FC_ELL] = entry(ne + 1 + e) * di;
       } else {
         cf[0][nc * cp + sl] = di;
-        for (int e = 0; e < nc; ++e) cf[1][e * cp + sl] = e < nu ? ldcg(V.ap + k0 + ne + 1 + e) : T(0);
+        for (int e = 0; e < nc; ++e) cf[1][e * cp + sl] = e < nu ? entry(ne + 1 + e) : T(0);
         cf[1][nc * cp + sl] = di;
         cf[1][(nc + 1) * cp + sl] = T(1) / (di + (T)FC_SMALL);
       }
@@ -852,21 +866,107 @@ __device__ __forceinline__ void ord_scatter_vec(const GridCtl& C, const OrdView&
     dst[__ldg(O.perm + q)] = (U)ldcg(y + q);
 }
 
-// row products in the new numbering (FMA accumulation in the row's original
-// entry order, as ax_cr / the residual loops of the reference)
-template <class T>
-__device__ __forceinline__ T ord_row_dot(const OrdView& O, const T* __restrict__ ap, const T* x, int q) {
-  const int k0 = __ldg(O.p_ptr + q), k1 = __ldg(O.p_ptr + q + 1);
-  T s = T(0);
-  for (int k = k0; k < k1; ++k) s = fma(__ldg(ap + k), ldcg(x + __ldg(O.p_col + k)), s);
+// Row products in the new numbering, FMA accumulation in the row's original
+// entry order (as ax_cr / the residual loops of the reference): done(q, s)
+// gets s = init(q) + (NEG: -) sum a_k x_k of every row.  A warp per slice:
+// columns and values of all entries are loaded before any is used, then the
+// gathers, then the FMAs, so that a warp waits for memory twice and not once
+// per entry.  W: the slice's width (hexes 7, tetrahedra 5), 0: any.
+template <class T, bool NEG, int W>
+__device__ __forceinline__ T sell_row(const OrdView& O, const T* __restrict__ ap, const T* x, int at, int w, T s) {
+  if constexpr (W > 0) {
+    int c[W];
+    T a[W], v[W];
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      c[k] = __ldg(O.sell_col + at + FC_SLICE * k);
+      a[k] = __ldg(ap + at + FC_SLICE * k);
+    }
+#pragma unroll
+    for (int k = 0; k < W; ++k) v[k] = c[k] >= 0 ? ldcg(x + c[k]) : T(0);
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+      if (c[k] >= 0) s = fma(NEG ? -a[k] : a[k], v[k], s);
+  } else {
+    for (int k = 0; k < w; ++k) {
+      const int c = __ldg(O.sell_col + at + FC_SLICE * k);
+      if (c < 0) break;
+      const T a = __ldg(ap + at + FC_SLICE * k);
+      s = fma(NEG ? -a : a, ldcg(x + c), s);
+    }
+  }
   return s;
 }
+template <class T, bool NEG, class Init, class Done>
+__device__ __forceinline__ void ord_rows(const GridCtl& C, const OrdView& O, const T* __restrict__ ap, const T* x,
+                                         Init init, Done done) {
+  const int lane = threadIdx.x & 31, ns = (O.n + FC_SLICE - 1) / FC_SLICE;
+  for (int sl = vg_gt(C) >> 5; sl < ns; sl += vg_G(C) >> 5) {
+    const int off = __ldg(O.sell_ptr + sl), w = (__ldg(O.sell_ptr + sl + 1) - off) / FC_SLICE;
+    const int q = sl * FC_SLICE + lane, at = off + lane;
+    T s = q < O.n ? init(q) : T(0);
+    if (w == 7) s = sell_row<T, NEG, 7>(O, ap, x, at, w, s);
+    else if (w == 5) s = sell_row<T, NEG, 5>(O, ap, x, at, w, s);
+    else s = sell_row<T, NEG, 0>(O, ap, x, at, w, s);
+    if (q < O.n) done(q, s);
+  }
+}
+
+// Element-wise passes over vectors of n values (16-byte aligned): f(e, i) gets
+// the values e[0..NV) of element i and may change them; bit j of STORE: v[j]
+// is written back.  16-byte accesses, two of them per vector in flight a
+// thread: with one 8-byte access each the 20 warps of an SM do not have
+// enough bytes under way for the HBM bandwidth.
 template <class T>
-__device__ __forceinline__ T ord_row_residual(const OrdView& O, const T* __restrict__ ap, const T* x, T bq, int q) {
-  const int k0 = __ldg(O.p_ptr + q), k1 = __ldg(O.p_ptr + q + 1);
-  T s = bq;
-  for (int k = k0; k < k1; ++k) s = fma(-__ldg(ap + k), ldcg(x + __ldg(O.p_col + k)), s);
-  return s;
+struct alignas(16) VecPack {
+  static constexpr int N = 16 / sizeof(T);
+  T v[N];
+};
+template <unsigned STORE, class T, int NV, class F>
+__device__ __forceinline__ void vec_map(const GridCtl& C, int n, T* const (&v)[NV], F f) {
+  using P = VecPack<T>;
+  const int gt = vg_gt(C), G = vg_G(C), np = n / P::N;
+  for (int i = gt; i < np; i += 2 * G) {
+    P a[2][NV];
+    const bool two = i + G < np;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const float4 t = __ldcg((const float4*)v[j] + i);
+      a[0][j] = *(const P*)&t;
+    }
+    if (two)
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const float4 t = __ldcg((const float4*)v[j] + i + G);
+        a[1][j] = *(const P*)&t;
+      }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (u == 1 && !two) break;
+#pragma unroll
+      for (int m = 0; m < P::N; ++m) {
+        T e[NV];
+#pragma unroll
+        for (int j = 0; j < NV; ++j) e[j] = a[u][j].v[m];
+        f(e, (i + u * G) * P::N + m);
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+          if ((STORE >> j) & 1u) a[u][j].v[m] = e[j];
+      }
+#pragma unroll
+      for (int j = 0; j < NV; ++j)
+        if ((STORE >> j) & 1u) ((float4*)v[j])[i + u * G] = *(const float4*)&a[u][j];
+    }
+  }
+  for (int i = np * P::N + gt; i < n; i += G) {
+    T e[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) e[j] = ldcg(v[j] + i);
+    f(e, i);
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+      if ((STORE >> j) & 1u) v[j][i] = e[j];
+  }
 }
 
 }  // namespace fcdev
