@@ -284,19 +284,17 @@ extern "C" int fc_grad(fc_ctx* ctx, int scheme, const double* phi, double* dphi)
   if (!ctx->has_mesh) return fc_fail_msg(ctx, FC_ERR_STATE, "no mesh");
   FieldStore& F = ctx_fields(ctx);
   const int nT = ctx->mesh.numTotal;
-  FC_CUDA_TRY(ctx, F.cscratch_big.alloc((size_t)4 * nT));
+  FC_CUDA_TRY(ctx, F.cscratch_big.alloc((size_t)7 * nT));
   double* dphi_in = F.cscratch_big.p;
-  double* gs = F.cscratch_big.p + nT;
+  double *gs = F.cscratch_big.p + nT, *aos = gs + (size_t)3 * nT;
   FC_CUDA_TRY(ctx, cudaMemcpyAsync(dphi_in, phi, nT * sizeof(double),
                                    is_device_ptr(phi) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream));
   int st = fv_grad(ctx, scheme, dphi_in, gs);
   if (st) return st;
   // SoA -> (3, numTotal)
-  DVec<double> aos;
-  FC_CUDA_TRY(ctx, aos.alloc((size_t)3 * nT));
-  launch_soa_to_aos(ctx->stream, gs, aos.p, nT);
+  launch_soa_to_aos(ctx->stream, gs, aos, nT);
   ctx->kernel_launches++;
-  FC_CUDA_TRY(ctx, cudaMemcpyAsync(dphi, aos.p, (size_t)3 * nT * sizeof(double),
+  FC_CUDA_TRY(ctx, cudaMemcpyAsync(dphi, aos, (size_t)3 * nT * sizeof(double),
                                    is_device_ptr(dphi) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                                    ctx->stream));
   FC_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
