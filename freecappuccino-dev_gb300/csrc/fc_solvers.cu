@@ -179,8 +179,8 @@ __device__ bool ord_prologue(const KArgs<T>& A, bool dilu, bool with_x, bool gs 
 template <class T>
 __device__ bool ord_residual_l1(const KArgs<T>& A, int& ph, double& l1out) {
   double s[1] = {0.0};
-  ord_rows<T, true>(A.C, A.O, (const T*)A.V.ap, (const T*)A.xo, [&](int q) { return ldcg(A.bo + q); },
-                    [&](int q, T rq) {
+  ord_rows<T, true>(A.C, A.O, (const T*)A.V.ap, (const T*)A.xo, (const T*)A.bo,
+                    [&](int q, T rq, T) {
                       A.r[q] = rq;
                       s[0] += fabs((double)rq);
                     });
@@ -252,10 +252,10 @@ __global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1) k_iccg(const __grid_constan
     if (!grid_sync(A.C)) return;
     tr.mark(TR_PUPD);
     double pap[1] = {0.0};
-    ord_rows<T, false>(A.C, A.O, (const T*)A.V.ap, (const T*)p, [](int) { return T(0); },
-                       [&](int i, T zi) {
+    ord_rows<T, false>(A.C, A.O, (const T*)A.V.ap, (const T*)p, (const T*)p,
+                       [&](int i, T zi, T pi) {
                          z[i] = zi;
-                         pap[0] += (double)ldcg(p + i) * (double)zi;
+                         pap[0] += (double)pi * (double)zi;
                        });
     if (!grid_reduce<1>(A.C, ph, pap)) return;
     tr.mark(TR_SPMV);
@@ -327,10 +327,10 @@ __device__ __forceinline__ void bicgstab_body(const KArgs<T>& A) {
     if (!precond_apply<T>(A, X, (const T*)p, yf, z, (const T*)nullptr, nullptr, &tr)) return;
     if (!grid_sync(A.C)) return;
     double ur[1] = {0.0};
-    ord_rows<T, false>(A.C, A.O, (const T*)A.V.ap, (const T*)z, [](int) { return T(0); },
-                       [&](int i, T ui) {
+    ord_rows<T, false>(A.C, A.O, (const T*)A.V.ap, (const T*)z, (const T*)r0,
+                       [&](int i, T ui, T r0i) {
                          u[i] = ui;
-                         ur[0] += (double)ui * (double)ldcg(r0 + i);
+                         ur[0] += (double)ui * (double)r0i;
                        });
     if (!grid_reduce<1>(A.C, ph, ur)) return;
     gam = bet / ur[0];
@@ -343,10 +343,10 @@ __device__ __forceinline__ void bicgstab_body(const KArgs<T>& A) {
     if (!precond_apply<T>(A, X, (const T*)r, yf, z, (const T*)nullptr, nullptr, &tr)) return;
     if (!grid_sync(A.C)) return;
     double vr[2] = {0.0, 0.0};
-    ord_rows<T, false>(A.C, A.O, (const T*)A.V.ap, (const T*)z, [](int) { return T(0); },
-                       [&](int i, T vi) {
+    ord_rows<T, false>(A.C, A.O, (const T*)A.V.ap, (const T*)z, (const T*)r,
+                       [&](int i, T vi, T ri) {
                          v[i] = vi;
-                         vr[0] += (double)vi * (double)ldcg(r + i);
+                         vr[0] += (double)vi * (double)ri;
                          vr[1] += (double)vi * (double)vi;
                        });
     if (!grid_reduce<2>(A.C, ph, vr)) return;
