@@ -27,14 +27,19 @@
 // is the relative reduction of the D-norm of r~; the refinement loop checks
 // the true residual.
 //
-// The inner solve is one CUDA graph per system: a prologue (the forward sweep
-// on the right-hand side, the first direction), a device-side while loop
-// whose body is one kernel per pass, and the final backward sweep x =
-// (D+U)^-1 y.  Every kernel runs at full occupancy with one thread per row;
-// the scalars of the iteration are finalised in device memory by the last
-// block of each reduction, in a fixed order, and the block that decides to
-// stop clears the loop's condition.  Dot products and norms are accumulated
-// in FP64 in both value types.
+// On two colours (hexahedra) a solve is a prologue (the forward sweep on the
+// right-hand side, the first direction), one persistent cooperative kernel for
+// all iterations (k_mc_loop2), and the final backward sweep x = (D+U)^-1 y.
+// With more colours it is one CUDA graph per system: the same prologue, a
+// device-side while loop whose body is one kernel per pass, and the final
+// sweep; the scalars of the iteration are finalised in device memory by the
+// last block of each reduction, in a fixed order, and the block that decides
+// to stop clears the loop's condition.  The line lies there because a pass
+// costs an exchange of all blocks in the one and a launch in the other, and an
+// iteration on C > 2 colours has 2 C of them on C-th parts of the rows:
+// 750,000 tetrahedra in FP32 took 39 ms by the graph and 54 by such a kernel,
+// 853,000 hexahedra 24.0 by the graph and 20.5 by the kernel.
+// Dot products and norms are accumulated in FP64 in both value types.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -43,6 +48,7 @@
 
 #include "fc_colour.hpp"
 #include "fc_internal.hpp"
+#include "fc_krylov.cuh"
 
 #define MCG_BLOCK 512
 // the loop-body kernels run grid-stride on at most this many waves of
@@ -63,6 +69,7 @@ struct McScal {
   double alpha, beta;
   int it, itmax, done, status;
   double rz0;
+  int fault;  // the loop kernel's exchanges: 0 or FC_ERR_TIMEOUT
 };
 
 // the buffers of one value type: FP32 (FC_PREC_MIXED_COLOURED) or FP64
@@ -73,7 +80,7 @@ struct McBuf {
   DVec<T> mval, adiag, invd, dvec, kdiag, x, r, p, q, y, t, w;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  int wave = 1;  // resident blocks of the widest loop-body kernel on the whole GPU
+  int wave = 1;  // resident blocks on the whole GPU: of the loop kernel, or of the graph's colour-0 kernel
   bool ready = false;
   ~McBuf() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -85,6 +92,7 @@ struct DevColoured {
   int n = 0, nP = 0, ncol = 0, maxblocks = 1;
   size_t nent = 1;  // ELLPACK entries of the layout
   std::vector<int> crow;
+  int w2 = 0;  // two colours: the wider of colour 0's upper and colour 1's lower block
   DVec<int> tab, perm, col, src, tsrc, dslot;
   DVec<double> dset, part;
   DVec<unsigned> cnt;
@@ -117,7 +125,7 @@ struct McDevT {
   double* dset;
   T *x, *r, *p, *q, *y, *t, *w;
   McScal* sc;
-  double* part;     // 2 * blocks of the widest launch
+  double* part;     // the reductions' partial sums, one per block; the loop's slots, MC_PARTS per block
   unsigned* cnt;    // arrival counter of the last-block reductions
   cudaGraphConditionalHandle h;
 };
@@ -279,7 +287,7 @@ __global__ void k_mc_gather(McDevT<T> D, const int* __restrict__ perm, const dou
     s.res0 = s.resl = s.rz = s.rzacc = s.pq = s.rz0 = 0.0;
     s.tol = tol;
     s.alpha = s.beta = 0.0;
-    s.it = 0; s.itmax = itmax; s.done = 0; s.status = 0;
+    s.it = 0; s.itmax = itmax; s.done = 0; s.status = 0; s.fault = 0;
     *D.sc = s;
   }
 }
@@ -482,88 +490,349 @@ __global__ void __launch_bounds__(MCG_BLOCK) k_e_pupd(McDevT<T> D) {
   }
 }
 
-// Two colours (red-black): the new direction p = z + beta p is folded into
-// the two colour passes, so an iteration is three kernels.  Colour 0 updates
-// its own p and gathers t_j = (z_j + beta p_j) / d_j of its colour-1
-// neighbours, whose p the colour-1 pass has not yet replaced.
-template <class T>
-__device__ __forceinline__ T ell_sum_t(const McDevT<T>& D, int e, int stride, int w, T beta, T acc) {
-  if (w <= MC_UNROLL) {
-    int c[MC_UNROLL];
-    T m[MC_UNROLL];
-#pragma unroll
-    for (int k = 0; k < MC_UNROLL; ++k)
-      if (k < w) {
-        c[k] = __ldg(D.col + e + k * stride);
-        m[k] = __ldcg(D.mval + e + k * stride);
-      }
-#pragma unroll
-    for (int k = 0; k < MC_UNROLL; ++k)
-      if (k < w) {
-        const T tj = mfma(beta, __ldcg(D.p + c[k]), __ldcg(D.y + c[k])) * __ldcg(D.invd + c[k]);
-        acc = mfma(m[k], tj, acc);
-      }
-    return acc;
-  }
-  for (int k = 0; k < w; ++k) {
-    const int cj = __ldg(D.col + e + k * stride);
-    acc = mfma(__ldcg(D.mval + e + k * stride), mfma(beta, __ldcg(D.p + cj), __ldcg(D.y + cj)) * __ldcg(D.invd + cj), acc);
-  }
-  return acc;
+// ------------------------------------- the loop kernel of two colours: passes
+// Each pass over n rows (or groups of four) is shared out to the first
+// mc_share(n) blocks of the grid, one row a thread and then grid-stride.
+__device__ __forceinline__ int mc_share(int n) {
+  return max(1, min((int)gridDim.x, (n + MCG_BLOCK - 1) / MCG_BLOCK));
+}
+struct McRange {
+  int i, end, stride;  // this thread's first row, the end, the step; i >= end: none
+};
+__device__ __forceinline__ McRange mc_range(int r0, int r1) {
+  const int nb = mc_share(r1 - r0);
+  return {(int)blockIdx.x < nb ? r0 + (int)blockIdx.x * MCG_BLOCK + (int)threadIdx.x : r1, r1, nb * MCG_BLOCK};
 }
 
-// colour 0 of two: p = z + beta p, t = (p - U t)/d, w = (p + K t)/d, q, p.q
+// y += alpha p, r~ -= alpha q, z = D r~; r~.z.  x, r and d of a thread's first
+// group, which the passes before leave alone, are loaded ahead (McUpd).
 template <class T>
-__global__ void __launch_bounds__(MCG_BLOCK) k_e2_c0(McDevT<T> D) {
-  const McBcast sc = mcg_scalars(D);
-  if (sc.done) return;
-  const T beta = (T)sc.beta;
-  const int r1 = __ldg(D.tab + MC_CR + 1);
-  const int ceu = __ldg(D.tab + MC_CEU), cwu = __ldg(D.tab + MC_CWU);
-  double v[1] = {0.0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < r1; i += gridDim.x * blockDim.x) {
-    const T pi = mfma(beta, __ldcg(D.p + i), __ldcg(D.y + i));
-    const T di = __ldcg(D.invd + i), ki = __ldcg(D.kdiag + i);
-    const T ti = (pi - ell_sum_t(D, ceu + i, r1, cwu, beta, T(0))) * di;
-    const T wi = mfma(ki, ti, pi) * di;
+struct McUpd {
+  T x[4], r[4], d[4];
+};
+template <class T>
+__device__ __forceinline__ void mc_upd_load(const McDevT<T>& D, const McRange& R, int i4, McUpd<T>& U) {
+  if (i4 >= R.end) return;
+  ld4(D.x, i4, U.x); ld4(D.r, i4, U.r); ld4(D.dvec, i4, U.d);
+}
+template <class T>
+__device__ __forceinline__ double mc_update(const McDevT<T>& D, const McRange& R, McUpd<T>& U, T alpha) {
+  double v = 0.0;
+  for (int i4 = R.i; i4 < R.end;) {
+    T p4[4], q4[4], zn[4];
+    ld4(D.p, i4, p4); ld4(D.q, i4, q4);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      U.r[k] = mfma(-alpha, q4[k], U.r[k]);
+      zn[k] = U.d[k] * U.r[k];
+      U.x[k] = mfma(alpha, p4[k], U.x[k]);
+      v += (double)U.r[k] * (double)zn[k];
+    }
+    st4(D.x, i4, U.x);
+    st4(D.r, i4, U.r);
+    st4(D.y, i4, zn);
+    i4 += R.stride;
+    mc_upd_load(D, R, i4, U);
+  }
+  return v;
+}
+
+// Two colours (red-black): the direction p = z + beta p is folded into the two
+// colour passes.  Colour 0 updates its own p and gathers t_j = (z_j + beta p_j) /
+// d_j of its colour-1 neighbours, whose p the colour-1 pass has not yet
+// replaced.  What a row reads that the passes before do not write (matrix,
+// diagonals, its own p, colour 1 also z) is loaded ahead (McRow).
+template <class T, int W>
+struct McRow {
+  int c[W];
+  T m[W], d, k, p, y;
+};
+template <class T, int W, int COLOUR>
+__device__ __forceinline__ void mc_row_load(const McDevT<T>& D, const McRange& R, int i, int e, int w, McRow<T, W>& P) {
+  if (i >= R.end) return;
+#pragma unroll
+  for (int k = 0; k < W; ++k)
+    if (k < w) {
+      P.c[k] = __ldg(D.col + e + k * (COLOUR ? R.end - D.c0end : R.end));
+      P.m[k] = __ldcg(D.mval + e + k * (COLOUR ? R.end - D.c0end : R.end));
+    }
+  P.d = __ldcg(D.invd + i);
+  P.k = __ldcg(D.kdiag + i);
+  P.p = __ldcg(D.p + i);
+  if (COLOUR) P.y = __ldcg(D.y + i);
+}
+// colour 0 of two: p = z + beta p, t = (p - U t)/d, w = (p + K t)/d, q; p.q
+template <class T, int W>
+__device__ __forceinline__ double mc_fold0(const McDevT<T>& D, const McRange& R, int e0, int w, McRow<T, W>& P, T beta) {
+  double v = 0.0;
+  for (int i = R.i; i < R.end;) {
+    const T pi = mfma(beta, P.p, __ldcg(D.y + i));
+    T acc = T(0);
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+      if (k < w) {
+        const T tj = mfma(beta, __ldcg(D.p + P.c[k]), __ldcg(D.y + P.c[k])) * __ldcg(D.invd + P.c[k]);
+        acc = mfma(P.m[k], tj, acc);
+      }
+    if (W == MC_UNROLL)
+      for (int k = W; k < w; ++k) {
+        const int cj = __ldg(D.col + e0 + i + k * R.end);
+        const T tj = mfma(beta, __ldcg(D.p + cj), __ldcg(D.y + cj)) * __ldcg(D.invd + cj);
+        acc = mfma(__ldcg(D.mval + e0 + i + k * R.end), tj, acc);
+      }
+    const T ti = (pi - acc) * P.d;
+    const T wi = mfma(P.k, ti, pi) * P.d;
     const T qi = ti + wi;
     D.p[i] = pi;
     D.w[i] = wi;
     D.q[i] = qi;
-    v[0] += (double)pi * (double)qi;
+    v += (double)pi * (double)qi;
+    i += R.stride;
+    mc_row_load<T, W, 0>(D, R, i, e0 + i, w, P);
   }
-  double tot[1];
-  if (!mcg_reduce<1>(D, v, tot) || threadIdx.x != 0) return;
-  D.sc->pq = tot[0];
+  return v;
 }
-
-// colour 1 of two: p = z + beta p, t = p/d, w = (p + K t - L w)/d, q, p.q, alpha
-template <class T>
-__global__ void __launch_bounds__(MCG_BLOCK) k_e2_c1(McDevT<T> D) {
-  const McBcast sc = mcg_scalars(D);
-  if (sc.done) return;
-  const T beta = (T)sc.beta;
-  const int r0 = __ldg(D.tab + MC_CR + 1), r1 = __ldg(D.tab + MC_CR + 2);
-  const int cel = __ldg(D.tab + MC_CEL + 1), cwl = __ldg(D.tab + MC_CWL + 1);
-  double v[1] = {0.0};
-  for (int i = r0 + blockIdx.x * blockDim.x + threadIdx.x; i < r1; i += gridDim.x * blockDim.x) {
-    const T pi = mfma(beta, __ldcg(D.p + i), __ldcg(D.y + i));
-    const T di = __ldcg(D.invd + i), ki = __ldcg(D.kdiag + i);
-    const T ti = pi * di;
-    const T wi = (mfma(ki, ti, pi) - ell_sum(D, cel + (i - r0), r1 - r0, cwl, D.w, T(0))) * di;
+// colour 1 of two: p = z + beta p, t = p/d, w = (p + K t - L w)/d, q; p.q
+template <class T, int W>
+__device__ __forceinline__ double mc_fold1(const McDevT<T>& D, const McRange& R, int e0, int w, McRow<T, W>& P, T beta) {
+  double v = 0.0;
+  for (int i = R.i; i < R.end;) {
+    const T pi = mfma(beta, P.p, P.y);
+    const T ti = pi * P.d;
+    T acc = T(0);
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+      if (k < w) acc = mfma(P.m[k], __ldcg(D.w + P.c[k]), acc);
+    if (W == MC_UNROLL)
+      for (int k = W; k < w; ++k) {
+        const int e = e0 + (i - D.c0end) + k * (R.end - D.c0end);
+        acc = mfma(__ldcg(D.mval + e), __ldcg(D.w + __ldg(D.col + e)), acc);
+      }
+    const T wi = (mfma(P.k, ti, pi) - acc) * P.d;
     const T qi = ti + wi;
     D.p[i] = pi;
     D.w[i] = wi;
     D.q[i] = qi;
-    v[0] += (double)pi * (double)qi;
+    v += (double)pi * (double)qi;
+    i += R.stride;
+    mc_row_load<T, W, 1>(D, R, i, e0 + (i - D.c0end), w, P);
   }
-  double tot[1];
-  if (!mcg_reduce<1>(D, v, tot) || threadIdx.x != 0) return;
-  McScal* S = D.sc;
-  S->pq += tot[0];
-  const double alpha = S->rz / S->pq;
-  if (!(alpha == alpha) || isinf(alpha)) mcg_stop(D, FC_ERR_BREAKDOWN);
-  else S->alpha = alpha;
+  return v;
+}
+
+// ------------------------------------------------------ exchanges of the grid
+// An exchange is a barrier that carries up to two FP64 values of every block:
+// a block writes its values into its slots and a warp of every block polls all
+// blocks' slots, so that arrival, completion and the values take one round trip
+// through L2 (a counter, its polling and the load of the values one after the
+// other take three).  One warp with relaxed loads and a fence at the end: with
+// an acquiring load by a thread per slot an exchange of 304 blocks took 7 us.
+// A slot without a value holds a sentinel (all bits set; a NaN that comes out
+// so is written as another one).  There are three sets of slots in turn: a
+// block clears its slots of the next exchange just before it writes those of
+// this one.  They were last read two exchanges ago, which all blocks have
+// left, since all have been seen to arrive at the one after; and nobody polls
+// them before this block has arrived here.
+#define MC_NOVAL 0xFFFFFFFFFFFFFFFFull
+#define MC_PARTS 6   // values of a block: two in each of three sets
+struct McGrid {
+  unsigned long long* slot;  // [3][2][gridDim.x]
+  int* fault;
+  int ph;
+};
+__device__ __forceinline__ unsigned long long* mc_slot(const McGrid& G, int ph, int j) {
+  return G.slot + ((size_t)(ph % 3) * 2 + j) * gridDim.x;
+}
+// one thread per value j publishes it (after a __syncthreads); the one with
+// value 0, which every exchange has, clears the next exchange's slots
+__device__ __forceinline__ void mc_publish(const McGrid& G, int j, double v) {
+  unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  if (b == MC_NOVAL) b = 0x7FF8000000000000ull;
+  if (j == 0)
+    for (int k = 0; k < 2; ++k) *(volatile unsigned long long*)(mc_slot(G, G.ph + 1, k) + blockIdx.x) = MC_NOVAL;
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(mc_slot(G, G.ph, j) + blockIdx.x), "l"(b) : "memory");
+}
+// A warp waits for value j of all blocks, use(b, value) gets them; false if the
+// wait ran out or another block gave up.  All loads of a round are in flight
+// together.
+#define MC_POLLS 10
+template <class F>
+__device__ __forceinline__ bool mc_poll(const McGrid& G, int j, F use) {
+  const unsigned long long* at = mc_slot(G, G.ph, j);
+  const int lane = threadIdx.x & 31, nb = gridDim.x;
+  bool ok = true;
+  for (int b0 = lane; b0 < nb && ok; b0 += 32 * MC_POLLS) {
+    unsigned pending = 0, spins = 0;
+#pragma unroll
+    for (int k = 0; k < MC_POLLS; ++k) pending |= (b0 + 32 * k < nb ? 1u : 0u) << k;
+    while (pending) {
+      unsigned long long x[MC_POLLS];
+#pragma unroll
+      for (int k = 0; k < MC_POLLS; ++k) {
+        x[k] = MC_NOVAL;
+        if ((pending >> k) & 1u)
+          asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x[k]) : "l"(at + b0 + 32 * k) : "memory");
+      }
+#pragma unroll
+      for (int k = 0; k < MC_POLLS; ++k)
+        if (x[k] != MC_NOVAL) {
+          use(b0 + 32 * k, __longlong_as_double((long long)x[k]));
+          pending &= ~(1u << k);
+        }
+      if (pending && (++spins > FC_SPIN_LIMIT || ((spins & 63u) == 0 && *((volatile int*)G.fault) != 0))) {
+        atomicCAS(G.fault, 0, FC_ERR_TIMEOUT);
+        ok = false;
+        break;
+      }
+    }
+  }
+  __threadfence();
+  return __all_sync(0xffffffffu, ok);
+}
+
+// The 512 values of a block are summed as 16 trees of 32 (neighbours at 16, 8,
+// 4, 2, 1 apart) and the trees' sums one after the other; so are the blocks'.
+// A lane holds half a tree's leaves, so a tree costs the FP64 pipe 16
+// instructions for all 16 trees instead of 5 in each of 16 warps.
+#define MC_PAD(i) ((i) + 2 * ((i) >> 5))   // a warp's 16 trees start in different banks
+__device__ __noinline__ double mc_tree(const double* sm, int trees) {
+  const int lane = threadIdx.x & 31, w = lane >> 1, h = lane & 1;
+  double a[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) a[k] = w < trees ? sm[MC_PAD(32 * w + 2 * k + h)] : 0.0;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < o; ++k) a[k] += a[k + o];
+  const double s = a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
+  double t = __shfl_sync(0xffffffffu, s, 0);
+  for (int u = 1; u < trees; ++u) t += __shfl_sync(0xffffffffu, s, 2 * u);
+  return t;
+}
+// barrier; false if it failed
+__device__ __forceinline__ bool mc_sync(McGrid& G) {
+  __syncthreads();
+  bool ok = true;
+  if (threadIdx.x < 32) {
+    if (threadIdx.x == 0) mc_publish(G, 0, 0.0);
+    ok = mc_poll(G, 0, [](int, double) {});
+  }
+  ++G.ph;
+  return __syncthreads_and(ok) != 0;
+}
+// v: the sums over the first nb blocks' values, warp j taking the j-th;
+// `ahead` is called while the block's sums are on their way
+template <int NV, class Ahead>
+__device__ __forceinline__ bool mc_sum(McGrid& G, double (&v)[NV], const int (&nb)[NV], Ahead ahead) {
+  __shared__ double sm[2][MC_PAD(MCG_BLOCK)], tot[2];
+  const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) sm[j][MC_PAD(tid)] = v[j];
+  __syncthreads();
+  bool ok = true;
+  if (wid < NV) {
+    const double t = mc_tree(sm[wid], MCG_BLOCK / 32);
+    if (lane == 0) mc_publish(G, wid, t);
+  }
+  ahead();
+  if (wid < NV) {
+    // the blocks' values in the places of the threads' (a wave has at most 512 blocks)
+    double* const own = sm[wid];
+    const int n = NV > 1 && wid ? nb[NV - 1] : nb[0], trees = (n + 31) / 32;
+    for (int b = lane; b < 32 * trees; b += 32) own[MC_PAD(b)] = 0.0;
+    ok = mc_poll(G, wid, [&](int b, double x) { if (b < n) own[MC_PAD(b)] = x; });
+    __syncwarp();
+    const double s = mc_tree(own, trees);
+    if (lane == 0) tot[wid] = s;
+  }
+  ++G.ph;
+  if (!__syncthreads_and(ok)) return false;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) v[j] = tot[j];
+  return true;
+}
+
+// the iteration's scalars of a block, from totals that are the same in all
+template <class T>
+struct McIter {
+  McScal s;
+  T alpha, beta;
+};
+// alpha = r~.z / p.q (thread 0)
+template <class T>
+__device__ __forceinline__ void mc_alpha(McIter<T>& I, double pq) {
+  const double alpha = I.s.rz / pq;
+  if (!(alpha == alpha) || isinf(alpha)) { I.s.status = FC_ERR_BREAKDOWN; I.s.done = 1; }
+  I.alpha = (T)alpha;
+}
+// the stopping test on the D-norm of r~ (relative to the start) or the
+// iteration limit, beta (thread 0); r~.z keeps the sign of A (negative for the
+// reference's pressure matrix)
+template <class T>
+__device__ __forceinline__ void mc_beta(McIter<T>& I, double rz) {
+  I.s.it += 1;
+  I.s.resl = rz;
+  if (!(rz == rz) || isinf(rz)) { I.s.status = FC_ERR_NAN; I.s.done = 1; }
+  else if (fabs(rz) <= I.s.tol * I.s.tol * fabs(I.s.rz0) || I.s.it >= I.s.itmax) I.s.done = 1;
+  else {
+    I.beta = (T)(rz / I.s.rz);
+    I.s.rz = rz;
+  }
+}
+template <class T>
+__device__ __forceinline__ void mc_finish(const McDevT<T>& D, const McIter<T>& I) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    D.sc->it = I.s.it;
+    D.sc->resl = I.s.resl;
+    D.sc->status = I.s.status;
+  }
+}
+template <class T>
+__device__ __forceinline__ McGrid mc_grid(const McDevT<T>& D) {
+  return {(unsigned long long*)D.part, &D.sc->fault, 0};
+}
+
+// All iterations of the inner PCG on two colours, three exchanges an iteration.  The matrix and the vectors (78 MB at 853,000 rows in
+// FP32) stay in L2; of the 74,000 cycles of an iteration a thread's passes take
+// 22,000, bound by the latency of a row's gathers, and the exchanges the rest:
+// waiting for the block with the most rows, the fence before its arrival, and
+// the sums' chains of 16 additions.  So what a pass reads of what the one
+// before does not write is loaded while the exchange is under way.
+// 575 iterations at 101x96x88 in FP32: 24.0 ms as a graph of one kernel per
+// pass, now 20.5.  W: see McRow; 4 for tetrahedra, 6 for hexahedra, MC_UNROLL
+// also for wider rows.
+template <class T, int W>
+__global__ void __launch_bounds__(MCG_BLOCK, sizeof(T) == 4 ? 2 : 1) k_mc_loop2(const __grid_constant__ McDevT<T> D) {
+  __shared__ McIter<T> I;
+  McGrid G = mc_grid(D);
+  const int e0 = __ldg(D.tab + MC_CEU), w0 = __ldg(D.tab + MC_CWU), e1 = __ldg(D.tab + MC_CEL + 1),
+            w1 = __ldg(D.tab + MC_CWL + 1);
+  const McRange R0 = mc_range(0, D.c0end), R1 = mc_range(D.c0end, __ldg(D.tab + MC_CR + 2)), RU = mc_range(0, D.nP >> 2);
+  const int nb[2] = {mc_share(D.c0end), mc_share(R1.end - D.c0end)}, nbu[1] = {mc_share(D.nP >> 2)};
+  if (threadIdx.x == 0) { I.s = *D.sc; I.beta = T(0); }
+  __syncthreads();
+  if (I.s.done) return;
+  McRow<T, W> P;
+  mc_row_load<T, W, 0>(D, R0, R0.i, e0 + R0.i, w0, P);
+  for (;;) {
+    const T beta = I.beta;
+    double v[2];
+    v[0] = mc_fold0<T, W>(D, R0, e0, w0, P, beta);
+    mc_row_load<T, W, 1>(D, R1, R1.i, e1 + (R1.i - D.c0end), w1, P);
+    if (!mc_sync(G)) return;
+    v[1] = mc_fold1<T, W>(D, R1, e1, w1, P, beta);
+    McUpd<T> U;
+    if (!mc_sum<2>(G, v, nb, [&]() { mc_upd_load(D, RU, RU.i, U); })) return;
+    if (threadIdx.x == 0) mc_alpha(I, v[0] + v[1]);
+    __syncthreads();
+    if (I.s.done) break;
+    double u[1] = {mc_update(D, RU, U, I.alpha)};
+    if (!mc_sum<1>(G, u, nbu, [&]() { mc_row_load<T, W, 0>(D, R0, R0.i, e0 + R0.i, w0, P); })) return;
+    if (threadIdx.x == 0) mc_beta(I, u[0]);
+    __syncthreads();
+    if (I.s.done) break;
+  }
+  mc_finish(D, I);
 }
 
 // colour c of x = (D+U)^-1 y, in place on x (higher colours already hold x)
@@ -593,7 +862,7 @@ static McDevT<T> mc_dev(DevColoured& m, McBuf<T>& b, const double* a) {
 
 static inline unsigned mc_blocks(int rows) { return (unsigned)std::max(1, (rows + MCG_BLOCK - 1) / MCG_BLOCK); }
 
-// The inner PCG graph: prologue (init, first preconditioner application) and
+// The inner PCG graph of more than two colours: prologue (init, first preconditioner application) and
 // a while node whose body is one iteration.  The kernels' arguments are fixed
 // (the system's own buffers); tolerance and iteration limit are read from the
 // scalar block, which k_mc_gather resets before every launch.
@@ -648,24 +917,18 @@ static int mc_build_graph(fc_ctx* ctx, DevColoured& m, McBuf<T>& b) {
   cudaGraph_t body = cp.conditional.phGraph_out[0];
   cudaGraphNode_t bp = nullptr;
   bool have = false;
-  if (C == 2) {  // red-black: three kernels per iteration
-    if ((st = add(body, bp, false, (const void*)k_e2_c0<T>, body_blocks(blocks_of(0)), a1))) return st;
-    if ((st = add(body, bp, true, (const void*)k_e2_c1<T>, body_blocks(blocks_of(1)), a1))) return st;
-    if ((st = add(body, bp, true, (const void*)k_e_upd<T>, body_blocks(mc_blocks(m.nP / 4)), a1))) return st;
-  } else {
-    for (int c = C - 2; c >= 1; --c) {
-      void* args[2] = {&D, &cs[c]};
-      if ((st = add(body, bp, have, (const void*)k_e_bwd<T>, body_blocks(blocks_of(c)), args))) return st;
-      have = true;
-    }
-    if ((st = add(body, bp, have, (const void*)k_e_bf0<T>, body_blocks(blocks_of(0)), a1))) return st;
-    for (int c = 1; c < C; ++c) {
-      void* args[2] = {&D, &cs[c]};
-      if ((st = add(body, bp, true, (const void*)k_e_fwd<T>, body_blocks(blocks_of(c)), args))) return st;
-    }
-    if ((st = add(body, bp, true, (const void*)k_e_upd<T>, body_blocks(mc_blocks(m.nP / 4)), a1))) return st;
-    if ((st = add(body, bp, true, (const void*)k_e_pupd<T>, body_blocks(mc_blocks(m.nP / 4)), a1))) return st;
+  for (int c = C - 2; c >= 1; --c) {
+    void* args[2] = {&D, &cs[c]};
+    if ((st = add(body, bp, have, (const void*)k_e_bwd<T>, body_blocks(blocks_of(c)), args))) return st;
+    have = true;
   }
+  if ((st = add(body, bp, have, (const void*)k_e_bf0<T>, body_blocks(blocks_of(0)), a1))) return st;
+  for (int c = 1; c < C; ++c) {
+    void* args[2] = {&D, &cs[c]};
+    if ((st = add(body, bp, true, (const void*)k_e_fwd<T>, body_blocks(blocks_of(c)), args))) return st;
+  }
+  if ((st = add(body, bp, true, (const void*)k_e_upd<T>, body_blocks(mc_blocks(m.nP / 4)), a1))) return st;
+  if ((st = add(body, bp, true, (const void*)k_e_pupd<T>, body_blocks(mc_blocks(m.nP / 4)), a1))) return st;
   // after the loop: x = (D+U)^-1 y, colours C-1..0
   prev = loop;
   for (int c = C - 1; c >= 0; --c) {
@@ -686,6 +949,7 @@ static int mc_prepare(fc_ctx* ctx, CsrSystem* s) {
   m->n = L.n; m->nP = L.nP; m->ncol = L.ncol;
   m->crow.resize(L.ncol + 1);
   for (int c = 0; c <= L.ncol; ++c) m->crow[c] = L.cslice[c] * FC_MC_SLICE;
+  if (L.ncol == 2) m->w2 = std::max(L.cwu[0], L.cwl[1]);
   std::vector<int> tab(MC_TAB, 0);
   for (int c = 0; c <= FC_MC_MAXCOL; ++c) tab[MC_CR + c] = c <= L.ncol ? m->crow[c] : L.nP;
   for (int c = 0; c < L.ncol; ++c) {
@@ -708,7 +972,8 @@ static int mc_prepare(fc_ctx* ctx, CsrSystem* s) {
   const size_t nP = std::max(1, L.nP);
   m->nent = std::max<size_t>(1, (size_t)L.nent);
   m->maxblocks = (int)mc_blocks(L.nP);
-  bool ok = m->dset.alloc(nP) == cudaSuccess && m->part.alloc((size_t)2 * m->maxblocks) == cudaSuccess &&
+  bool ok = m->dset.alloc(nP) == cudaSuccess && 
+            m->part.alloc((size_t)std::max(2 * m->maxblocks, 2 * MC_PARTS * std::max(1, ctx->num_sms))) == cudaSuccess &&
             m->cnt.alloc(1) == cudaSuccess && m->sc.alloc(1) == cudaSuccess &&
             cudaMallocHost(&m->h_sc, sizeof(McScal)) == cudaSuccess;
   if (!ok) {
@@ -720,7 +985,15 @@ static int mc_prepare(fc_ctx* ctx, CsrSystem* s) {
   return FC_OK;
 }
 
-// the buffers and the graph of value type T, on first use
+// the loop kernel for the widths of a layout of two colours
+template <class T>
+static const void* mc_loop_of(const DevColoured& m) {
+  if (m.w2 <= 4) return (const void*)k_mc_loop2<T, 4>;
+  if (m.w2 <= 6) return (const void*)k_mc_loop2<T, 6>;
+  return (const void*)k_mc_loop2<T, MC_UNROLL>;
+}
+
+// the buffers and, for more than two colours, the graph of value type T, on first use
 template <class T>
 static int mc_prepare_buf(fc_ctx* ctx, DevColoured& m, McBuf<T>& b) {
   if (b.ready) return FC_OK;
@@ -732,11 +1005,18 @@ static int mc_prepare_buf(fc_ctx* ctx, DevColoured& m, McBuf<T>& b) {
   if (!ok) return fc_fail_msg(ctx, FC_ERR_NOMEM, "multicolour buffers");
   // padding entries keep the value 0 (the setup writes real entries only)
   FC_CUDA_TRY(ctx, fc_zero(ctx->stream, b.mval.p, m.nent * sizeof(T)));
-  int nb = 0;  // resident blocks per SM of the widest body kernel
-  FC_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_e2_c0<T>, MCG_BLOCK, 0));
-  b.wave = std::max(1, ctx->num_sms) * std::max(1, nb);
-  int st = mc_build_graph(ctx, m, b);
-  if (st) return st;
+  int nb = 0;  // resident blocks per SM
+  if (m.ncol == 2) {
+    FC_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, mc_loop_of<T>(m), MCG_BLOCK, 0));
+    if (nb < 1) return fc_fail_msg(ctx, FC_ERR_UNSUPPORTED, "multicolour loop kernel does not fit an SM");
+    // the loop's sums hold the values of MCG_BLOCK blocks
+    b.wave = std::min(MCG_BLOCK, std::max(1, ctx->num_sms) * std::min(2, nb));
+  } else {
+    FC_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_e_bf0<T>, MCG_BLOCK, 0));
+    b.wave = std::max(1, ctx->num_sms) * std::max(1, nb);
+    int st = mc_build_graph(ctx, m, b);
+    if (st) return st;
+  }
   b.ready = true;
   return FC_OK;
 }
@@ -768,26 +1048,32 @@ static int mc_inner_solve_t(fc_ctx* ctx, DevColoured& m, const double* a, const 
     }
   }
   FC_CUDA_TRY(ctx, cudaGetLastError());
-  if (!ctx->tracing) {
+  const int nc = m.ncol;
+  auto blocks_of = [&](int c) { return mc_blocks(m.crow[c + 1] - m.crow[c]); };
+  auto body_blocks = [&](unsigned nat) { return std::min(nat, (unsigned)(MC_WAVES * b.wave)); };
+  if (nc == 2) {
+    for (int c = 0; c < nc; ++c) k_e_fwdb<<<blocks_of(c), MCG_BLOCK, 0, ctx->stream>>>(D, c);
+    k_e_start<<<mc_blocks(m.nP), MCG_BLOCK, 0, ctx->stream>>>(D);
+    // one wave of blocks, or as many as the widest pass needs
+    const unsigned blocks = body_blocks(std::max(mc_blocks(m.nP / 4), std::max(blocks_of(0), blocks_of(1))));
+    FC_CUDA_TRY(ctx, cudaMemsetAsync(m.part.p, 0xFF, (size_t)MC_PARTS * blocks * sizeof(double), ctx->stream));
+    void* args[1] = {&D};
+    cudaError_t e = cudaLaunchCooperativeKernel(mc_loop_of<T>(m), dim3(blocks), dim3(MCG_BLOCK), args, 0, ctx->stream);
+    if (e != cudaSuccess) return fc_fail(ctx, FC_ERR_CUDA, "cooperative launch", e);
+    for (int c = nc - 1; c >= 0; --c) k_e_xb<<<blocks_of(c), MCG_BLOCK, 0, ctx->stream>>>(D, c);
+    FC_CUDA_TRY(ctx, cudaGetLastError());
+  } else if (!ctx->tracing) {
     FC_CUDA_TRY(ctx, cudaGraphLaunch(b.exec, ctx->stream));
   } else {
     // diagnostic mode (fc_set_tracing): the same kernels launched from the
     // host, so that profilers see every launch; the loop checks the stop
     // flag every 32 iterations (the kernels of later iterations return at once)
-    const int C = m.ncol;
-    auto blocks_of = [&](int c) { return mc_blocks(m.crow[c + 1] - m.crow[c]); };
-    auto body_blocks = [&](unsigned nat) { return std::min(nat, (unsigned)(MC_WAVES * b.wave)); };
+    const int C = nc;
     for (int c = 0; c < C; ++c) k_e_fwdb<<<blocks_of(c), MCG_BLOCK, 0, ctx->stream>>>(D, c);
     k_e_start<<<mc_blocks(m.nP), MCG_BLOCK, 0, ctx->stream>>>(D);
     for (int base = 0; base < std::max(itmax, 1); base += 32) {
       for (int k = 0; k < 32; ++k) {
         const unsigned bv = body_blocks(mc_blocks(m.nP / 4));
-        if (C == 2) {
-          k_e2_c0<<<body_blocks(blocks_of(0)), MCG_BLOCK, 0, ctx->stream>>>(D);
-          k_e2_c1<<<body_blocks(blocks_of(1)), MCG_BLOCK, 0, ctx->stream>>>(D);
-          k_e_upd<<<bv, MCG_BLOCK, 0, ctx->stream>>>(D);
-          continue;
-        }
         for (int c = C - 2; c >= 1; --c) k_e_bwd<<<body_blocks(blocks_of(c)), MCG_BLOCK, 0, ctx->stream>>>(D, c);
         k_e_bf0<<<body_blocks(blocks_of(0)), MCG_BLOCK, 0, ctx->stream>>>(D);
         for (int c = 1; c < C; ++c) k_e_fwd<<<body_blocks(blocks_of(c)), MCG_BLOCK, 0, ctx->stream>>>(D, c);
@@ -804,11 +1090,11 @@ static int mc_inner_solve_t(fc_ctx* ctx, DevColoured& m, const double* a, const 
   k_mc_scatter_add<<<eb, MCG_BLOCK, 0, ctx->stream>>>(m.nP, m.perm.p, b.x.p, x64);
   FC_CUDA_TRY(ctx, cudaMemcpyAsync(m.h_sc, m.sc.p, sizeof(McScal), cudaMemcpyDeviceToHost, ctx->stream));
   FC_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  // graph kernels: prologue C + 1, per iteration 2 C (3 for two colours; the
-  // last iteration may stop early), the final backward sweep C
-  ctx->kernel_launches += 2LL * m.ncol + 1 + (long long)m.h_sc->it * (m.ncol == 2 ? 3 : 2 * m.ncol);
+  // prologue C + 1, per iteration 2 C (the last one may stop early) or one
+  // kernel for all, the final backward sweep C
+  ctx->kernel_launches += 2LL * nc + 1 + (nc == 2 ? 1 : (long long)m.h_sc->it * 2 * nc);
   *itr_out = m.h_sc->it;
-  *status_out = m.h_sc->status;
+  *status_out = m.h_sc->fault ? m.h_sc->fault : m.h_sc->status;
   return FC_OK;
 }
 
