@@ -81,7 +81,7 @@ struct DVec {
 };
 
 // Cross-block control block of the persistent solver kernels: a bounded
-// generation barrier, per-block partial sums and a sticky status word.
+// barrier, per-block partial sums and a sticky status word.
 struct GridCtl {
   unsigned* bar = nullptr;     // arrival count (two words kept)
   double* part = nullptr;      // nblocks * FC_NPART partial sums
