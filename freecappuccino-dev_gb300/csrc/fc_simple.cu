@@ -917,9 +917,10 @@ __device__ __forceinline__ void facefluxsc_inner(const MeshView& M, int i, int i
   dfiyi = dfiyi * (ary - Df * ypn);
   dfizi = dfizi * (arz - Df * zpn);
   const double fdfie = dcoef * (dfixi + dfiyi + dfizi);
-  double fii;
-  if (fm >= 0.0) fii = face_value(M, ijp, ijn, M.xf[i], M.yf[i], M.zf[i], fxp, fi, g, scheme);
-  else fii = face_value(M, ijn, ijp, M.xf[i], M.yf[i], M.zf[i], fxn, fi, g, scheme);
+  // the upwind cell first, as in k_mom_face
+  const bool out = fm >= 0.0;
+  const double fii = face_value(M, out ? ijp : ijn, out ? ijn : ijp, M.xf[i], M.yf[i], M.zf[i], out ? fxp : fxn, fi, g,
+                                scheme);
   double fcfie = fm * fii;
   const double fcfii = ce * fi[ijn] + cp * fi[ijp];
   fcfie = gam * (fcfie - fcfii);
