@@ -1090,7 +1090,7 @@ def run_gpu(args, rank, world, dist):
         ctx.set_tracing(True)
     mixed = mixed_run(fc.FC_PREC_MIXED_COLOURED, MIXED_INNER_TOL)
     ctx.set_tracing(False)
-    mixed["inner_solver"] = ("FP32 ICCG, multicolour DIC (%d colours) in Eisenstat form, one CUDA graph"
+    mixed["inner_solver"] = ("FP32 ICCG, multicolour DIC (%d colours) in Eisenstat form, one persistent kernel"
                              % ctx.mixed_colours(0))
     mixed_nat = mixed_run(fc.FC_PREC_MIXED, MIXED_NATURAL_INNER_TOL)
     mixed_nat["inner_solver"] = "FP32 ICCG, natural-order DIC (the FP64 path's sweeps)"
