@@ -66,14 +66,14 @@ constexpr float kFreeRatio = KIND == FC_LIMITER_BJ ? 1.01f : 2.02f;
 // fimin/fimax: min/max of phi over all cells
 //
 // A neighbour is screened first: the projection d in FP32 with a bound of its
-// error (six roundings; the coordinate differences are taken in FP64).  If it
-// is certain that |d| is above kTinyDelta and r above kFreeRatio, the limiter
-// value is 1 or more and the neighbour is passed over; if |d| is certainly
-// below kTinyDelta, r is 1.  NaN and infinities fail both tests.  The others
-// are evaluated in FP64 as written: 38 FP64 instructions, two divisions among
-// them, at 17 cycles a warp, which bounded the kernel; the screening takes 3
-// and three conversions.  128^3, Venkatakrishnan, a smooth front with noise:
-// 1,005 us a launch without it, now 252.
+// error (the coordinates' rounding and six more).  If it is certain that |d| is
+// above kTinyDelta and r above kFreeRatio, the limiter value is 1 or more and
+// the neighbour is passed over; if |d| is certainly below kTinyDelta, r is 1.
+// NaN and infinities fail both tests.  The others are evaluated in FP64 as
+// written: 38 FP64 instructions, two divisions among them, at 17 cycles a warp,
+// which bounded the kernel; the screening takes three conversions.  fc_grad at
+// 128^3, least squares with Venkatakrishnan, a smooth front with noise: 1,483 us
+// without it (the limiter 1,005), 650 with the differences in FP64, now 607.
 template <int KIND>
 FC_HD double limit_factor(int c, const int* ia, const int* ja, const int* dg, const double* xc, const double* yc,
                           const double* zc, const double* phi, double gx, double gy, double gz, double fimin,
@@ -82,21 +82,25 @@ FC_HD double limit_factor(int c, const int* ia, const int* ja, const int* dg, co
   const double deltamin = fimin - phi[c];
   const double x = xc[c], y = yc[c], z = zc[c];
   const float gxf = (float)gx, gyf = (float)gy, gzf = (float)gz, room_up = (float)deltamax, room_dn = -(float)deltamin;
+  const float xf = (float)x, yf = (float)y, zf = (float)z;
+  const float ex = 1.e-7f * fabsf(gxf), ey = 1.e-7f * fabsf(gyf), ez = 1.e-7f * fabsf(gzf);
   double slopelimit = 1.0;
   const int kd = dg[c];
   for (int k = ia[c]; k < ia[c + 1]; ++k) {
     if (k == kd) continue;
     const int n = ja[k];
-    const double dx = xc[n] - x, dy = yc[n] - y, dz = zc[n] - z;
-    const float px = gxf * (float)dx, py = gyf * (float)dy, pz = gzf * (float)dz;
+    const double xn = xc[n], yn = yc[n], zn = zc[n];
+    const float xnf = (float)xn, ynf = (float)yn, znf = (float)zn;
+    const float px = gxf * (xnf - xf), py = gyf * (ynf - yf), pz = gzf * (znf - zf);
     const float d = px + py + pz, size = fabsf(d);
-    const float err = 1.e-6f * (fabsf(px) + fabsf(py) + fabsf(pz)) + 1.e-30f;
+    const float err = 1.e-6f * (fabsf(px) + fabsf(py) + fabsf(pz)) + ex * (fabsf(xnf) + fabsf(xf)) +
+                      ey * (fabsf(ynf) + fabsf(yf)) + ez * (fabsf(znf) + fabsf(zf)) + 1.e-30f;
     if (size + err < 0.9e-6f) {
       slopelimit = dmin(slopelimit, limiter_fn<KIND>(1.0));
       continue;
     }
     if (size - err > 1.1e-6f && kFreeRatio<KIND> * (size + err) < (d > 0.f ? room_up : room_dn)) continue;
-    const double delta_face = gx * dx + gy * dy + gz * dz;
+    const double delta_face = gx * (xn - x) + gy * (yn - y) + gz * (zn - z);
     if ((delta_face < 0.0 ? -delta_face : delta_face) < kTinyDelta) {
       slopelimit = dmin(slopelimit, limiter_fn<KIND>(1.0));
       continue;
