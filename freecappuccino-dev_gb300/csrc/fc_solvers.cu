@@ -628,7 +628,6 @@ __global__ void __launch_bounds__(FC_SWEEP_BLOCK, 1)
 // residual after which the inner solve ends (the longest such run in the
 // converging solves of the batched convection-diffusion set is 22)
 #define FC_INNER_STALL_WINDOW 32
-#define FC_SWEEP_SMEM (200 * 1024)   // dynamic shared memory budget of a sweep kernel
 
 bool is_device_ptr(const void* p) {
   if (!p) return false;
@@ -684,68 +683,6 @@ static cudaError_t upload_vec(cudaStream_t s, DVec<int>& d, const V& h) {
   return fc_h2d(s, d.p, h.data(), h.size() * sizeof(int));
 }
 
-// A structure's steps in groups of G, one stage buffer each: the
-// descriptors of the steps (OrdView::desc) and the largest group; false if
-// a descriptor's 16-bit fields do not hold it.
-static bool group_steps(const OrderedSweep& O, int G, OrdView& V, std::vector<int>* desc) {
-  V.G = G;
-  V.gen = O.max_entries > FC_ELL || O.maxW > FC_SET_ROWS;
-  V.nc = O.max_entries > 3 ? FC_ELL : 3;
-  V.g_rows = V.g_padded = V.g_push = V.g_x = 0;
-  if (desc)
-    for (int d = 0; d < 2; ++d) desc[d].assign((size_t)4 * O.nsteps, 0);
-  for (int d = 0; d < 2; ++d) {
-    const OrderedDir& H = O.dir[d];
-    for (int t = 0; t < O.ntiles; ++t) {
-      const int s0 = O.tile_step_ptr[t], ns = O.tile_step_ptr[t + 1] - s0;
-      for (int k0 = 0; k0 < ns; k0 += G) {
-        const int k1 = std::min(k0 + G, ns), lo = s0 + (d ? ns - k1 : k0), hi = s0 + (d ? ns - k0 : k1);
-        V.g_rows = std::max(V.g_rows, O.step_ptr[hi] - O.step_ptr[lo]);
-        V.g_padded = std::max(V.g_padded, O.rp_ptr[hi] - O.rp_ptr[lo]);
-        V.g_push = std::max(V.g_push, H.push_ptr[hi] - H.push_ptr[lo]);
-        V.g_x = std::max(V.g_x, H.xv_ptr[hi] - H.xv_ptr[lo]);
-        if (!desc) continue;
-        for (int s = lo; s < hi; ++s) {
-          int* q = desc[d].data() + 4 * (size_t)s;
-          q[0] = O.step_ptr[s];
-          q[1] = (O.step_ptr[s + 1] - O.step_ptr[s]) | ((H.push_ptr[s + 1] - H.push_ptr[s]) << 16);
-          q[2] = (O.rp_ptr[s] - O.rp_ptr[lo]) | ((H.push_ptr[s] - H.push_ptr[lo]) << 16);
-          q[3] = (O.step_ptr[s] - (O.step_ptr[lo] & ~3)) | ((H.xv_ptr[s] - H.xv_ptr[lo]) << 16);
-        }
-      }
-    }
-  }
-  return V.g_rows < 65530 && V.g_padded < 65536 && V.g_push < 65536 && V.g_x < 65536;
-}
-
-// the stage area of the ordered sweeps: the shared memory the fixed parts
-// leave (the sweep modes cut it into as many buffers as fit, at most
-// FC_MAX_STAGES); 0 when nothing is left
-static size_t ordered_stage_area(int R, int maxW) {
-  const size_t fixed = osweep_fixed_bytes<double>(R, maxW);
-  return fixed >= (size_t)FC_SWEEP_SMEM ? 0 : ((size_t)FC_SWEEP_SMEM - fixed) & ~(size_t)15;
-}
-
-// The most steps of a stage buffer with which every mode (gs: Gauss-Seidel,
-// else the setups and applications) gets the FC_SETS buffers the sweeps need
-// (see fc_sweep.cuh); 0 if none.
-static int steps_per_buffer(const OrderedSweep& O, bool gs) {
-  // Gauss-Seidel steps take one row per thread (their loads include the
-  // upper triangle's values)
-  if (gs && O.maxW > FC_SET_ROWS) return 0;
-  const size_t area = ordered_stage_area(O.R, O.maxW);
-  for (int G = FC_SETS; G >= 1; G /= 2) {
-    OrdView V;
-    bool ok = group_steps(O, G, V, nullptr);
-    for (int m = gs ? OS_GS : OS_SETUP_DIC; m <= (gs ? OS_GS : OS_BWD_DOT); ++m) {
-      const int bytes = StageLayout::of<double>(V, m).bytes;
-      ok = ok && (size_t)bytes <= area && stages_in(area, bytes) >= FC_SETS;
-    }
-    if (ok) return G;
-  }
-  return 0;
-}
-
 // rows in new order (p_ptr, p_col, p_slot) into slices, a warp per slice
 __global__ void k_sell(int n, const int* __restrict__ p_ptr, const int* __restrict__ p_col,
                        const int* __restrict__ p_slot, const int* __restrict__ sell_ptr, int* __restrict__ col,
@@ -769,7 +706,7 @@ static int upload_ordered(fc_ctx* ctx, const OrderedSweep& O, DevOrdered& D, boo
     DevOrdered::Groups& P = D.grp[gs];
     P.G = gs && !for_gs ? 0 : steps_per_buffer(O, gs != 0);
     if (P.G == 0) continue;
-    OrdView V;
+    StepGroups V;
     std::vector<int> desc[2];
     group_steps(O, P.G, V, desc);
     D.nc = V.nc; D.gen = V.gen;

@@ -62,18 +62,8 @@
 #pragma once
 #include <type_traits>
 #include "fc_krylov.cuh"
-#include "fc_schedule.hpp"
+#include "fc_stage.hpp"
 
-// Warp roles of a block: FC_SETS x FC_SET_WARPS compute warps, the importers,
-// the stager.  A set is one warp per SM sub-partition and covers a step of
-// FC_SET_ROWS rows with one row per thread: four warps issue their FMAs in
-// about the 64 cycles one FMA takes, so more rows per step would lengthen the
-// step in proportion.  20 warps leave 96 registers a thread (21 would leave 80).
-#define FC_SETS 4
-#define FC_SET_WARPS 4
-#define FC_IMP_WARPS 3
-#define FC_SET_ROWS (32 * FC_SET_WARPS)
-static_assert(FC_SET_ROWS == FC_STEP_ROWS, "the schedule's cost model counts these steps");
 static_assert(FC_SWEEP_BLOCK == 32 * (FC_SETS * FC_SET_WARPS + FC_IMP_WARPS + 1), "warp roles fill the block");
 
 namespace fcdev {
@@ -105,8 +95,6 @@ __device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned
                "l"(src), "r"(bytes), "r"(mb)
                : "memory");
 }
-#define FC_MAX_STAGES 16
-#define FC_SMEM_HDR (2 * FC_MAX_STAGES * 8)  // full and empty mbarriers at the start of the dynamic area
 #define FC_MBAR_SPIN_LIMIT (1u << 22)
 // bounded wait for the completion of phase `parity`; false if it ran out or
 // the block is leaving.  backoff_ns > 0 sleeps between polls (a thread that
@@ -128,10 +116,6 @@ __device__ __forceinline__ bool mbar_wait_warp(unsigned mb, unsigned parity, vol
   if ((threadIdx.x & 31) == 0) ok = mbar_wait(mb, parity, abort_flag);
   return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
 }
-// Named barriers 1..FC_STEP_BARS: the barrier of step k releases the set of
-// step k once the set of step k-1 and the importer of step k have arrived.  The
-// importers stay less than FC_STEP_BARS steps ahead, so that none arrives twice.
-#define FC_STEP_BARS (FC_IMP_WARPS * FC_SETS)
 __device__ __forceinline__ void bar_wait(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
@@ -243,60 +227,6 @@ struct OrdVals {
   T* xv[2];    // exchange arrays (per-step blocks)
 };
 
-// the form of the applications (see the file header)
-template <class T> struct ScaledApply { static constexpr bool value = sizeof(T) == 8; };
-// values per row of a step's block
-template <class T>
-__host__ __device__ inline int blob_fields(int nc, int dirn) { return nc + dirn + (ScaledApply<T>::value ? 0 : 1); }
-// byte offset of the block of a step: rp padded rows and pp push targets precede it
-template <class T>
-__host__ __device__ inline size_t blob_offset(int rp, int pp, int fields) {
-  return (size_t)rp * (16 + sizeof(T) * fields) + 4 * (size_t)pp;
-}
-// ------------------------------------------------------------------ modes
-enum { OS_SETUP_DIC = 0, OS_SETUP_DILU, OS_FWD, OS_BWD, OS_BWD_DOT, OS_GS };
-
-// ----------------------------------------------------------- staging area
-// One stage buffer of a sweep mode, for a group of steps: the blocks, the
-// a_ii and transposes of the setups, for Gauss-Seidel a_ii and the blocks of the upper triangle, the q and e windows (rows
-// widened to 16-byte bounds) and the exchanged values.
-struct StageLayout {
-  int oX, oT, oU, oQ, oE, oI, bytes;
-  template <class T>
-  __host__ __device__ static StageLayout of(const OrdView& O, int mode) {
-    StageLayout L;
-    const int sz = (int)sizeof(T), dirn = mode == OS_BWD || mode == OS_BWD_DOT;
-    const bool setup = mode == OS_SETUP_DIC || mode == OS_SETUP_DILU, gs = mode == OS_GS;
-    int o = 0;
-    auto take = [&](bool used, int b) { const int r = o; if (used) o += (b + 15) & ~15; return r; };
-    take(true, 4 * O.g_push + (16 + blob_fields<T>(O.nc, dirn) * sz) * O.g_padded);
-    L.oX = take(setup || gs, sz * O.g_padded);
-    L.oT = take(mode == OS_SETUP_DILU, sz * O.g_padded * O.nc);
-    L.oU = take(gs, 4 * O.g_push + (16 + blob_fields<T>(O.nc, 1) * sz) * O.g_padded);
-    L.oQ = take(!setup, sz * (O.g_rows + 8));
-    L.oE = take(mode == OS_BWD_DOT || gs, sz * (O.g_rows + 8));
-    L.oI = take(true, sz * O.g_x);
-    L.bytes = o;
-    return L;
-  }
-};
-
-// stage buffers of one mode within a stage area of `area` bytes: the largest
-// power of two (at most FC_MAX_STAGES) whose buffers fit
-__host__ __device__ inline int stages_in(size_t area, int buffer_bytes) {
-  int K = 1;
-  while (2 * K <= FC_MAX_STAGES && (size_t)(2 * K) * (size_t)buffer_bytes <= area) K *= 2;
-  return K;
-}
-
-// dynamic shared memory of an ordered-sweep kernel: mbarriers, ring (and the
-// zero past its end), the stage area (cut by every sweep mode into its own
-// buffers) and the abort flag
-template <class T>
-inline size_t osweep_fixed_bytes(int R, int maxW) {
-  size_t ring = (((size_t)R * maxW + 1) * sizeof(T) + 15) & ~(size_t)15;
-  return FC_SMEM_HDR + ring + 16;
-}
 template <class T>
 inline size_t osweep_smem_bytes(int R, size_t stage_area, int maxW) {
   return osweep_fixed_bytes<T>(R, maxW) + stage_area;
