@@ -33,11 +33,14 @@
 // A stage buffer is handed over with two mbarriers: full (copies landed) and
 // empty (the compute warps are done with its steps).  A wait names a phase by
 // its parity, so it must come after the phase before it has completed and
-// before the one after it does.  With at least FC_SETS buffers that holds: a
-// set looks for step k after its own step k - FC_SETS and nobody refills the
-// buffer without it; the stager waits for every group in order; an importer
-// looks for group g - ahead (ahead <= K) after it looked for group g - ahead -
-// FC_IMP_WARPS, and group g and what follows cannot pass before it.
+// before the one after it does.  With at least FC_SETS buffers that holds for
+// the sets (a set looks for step k after its own step k - FC_SETS and nobody
+// refills the buffer without it) and for the stager, which waits for every
+// group in order.  An importer of group g looks for group g - ahead (ahead <=
+// K); what comes after cannot pass before it, as group g needs it, but what
+// was before is only known to be complete with enough buffers.  With fewer,
+// importers go by a word in which the stager counts the groups whose buffer it
+// has found free (import_ahead and import_by_parity in fc_stage.hpp).
 //
 // Measured on a GB300, FP64, per level of one tile: 350 cycles forward with 30
 // rows a level, 400 forward and 500 backward with 108 rows (the FP64 pipe
@@ -115,6 +118,28 @@ __device__ __forceinline__ bool mbar_wait_warp(unsigned mb, unsigned parity, vol
   bool ok = true;
   if ((threadIdx.x & 31) == 0) ok = mbar_wait(mb, parity, abort_flag);
   return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+}
+// The word in which the stager counts the groups whose buffer it has found
+// free: written by one lane at a time, in order; a warp waits until it reaches
+// count (bounded; false also if the block is leaving).  It wraps like the
+// counts it is compared with.
+__device__ __forceinline__ void word_publish(unsigned a, unsigned count) {
+  asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(a), "r"(count) : "memory");
+}
+__device__ __forceinline__ bool word_wait_warp(unsigned a, unsigned count, volatile int* abort_flag) {
+  bool ok = true;
+  if ((threadIdx.x & 31) == 0) {
+    unsigned v, spins = 0;
+    for (;;) {
+      asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+      if ((int)(v - count) >= 0) break;
+      if (++spins > FC_MBAR_SPIN_LIMIT || ((spins & 15u) == 0 && *abort_flag)) { ok = false; break; }
+      __nanosleep(20);
+    }
+  }
+  ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+  __syncwarp();  // orders what follows in all lanes after lane 0's wait
+  return ok;
 }
 __device__ __forceinline__ void bar_wait(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
@@ -239,6 +264,8 @@ struct OsCtx {
   int s0, ns;                 // the tile's first step, its steps
   int* abort_flag;
   unsigned parity;            // bit b: parity of the next use of stage buffer b
+  unsigned free_word;         // shared address of the stager's word
+  unsigned groups;            // groups of the sweeps before
 };
 
 template <class T>
@@ -262,8 +289,11 @@ __device__ __forceinline__ OsCtx osweep_ctx(const OrdView& O, unsigned char* sme
   off += (size_t)O.stage_area;
   X.abort_flag = (int*)(smem + off);
   X.parity = 0;
+  X.free_word = smem_addr(X.abort_flag + 1);
+  X.groups = 0;
   if (threadIdx.x == 0) {
     *X.abort_flag = 0;
+    X.abort_flag[1] = 0;
     for (int b = 0; b < FC_MAX_STAGES; ++b) {
       mbar_init(X.full + 8 * b, 1);
       mbar_init(X.empty + 8 * b, O.G * X.ncw);  // every step's warps
@@ -533,7 +563,8 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
     // ----------------------------------------------------------- importers
     constexpr int U = 4;  // polls in flight per lane
     const int* const xp = O.xv_ptr[dirn] + X.s0;
-    const int ng = (ns + G - 1) >> gshift, ahead = min(K, FC_STEP_BARS >> gshift);  // groups
+    const int ng = (ns + G - 1) >> gshift, ahead = import_ahead(K, G);  // groups
+    const bool by_parity = import_by_parity(K, G);
     bool ok = true;   // false: only the barriers are kept up
     for (int g = wid - FC_SETS * FC_SET_WARPS; g < ng; g += FC_IMP_WARPS) {
       const int k0 = g << gshift, k1 = min(k0 + G, ns), b = g & (K - 1);
@@ -554,7 +585,9 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
       };
       // the place of the values, and the barriers of the steps, are free once
       // group g - ahead is done
-      if (ok && g >= ahead) ok = mbar_wait_warp(X.empty + 8 * ((g - ahead) & (K - 1)), use_parity(g - ahead), abort_flag);
+      if (ok && g >= ahead)
+        ok = by_parity ? mbar_wait_warp(X.empty + 8 * ((g - ahead) & (K - 1)), use_parity(g - ahead), abort_flag)
+                       : word_wait_warp(X.free_word, X.groups + g + 1, abort_flag);
       if (ok) release(0);
       for (int c0 = 0; c0 < nx && ok; c0 += 32 * U) {
         unsigned pending = 0, spins = 0;
@@ -601,6 +634,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
     // copies are not ordinary loads.
     asm volatile("fence.proxy.async;" ::: "memory");
     const int ng = (ns + G - 1) >> gshift;
+    const bool by_parity = import_by_parity(K, G);
     int issued = 0;
     bool ok = true;
     for (int g0 = 0; g0 < ng && ok; g0 += 32) {
@@ -633,6 +667,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
             fail();
             ok = false;
           } else {
+            if (!by_parity) word_publish(X.free_word, X.groups + g + 1);
             if (tr) tr->staged(k0);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_arrive_tx(mb, bytes);
@@ -647,6 +682,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
           }
         }
         ok = __shfl_sync(0xffffffffu, (int)ok, j) != 0;
+        __syncwarp();  // the next lane's word comes after this one's
         issued += ok ? 1 : 0;
       }
     }
@@ -664,6 +700,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
     const int ng = (ns + G - 1) >> gshift, rounds = ng >> kshift, rest = ng & (K - 1);
     const unsigned all = (1u << K) - 1u, first = (1u << rest) - 1u;
     Xr.parity = X.parity ^ first ^ (rounds & 1 ? all : 0u);
+    Xr.groups = X.groups + (unsigned)ng;
   }
   if (MODE == OS_BWD_DOT || kGS) red_out[0] += red[0];
   if (kGS) red_out[1] += red[1];
