@@ -117,7 +117,9 @@ __device__ __forceinline__ bool mbar_wait(unsigned mb, unsigned parity, volatile
 __device__ __forceinline__ bool mbar_wait_warp(unsigned mb, unsigned parity, volatile int* abort_flag) {
   bool ok = true;
   if ((threadIdx.x & 31) == 0) ok = mbar_wait(mb, parity, abort_flag);
-  return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+  ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+  __syncwarp();  // orders what follows in all lanes after lane 0's wait: the shuffle does not
+  return ok;
 }
 // The word in which the stager counts the groups whose buffer it has found
 // free: written by one lane at a time, in order; a warp waits until it reaches
