@@ -876,9 +876,8 @@ int sys_set_pattern(fc_ctx* ctx, CsrSystem* s, int n, int nnz, const int* ia1, c
       if (nocut >= 0) continue;
     }
     if (steps_per_buffer(O, false) > 0 && (!with_gs || steps_per_buffer(O, true) > 0)) break;
-    if (chunk > FC_SET_ROWS) chunk = std::max(FC_SET_ROWS, (3 * chunk / 4) & ~31);
-    else if (chunk > 32) chunk = 32;
-    else return fc_fail_msg(ctx, FC_ERR_UNSUPPORTED, "sweep tiles too large for shared memory");
+    chunk = narrower_steps(chunk);
+    if (chunk == 0) return fc_fail_msg(ctx, FC_ERR_UNSUPPORTED, "sweep tiles too large for shared memory");
   }
   s->t_schedule = since(t0);
   s->xyz_src = xyz;

@@ -131,4 +131,14 @@ inline size_t ordered_stage_area(int R, int maxW) {
 // (see fc_sweep.cuh); 0 if none.
 int steps_per_buffer(const OrderedSweep& O, bool gs);
 
+// The most rows of a step to try next when steps of at most `chunk` rows leave
+// a mode too few stage buffers; 0: none.  Exchanged values and push targets
+// are staged, up to 255 of each a row, so that wide steps of densely coupled
+// rows do not fit; four rows always do (4 x 255 x (8 + 2 x 4) bytes a buffer).
+inline int narrower_steps(int chunk) {
+  if (chunk > FC_SET_ROWS) return std::max(FC_SET_ROWS, (3 * chunk / 4) & ~31);
+  if (chunk > 32) return 32;
+  return chunk > 4 ? std::max(4, chunk / 2) : 0;
+}
+
 }  // namespace fcdev

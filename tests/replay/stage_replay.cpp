@@ -9,6 +9,10 @@
 // parity of `empty`.  Reports buffers written before they were read, read
 // before they were written, named barriers arrived at twice and dead ends.
 //
+//   stage_replay fits file tiles
+// the widest steps that get their buffers, as the pattern analysis looks for
+// them.
+//
 //   stage_replay groups file tiles chunk
 // reads a pattern (n, nnz, ia, ja, diagonal places; 0-based) and prints the
 // groups and buffers of its sweeps; checks the steps' descriptors for G = 1, 2
@@ -177,7 +181,7 @@ int model(int K, int G, const std::string& rule) {
   return 0;
 }
 
-int groups(const char* file, int tiles, int chunk) {
+int build(const char* file, int tiles, int chunk, OrderedSweep& O) {
   FILE* f = std::fopen(file, "rb");
   if (!f) return 2;
   int head[2];
@@ -189,13 +193,33 @@ int groups(const char* file, int tiles, int chunk) {
   const bool ok = std::fread(head, sizeof(int), 2, f) == 2 && get(ia, head[0] + 1) && get(ja, head[1]) && get(dg, head[0]);
   std::fclose(f);
   if (!ok) return 2;
-  OrderedSweep O;
   SweepSchedule S;
   std::string err;
   if (!build_ordered_sweep(head[0], ia.data(), ja.data(), dg.data(), nullptr, tiles, nullptr, 4, O, S, err, 0, chunk)) {
     std::printf("%s\n", err.c_str());
     return 1;
   }
+  return 0;
+}
+
+int fits(const char* file, int tiles) {
+  for (int chunk = FC_SET_ROWS; chunk > 0; chunk = narrower_steps(chunk)) {
+    OrderedSweep O;
+    const int st = build(file, tiles, chunk, O);
+    if (st) return st;
+    const int G = steps_per_buffer(O, false), G_gs = steps_per_buffer(O, true);
+    if (!G || !G_gs) continue;
+    std::printf("rows %d G %d %d\n", chunk, G, G_gs);
+    return 0;
+  }
+  std::printf("no buffers\n");
+  return 1;
+}
+
+int groups(const char* file, int tiles, int chunk) {
+  OrderedSweep O;
+  const int st = build(file, tiles, chunk, O);
+  if (st) return st;
   int bad = 0, most = 0;
   for (int d = 0; d < 2; ++d)
     for (int q = 0; q < O.n; ++q) most = std::max(most, O.dir[d].rec[4 * (size_t)q] & 255);
@@ -243,6 +267,7 @@ int groups(const char* file, int tiles, int chunk) {
 
 int main(int argc, char** argv) {
   if (argc > 4 && !std::strcmp(argv[1], "model")) return model(std::atoi(argv[2]), std::atoi(argv[3]), argv[4]);
+  if (argc > 3 && !std::strcmp(argv[1], "fits")) return fits(argv[2], std::atoi(argv[3]));
   if (argc > 4 && !std::strcmp(argv[1], "groups")) return groups(argv[2], std::atoi(argv[3]), std::atoi(argv[4]));
   return 2;
 }

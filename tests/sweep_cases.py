@@ -61,6 +61,14 @@ def write_pattern(path, ia, ja, dg):
             f.write(np.ascontiguousarray(v, np.int32).tobytes())
 
 
+# structures whose exchanged values leave no room for steps of 32 rows: pattern, tiles
+DENSE = {
+    "hubs_16": (lambda: red_black(16, 16, 16, 40, 200), 4),
+    "hubs_24": (lambda: red_black(24, 24, 24, 40, 200), 12),
+    "blocks": (lambda: blocks_coupled(250, 250, 0), 8),
+    "most": (lambda: blocks_coupled(255, 255, 0), 3),
+}
+
 # pattern, tiles, steps of a buffer (setups and applications, Gauss-Seidel)
 STAGED = {
     "red_black": (dict(nx=24, ny=24, nz=24), 12, 2, 2),

@@ -47,3 +47,23 @@ def test_iterates(system, ctx, oracle, solver):
         assert r0 == pytest.approx(r0o, rel=1e-12)
         np.testing.assert_allclose(x, xo, rtol=0, atol=1e-10 * np.abs(xo).max())
     assert ctx.sweep_stats(1)["tiles"] == tiles
+
+
+@pytest.mark.parametrize("solver", ["iccg", "bicgstab", "gauss-seidel"])
+@pytest.mark.parametrize("name", sorted(cases.DENSE))
+def test_densely_coupled_rows(ctx, oracle, name, solver):
+    make, tiles = cases.DENSE[name]
+    ia, ja, dg, a = make()
+    b = np.random.default_rng(8).uniform(-1.0, 1.0, len(dg))
+    args = (ia + 1, ja + 1, a, dg + 1, np.zeros(len(dg)), b, 5, 1e-30, 1e-30)
+    xo, r0o, info_o, _ = oracle.solve(solver, *args)
+    ctx.set_sweep_tiles(tiles)
+    ctx.pattern_forget()
+    try:
+        x, r0, info, st = ctx.csrsolve(solver, *args)
+    finally:
+        ctx.set_sweep_tiles(0)
+        ctx.pattern_forget()
+    assert st >= 0 and info.itr_used == int(info_o[0])
+    assert r0 == pytest.approx(r0o, rel=1e-12)
+    np.testing.assert_allclose(x, xo, rtol=0, atol=1e-10 * np.abs(xo).max())

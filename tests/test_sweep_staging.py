@@ -51,3 +51,12 @@ def test_groups_of_wide_steps(replay, tmp_path, name):
     # DILU setup, backward sweep with the dot product; Gauss-Seidel
     buffers = lambda w: {w[i]: int(w[i + 1]) for i in range(4, len(w), 3)}
     assert buffers(solve)["K1"] == 4 and buffers(solve)["K4"] == 4 and buffers(gs)["K5"] == 4
+
+
+@pytest.mark.parametrize("name", sorted(cases.DENSE))
+def test_densely_coupled_rows_get_their_buffers(replay, tmp_path, name):
+    make, tiles = cases.DENSE[name]
+    path = tmp_path / "pattern.bin"
+    cases.write_pattern(path, *make()[:3])
+    out = replay("fits", path, tiles)
+    assert out.returncode == 0 and out.stdout.startswith("rows "), out.stdout + out.stderr
