@@ -327,7 +327,7 @@ struct OsRow {
   T aii, xo;            // Gauss-Seidel: diagonal, previous iterate
   T di;                 // plain applications: d_i
   int push;             // push targets | place of the first << 8
-  int ovf;              // entries | exchanged ones among the first FC_ELL << 8 | exchange offset << 16
+  int ovf;              // last word of the record
 };
 
 // One ordered sweep of tile vg_bid(C).  Directions: forward over the lower
@@ -426,7 +426,8 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
             const int s = X.s0 + k, p1 = __ldg(O.push_ptr[1] + s), p0 = __ldg(O.push_ptr[1] + X.s0 + (k & ~(G - 1)));
             const unsigned U = S + L.oU + (unsigned)(rpo * (kStride + SZ * blob_fields<T>(nc, 1)) + 4 * (p1 - p0));
             const unsigned UC = U + kStride * cp + 4 * (__ldg(O.push_ptr[1] + s + 1) - p1);
-            const int nu = lds(U + kStride * sl + 12, int()) & 255, k0 = sell_at(O, base + sl, (w.ovf & 255) + 1);
+            const int nu = FC_REC_ENTRIES(lds(U + kStride * sl + 12, int())),
+                      k0 = sell_at(O, base + sl, FC_REC_ENTRIES(w.ovf) + 1);
 #pragma unroll
             for (int e = 0; e < NC; ++e)
               w.x[e] = e < nu ? mul_rn(lds(UC + (unsigned)((e * cp + sl) * SZ), T()), ldcg(io.e + __ldg(O.sell_col + k0 + FC_SLICE * e)))
@@ -443,15 +444,15 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
           const int o = __ldg(O.ovf_ptr[dirn] + q) + e - FC_ELL;
           a = ldcg(V.aovf[dirn] + o);
           const int c = __ldg(O.ovf_code[dirn] + o);
-          return lds(c >= 0 ? X.ring + c * SZ : I + (rw + 1 + ((unsigned)w.ovf >> 16) + m++) * SZ, T());
+          return lds(c >= 0 ? X.ring + c * SZ : I + (rw + 1 + FC_REC_OFFSET(w.ovf) + m++) * SZ, T());
         };
         // the row's value from its dependencies
         auto value = [&](int sl, OsRow<T>& w) {
           T v[NC];
 #pragma unroll
           for (int e = 0; e < NC; ++e) v[e] = lds(w.at[e], T());
-          int m = (w.ovf >> 8) & 255;
-          const int ne = GEN ? w.ovf & 255 : 0, q = base + sl;
+          int m = FC_REC_EXCHANGED(w.ovf);
+          const int ne = GEN ? FC_REC_ENTRIES(w.ovf) : 0, q = base + sl;
           T val = w.acc;
           if constexpr (kSetup) {
             // d_i = a_ii - sum a_k^2 d_j (DIC) or a_k d_j a_(j,i) (DILU), then
@@ -481,7 +482,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
             val = sub_rn(val, mul_rn(w.aii, w.xo));
 #pragma unroll
             for (int e = 0; e < NC; ++e) val = sub_rn(val, w.x[e]);
-            const int nu = GEN ? __ldg(&O.rec[1][q].w) & 255 : 0;
+            const int nu = GEN ? FC_REC_ENTRIES(__ldg(&O.rec[1][q].w)) : 0;
             for (int e = FC_ELL; e < nu; ++e) {
               const int o = __ldg(O.ovf_ptr[1] + q) + e - FC_ELL;
               val = sub_rn(val, mul_rn(ldcg(V.aovf[1] + o), ldcg(io.e + __ldg(O.ovf_col[1] + o))));
@@ -749,7 +750,7 @@ __device__ void ord_gather_values(const GridCtl& C, const OrdView& O, const OrdV
     for (int sl = lane; sl < cnt; sl += 32) {
       const int q = base + sl, slice = q / FC_SLICE, off = __ldg(O.sell_ptr + slice), k0 = off + q % FC_SLICE;
       const int w = (__ldg(O.sell_ptr + slice + 1) - off) / FC_SLICE;
-      const int ne = __ldg(&O.rec[0][q].w) & 255;
+      const int ne = FC_REC_ENTRIES(__ldg(&O.rec[0][q].w));
       auto slot_of = [&](int k) { return __ldg(O.sell_slot + k0 + FC_SLICE * k); };
       auto value_of = [&](int slot) { return slot >= 0 ? __ldg(a + slot) : T(0); };
       int slot[FC_ROW_LOADS], tslot[FC_ELL];
@@ -783,7 +784,7 @@ __device__ void ord_gather_values(const GridCtl& C, const OrdView& O, const OrdV
           if (dilu) tx[e * cp + sl] = t[e];
         }
       if (gs) {
-        const int nu = __ldg(&O.rec[1][q].w) & 255;
+        const int nu = FC_REC_ENTRIES(__ldg(&O.rec[1][q].w));
         for (int e = 0; e < nc; ++e) cf[1][e * cp + sl] = e < nu ? value_of(slot_of(ne + 1 + e)) : T(0);
       }
     }
@@ -829,7 +830,7 @@ __device__ void ord_apply_values(const GridCtl& C, const OrdView& O, const OrdVa
       const int q = base + sl, k0 = sell_at(O, q, 0);
       auto entry = [&](int k) { return ldcg(V.ap + k0 + FC_SLICE * k); };
       auto column = [&](int k) { return __ldg(O.sell_col + k0 + FC_SLICE * k); };
-      const int ne = __ldg(&O.rec[0][q].w) & 255, nu = __ldg(&O.rec[1][q].w) & 255;
+      const int ne = FC_REC_ENTRIES(__ldg(&O.rec[0][q].w)), nu = FC_REC_ENTRIES(__ldg(&O.rec[1][q].w));
       const T di = ldcg(d + q);
       T lo[FC_ELL], up[FC_ELL], dj[FC_ELL];
       int col[FC_ELL];

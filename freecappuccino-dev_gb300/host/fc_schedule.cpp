@@ -740,6 +740,7 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
     for (int q = 0; q < n; ++q) {
       const int np = cons_ptr[q + 1] - cons_ptr[q];
       if (nx[q] > 255 || np > 255) { derr = "ordered sweep: more than 255 exchanged entries in a row"; return false; }
+      if (D.ne[q] > FC_REC_MAX_ENTRIES) { derr = "ordered sweep: more than 8191 entries in a row"; return false; }
       D.srec[4 * (size_t)q] = D.ne[q] | (np << 8) | (xoff[q] << 16);
       D.srec[4 * (size_t)q + 1] = poff[q];
       {
@@ -756,7 +757,7 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
         r[0] = np | (poff[q] << 8);
         r[1] = (int)(place[0] | (place[1] << 16));
         r[2] = (int)(place[2] | (place[3] << 16));
-        r[3] = D.ne[q] | (mx << 8) | (xoff[q] << 16);
+        r[3] = FC_REC_PACK(D.ne[q], mx, xoff[q]);
       }
       for (int m = 0; m < np; ++m) {
         const int qc = cons_q[cons_ptr[q] + m], mc = cons_m[cons_ptr[q] + m];

@@ -87,6 +87,16 @@ double estimate_sweep_us(const SweepSchedule& S, double tau0, double per_row, do
 #define FC_ELL 4
 #define FC_RING_BYTES (64 * 1024)  // most shared memory of a value ring deepened for chunked levels
 
+// Last word of a row record: the row's entries, the exchanged ones among the
+// first FC_ELL of them, its first exchanged value in the step's block.  A row
+// served by the ring may have as many entries as the ring has values; in 8 bits
+// rows of more than 255 were solved with a truncated count.
+#define FC_REC_MAX_ENTRIES 8191
+#define FC_REC_PACK(entries, exchanged, offset) ((entries) | ((exchanged) << 13) | (int)((unsigned)(offset) << 16))
+#define FC_REC_ENTRIES(w) ((w) & FC_REC_MAX_ENTRIES)
+#define FC_REC_EXCHANGED(w) (((w) >> 13) & 7)
+#define FC_REC_OFFSET(w) ((unsigned)(w) >> 16)
+
 struct OrderedDir {
   std::vector<int> ne;        // [nE] entries of this triangle in the row
   std::vector<int> slot;      // [FC_ELL*nE] original CSR slot, -1 past ne (coefficient gather)
@@ -103,7 +113,7 @@ struct OrderedDir {
   //   [1], [2] places of the values of entries 0..3, 16 bits each: a ring
   //       index (below R * W of the tile), R * W: a zero (past the row's
   //       entries), R * W + 1 + j: value j of the step's exchange block
-  //   [3] ne | exchanged entries among 0..3 << 8 | xoff << 16
+  //   [3] FC_REC_ENTRIES, FC_REC_EXCHANGED, FC_REC_OFFSET below
   std::vector<int> rec;
   std::vector<int> xv_ptr;    // [nsteps+1] exchange block of each step
   std::vector<int> push_ptr;  // [nsteps+1] push block of each step (multiples of 4)
