@@ -189,6 +189,9 @@ void build_sweep_schedule(int n, const int* ia, const int* ja, const int* dg, co
   const long long target = (n + T - 1) / T;
   std::vector<int> tile_of_chain(nch, -1);
   std::vector<long long> tile_rows;
+  // chains that lie in one point (or nowhere) cannot be told apart by
+  // coordinates: their tiles are grown as well
+  bool cut = false;
   if (xyz) {
     std::vector<double> cx(nch, 0.0), cy(nch, 0.0), cz(nch, 0.0);
     for (int i = 0; i < n; ++i) {
@@ -207,20 +210,24 @@ void build_sweep_schedule(int n, const int* ia, const int* ja, const int* dg, co
     int slabs[3];
     S.cut_axes = cut_counts(T, ext, nocut, slabs);
     if (nocut == FC_CUT_UNLESS_3 && S.cut_axes == 3) return;
-    int ax[3] = {0, 1, 2};  // the longest axes first
-    std::stable_sort(ax, ax + 3, [&](int p, int q) { return ext[p] > ext[q]; });
-    axis_cuts(items, cen, chain_rows, ax, slabs, 0, T, 0, tile_of_chain);
-    // drop empty parts
-    std::vector<int> used(T, 0);
-    for (int c = 0; c < nch; ++c) used[tile_of_chain[c]] = 1;
-    std::vector<int> nid(T, -1);
-    int m = 0;
-    for (int t = 0; t < T; ++t)
-      if (used[t]) nid[t] = m++;
-    for (int c = 0; c < nch; ++c) tile_of_chain[c] = nid[tile_of_chain[c]];
-    tile_rows.assign(m, 0);
-    for (int c = 0; c < nch; ++c) tile_rows[tile_of_chain[c]] += chain_rows[c];
-  } else {
+    cut = S.cut_axes > 0 || T == 1;
+    if (cut) {
+      int ax[3] = {0, 1, 2};  // the longest axes first
+      std::stable_sort(ax, ax + 3, [&](int p, int q) { return ext[p] > ext[q]; });
+      axis_cuts(items, cen, chain_rows, ax, slabs, 0, T, 0, tile_of_chain);
+      // drop empty parts
+      std::vector<int> used(T, 0);
+      for (int c = 0; c < nch; ++c) used[tile_of_chain[c]] = 1;
+      std::vector<int> nid(T, -1);
+      int m = 0;
+      for (int t = 0; t < T; ++t)
+        if (used[t]) nid[t] = m++;
+      for (int c = 0; c < nch; ++c) tile_of_chain[c] = nid[tile_of_chain[c]];
+      tile_rows.assign(m, 0);
+      for (int c = 0; c < nch; ++c) tile_rows[tile_of_chain[c]] += chain_rows[c];
+    }
+  }
+  if (!cut) {
     chain_graph();
     std::deque<int> q;
     int next_seed = 0;

@@ -4,10 +4,13 @@
 // the exchanged values of its further entries, its pushes.  Forward and backward
 // substitution, bit for bit against the plain ones in the original numbering.
 //
-//   record_replay file tiles chunk    (pattern: n, nnz, ia, ja, diagonal places; 0-based)
+//   record_replay file tiles chunk [coords]    (pattern: n, nnz, ia, ja, diagonal places; 0-based)
+//
+// coords: none; or "same", "nan", "inf": rows that all lie in one point, or nowhere.
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <limits>
 #include <random>
 #include <string>
 #include <vector>
@@ -31,8 +34,11 @@ int main(int argc, char** argv) {
   OrderedSweep O;
   SweepSchedule S;
   std::string err;
-  if (!build_ordered_sweep(n, ia.data(), ja.data(), dg.data(), nullptr, std::atoi(argv[2]), nullptr, 4, O, S, err, 0,
-                           std::atoi(argv[3]))) {
+  const std::string where = argc > 4 ? argv[4] : "";
+  const double at = where == "nan" ? std::nan("") : where == "inf" ? std::numeric_limits<double>::infinity() : 1.5;
+  const std::vector<double> xyz(where.empty() ? 0 : 3 * (size_t)n, at);
+  if (!build_ordered_sweep(n, ia.data(), ja.data(), dg.data(), nullptr, std::atoi(argv[2]),
+                           where.empty() ? nullptr : xyz.data(), 4, O, S, err, 0, std::atoi(argv[3]))) {
     std::printf("refused: %s\n", err.c_str());
     return 0;
   }

@@ -61,3 +61,12 @@ def test_rows_of_more_entries_than_a_record_counts(replay, tmp_path):
     cases.write_pattern(path, *cases.blocks_coupled(8192, 2, 0)[:3])
     out = replay(path, 1, 2048)
     assert out.returncode == 0 and out.stdout.startswith("refused"), out.stdout + out.stderr
+
+
+@pytest.mark.parametrize("where", ["same", "nan", "inf"])
+def test_rows_without_distinct_coordinates_get_their_tiles(replay, tmp_path, where):
+    path = tmp_path / "pattern.bin"
+    cases.write_pattern(path, *cases.red_black(16, 16, 16)[:3])
+    plain, out = replay(path, 12, 128), replay(path, 12, 128, where)
+    assert out.returncode == 0 and out.stdout == plain.stdout, out.stdout + out.stderr
+    assert int(out.stdout.split()[1]) == 12
