@@ -25,16 +25,21 @@ struct Deps {
 
 }  // namespace
 
-// body(i) for i in [0, count) on up to hardware_concurrency threads, this one
-// among them; on fewer where no more can be started
+// Rows from which the choice of the tiles uses threads: one takes 30 us to
+// start, as long as a trial on 3,000 rows (1,386 rows on 16 Arm cores: 0.6 ms
+// more with threads).
+#define FC_THREADS_ROWS 8192
+
+// body(i) for i in [0, count) on up to `most` and hardware_concurrency threads,
+// this one among them; on fewer where no more can be started
 template <class F>
-static void parallel_items(int count, F body) {
+static void parallel_items(int count, int most, F body) {
   std::atomic<int> next{0};
   auto work = [&]() {
     for (int i = next++; i < count; i = next++) body(i);
   };
   std::vector<std::thread> th;
-  const int nt = std::min(count, (int)std::thread::hardware_concurrency());
+  const int nt = std::min(std::min(count, most), (int)std::thread::hardware_concurrency());
   try {
     for (int k = 1; k < nt; ++k) th.emplace_back(work);
   } catch (const std::system_error&) {
@@ -130,7 +135,7 @@ static void axis_cuts(std::vector<int>& items, const std::vector<double>* const 
     axis_cuts(slab[s], c, w, ax, slabs, level + 1, parts_before(s + 1) - p0, first_part + p0, part_of, false);
   };
   if (threads && !last && items.size() > 4096) {
-    parallel_items(np, run);
+    parallel_items(np, np, run);
   } else {
     for (int s = 0; s < np; ++s) run(s);
   }
@@ -534,13 +539,15 @@ struct LevelOrder {
     for (int i = 0; i < n; ++i) row[pos[i] = at[lev[i]]++] = i;
     for (int q = 0; q < n; ++q) dep_ptr[q + 1] = dep_ptr[q] + G.D.end(row[q]) - G.D.begin(row[q]);
     dep.resize(dep_ptr[n]);
-    parallel_chunks(n, [&](int lo, int hi) {
+    auto fill = [&](int lo, int hi) {
       for (int q = lo; q < hi; ++q) {
         const int i = row[q], k0 = G.D.begin(i);
         chain[q] = G.of[i];
         for (int e = dep_ptr[q]; e < dep_ptr[q + 1]; ++e) dep[e] = pos[G.D.ja[k0 + e - dep_ptr[q]]];
       }
-    });
+    };
+    if (n > FC_THREADS_ROWS) parallel_chunks(n, fill);
+    else fill(0, n);
   }
 };
 
@@ -589,7 +596,7 @@ int pick_sweep_tiles(int n, const int* ia, const int* ja, const int* dg, const d
   const LevelOrder L(G, lev, nls);
   struct Trial { int c, out; double est; bool cut3; };
   auto run = [&](std::vector<Trial>& tr) {
-    parallel_items((int)tr.size(), [&](int k) {
+    parallel_items((int)tr.size(), n > FC_THREADS_ROWS ? (int)tr.size() : 1, [&](int k) {
       Trial& t = tr[k];
       std::vector<int> tile_of_chain;
       int cut_axes = 0;
