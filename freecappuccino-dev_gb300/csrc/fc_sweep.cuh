@@ -264,9 +264,8 @@ struct OsCtx {
   unsigned ring, stage;       // shared addresses
   int W, ncw;                 // the tile's widest step; compute warps of a set
   int s0, ns;                 // the tile's first step, its steps
-  int* abort_flag;
+  int* abort_flag;            // the stager's word after it
   unsigned parity;            // bit b: parity of the next use of stage buffer b
-  unsigned free_word;         // shared address of the stager's word
   unsigned groups;            // groups of the sweeps before
 };
 
@@ -291,7 +290,6 @@ __device__ __forceinline__ OsCtx osweep_ctx(const OrdView& O, unsigned char* sme
   off += (size_t)O.stage_area;
   X.abort_flag = (int*)(smem + off);
   X.parity = 0;
-  X.free_word = smem_addr(X.abort_flag + 1);
   X.groups = 0;
   if (threadIdx.x == 0) {
     *X.abort_flag = 0;
@@ -361,6 +359,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
   const int kshift = __ffs(K) - 1, gshift = __ffs(G) - 1;  // both powers of two
   T* const xv = V.xv[dirn];
   volatile int* const abort_flag = X.abort_flag;
+  const unsigned free_word = smem_addr(X.abort_flag + 1);
   const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5;
   double red[2] = {0.0, 0.0};
   auto step_of = [&](int k) { return dirn ? ns - 1 - k : k; };
@@ -590,7 +589,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
       // group g - ahead is done
       if (ok && g >= ahead)
         ok = by_parity ? mbar_wait_warp(X.empty + 8 * ((g - ahead) & (K - 1)), use_parity(g - ahead), abort_flag)
-                       : word_wait_warp(X.free_word, X.groups + g + 1, abort_flag);
+                       : word_wait_warp(free_word, X.groups + g + 1, abort_flag);
       if (ok) release(0);
       for (int c0 = 0; c0 < nx && ok; c0 += 32 * U) {
         unsigned pending = 0, spins = 0;
@@ -670,7 +669,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
             fail();
             ok = false;
           } else {
-            if (!by_parity) word_publish(X.free_word, X.groups + g + 1);
+            if (!by_parity) word_publish(free_word, X.groups + g + 1);
             if (tr) tr->staged(k0);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_arrive_tx(mb, bytes);

@@ -95,7 +95,12 @@ inline size_t osweep_fixed_bytes(int R, int maxW) {
 // The importer of group g fills the exchanged values of the buffer that group
 // g - K used, and releases steps whose named barriers the steps FC_STEP_BARS
 // before used: both are free once group g - import_ahead is done.
-FC_STAGE_HD int import_ahead(int K, int G) { return K < FC_STEP_BARS / G ? K : FC_STEP_BARS / G; }
+// (Both functions run at the start of every sweep, where a division costs a
+// hundredth of a short one; G is FC_SETS, 2 or 1.)
+FC_STAGE_HD int import_ahead(int K, int G) {
+  const int most = G == FC_SETS ? FC_STEP_BARS / FC_SETS : G == 2 ? FC_STEP_BARS / 2 : FC_STEP_BARS;
+  return K < most ? K : most;
+}
 
 // How it learns that.  By the parity of that group's `empty` barrier, the use
 // before must be known to be complete (else the test answers for the phase
@@ -106,7 +111,7 @@ FC_STAGE_HD int import_ahead(int K, int G) { return K < FC_STEP_BARS / G ? K : F
 // is group g - ahead - K, so the parity tells for K >= FC_IMP_WARPS +
 // FC_SETS / G.  Below (four buffers of one or two steps) ahead is K, and the
 // stager, which waits for all groups in order, says how far it has come.
-FC_STAGE_HD bool import_by_parity(int K, int G) { return K >= FC_IMP_WARPS + FC_SETS / G; }
+FC_STAGE_HD bool import_by_parity(int K, int G) { return K * G >= FC_IMP_WARPS * G + FC_SETS; }
 
 // A structure's steps in groups of G, one stage buffer each: the largest group
 // and, with desc, the descriptors of the steps (OrdView::desc).
