@@ -114,7 +114,7 @@ struct DevOrdered {
   DVec<int> tile_step_ptr, step_ptr, rp_ptr, tile_W, perm;
   DVec<int> rec[2], xv_ptr[2], push_ptr[2], push[2];
   DVec<int> ovf_ptr[2], ovf_code[2], ovf_col[2], ovf_slot[2];
-  DVec<int> lo_tslot, lo_ovf_tslot, p_ptr, p_col, p_slot, sell_ptr, sell_col, sell_slot;
+  DVec<int> lo_tslot, lo_ovf_tslot, sell_ptr, sell_col, sell_slot;
   size_t nsell = 0;                  // entries of the sliced matrix
   long long ring_entries = 0, pushed_entries = 0, cross_tile_entries = 0;
 };

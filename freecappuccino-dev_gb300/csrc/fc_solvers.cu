@@ -739,9 +739,6 @@ static int upload_ordered(fc_ctx* ctx, const OrderedSweep& O, DevOrdered& D, boo
   }
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.lo_tslot, O.lo_tslot));
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.lo_ovf_tslot, O.lo_ovf_tslot));
-  FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.p_ptr, O.p_ptr));
-  FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.p_col, O.p_col));
-  FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.p_slot, O.p_slot));
   // the matrix in slices
   const int nsl = (O.n + FC_SLICE - 1) / FC_SLICE;
   std::vector<int> sell_ptr(nsl + 1, 0);
@@ -757,10 +754,19 @@ static int upload_ordered(fc_ctx* ctx, const OrderedSweep& O, DevOrdered& D, boo
   FC_CUDA_TRY(ctx, upload_vec(ctx->stream, D.sell_ptr, sell_ptr));
   FC_CUDA_TRY(ctx, D.sell_col.alloc(D.nsell));
   FC_CUDA_TRY(ctx, D.sell_slot.alloc(D.nsell));
-  k_sell<<<std::max(1, std::min(4096, (nsl + 7) / 8)), 256, 0, ctx->stream>>>(O.n, D.p_ptr.p, D.p_col.p, D.p_slot.p,
-                                                                            D.sell_ptr.p, D.sell_col.p, D.sell_slot.p);
+  // the rows in new order, given back once the slices are written
+  const size_t np = O.p_ptr.size(), nnz = O.p_col.size();
+  DVec<int> rows;
+  FC_CUDA_TRY(ctx, rows.alloc(np + 2 * nnz));
+  int *p_ptr = rows.p, *p_col = p_ptr + np, *p_slot = p_col + nnz;
+  FC_CUDA_TRY(ctx, fc_h2d(ctx->stream, p_ptr, O.p_ptr.data(), np * sizeof(int)));
+  FC_CUDA_TRY(ctx, fc_h2d(ctx->stream, p_col, O.p_col.data(), nnz * sizeof(int)));
+  FC_CUDA_TRY(ctx, fc_h2d(ctx->stream, p_slot, O.p_slot.data(), nnz * sizeof(int)));
+  k_sell<<<std::max(1, std::min(4096, (nsl + 7) / 8)), 256, 0, ctx->stream>>>(O.n, p_ptr, p_col, p_slot, D.sell_ptr.p,
+                                                                            D.sell_col.p, D.sell_slot.p);
   ctx->kernel_launches++;
   FC_CUDA_TRY(ctx, cudaGetLastError());
+  FC_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   return FC_OK;
 }
 
