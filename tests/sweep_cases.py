@@ -4,6 +4,14 @@ staging, on the CPU and on the GPU)."""
 import numpy as np
 
 
+def grid(nx, ny, nz, seed=1):
+    """Seven-point pattern in its natural numbering (five-point for nz = 1)."""
+    i = np.arange(nx * ny * nz).reshape(nz, ny, nx)
+    pairs = [np.stack([i[:-1].ravel(), i[1:].ravel()]), np.stack([i[:, :-1].ravel(), i[:, 1:].ravel()]),
+             np.stack([i[:, :, :-1].ravel(), i[:, :, 1:].ravel()])]
+    return symmetric(nx * ny * nz, np.concatenate(pairs, axis=1), np.random.default_rng(seed))
+
+
 def red_black(nx, ny, nz, hubs=0, spokes=0, seed=1):
     """Symmetric seven-point pattern, cells of one colour numbered first, and
     `hubs` of them coupled to `spokes` cells of the other colour each; values
@@ -39,7 +47,8 @@ def blocks_coupled(n1, n2, between, seed=2):
 
 
 def symmetric(n, pairs, rng):
-    p = np.unique(np.sort(pairs, axis=0), axis=1)
+    key = np.unique(np.min(pairs, axis=0).astype(np.int64) * n + np.max(pairs, axis=0))
+    p = np.stack([key // n, key % n])
     v = -rng.uniform(0.5, 1.5, p.shape[1])
     diag = np.zeros(n)
     np.add.at(diag, p[0], -1.1 * v)
