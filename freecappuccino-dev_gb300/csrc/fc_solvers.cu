@@ -873,7 +873,7 @@ int sys_set_pattern(fc_ctx* ctx, CsrSystem* s, int n, int nnz, const int* ia1, c
   if (ctx->stage_rows > 0) chunk = wide && with_gs ? 32 : ctx->stage_rows;
   for (;;) {
     if (!build_ordered_sweep(n, ia.data(), ja.data(), dg.data(), ts.data(), tiles, xyz, FC_RING, O, S, err,
-                             ctx->sweep_cap, chunk, nocut))
+                             ctx->sweep_cap, chunk, nocut, false))
       return fc_fail_msg(ctx, FC_ERR_BAD_INPUT, err);
     if (tiles_req > 0 && nocut < 0 && S.cut_axes == 3) {
       // a given tile count: the axis to leave out is still chosen

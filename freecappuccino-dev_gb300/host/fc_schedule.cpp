@@ -692,7 +692,7 @@ static int split_wide_levels(int n, const int* ia, const int* ja, const int* dg,
 
 bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, const int* ts, int ntiles,
                          const double* xyz, int R, OrderedSweep& O, SweepSchedule& S, std::string& err, int wmax,
-                         int chunk, int nocut) {
+                         int chunk, int nocut, bool checks) {
   O = OrderedSweep();
   O.n = n;
   O.R = std::max(2, R);
@@ -765,9 +765,11 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
   auto build_dir = [&](int dirn, std::string& derr) -> bool {
     OrderedDir& D = O.dir[dirn];
     D.ne.assign(nE, 0);
-    D.slot.assign(E, -1);
-    D.col.assign(E, 0);
-    D.srec.assign((size_t)4 * nE, 0);
+    if (checks) {
+      D.slot.assign(E, -1);
+      D.col.assign(E, 0);
+      D.srec.assign((size_t)4 * nE, 0);
+    }
     D.rec.assign((size_t)4 * nE, 0);
     D.ovf_ptr.assign(n + 1, 0);
     for (int q = 0; q < n; ++q) {
@@ -816,9 +818,11 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
           D.ring_entries++;
         }
         if (e < FC_ELL) {
-          D.slot[(size_t)e * nE + q] = k;
-          D.col[(size_t)e * nE + q] = qj;
           codes[e] = c + 1;
+          if (checks) {
+            D.slot[(size_t)e * nE + q] = k;
+            D.col[(size_t)e * nE + q] = qj;
+          }
         } else {
           const int o = D.ovf_ptr[q] + e - FC_ELL;
           D.ovf_slot[o] = k;
@@ -826,8 +830,9 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
           D.ovf_col[o] = qj;
         }
       }
-      D.srec[4 * (size_t)q + 2] = codes[0] | (codes[1] << 16);
-      D.srec[4 * (size_t)q + 3] = codes[2] | (codes[3] << 16);
+      // the codes wait where the places will be
+      D.rec[4 * (size_t)q + 1] = codes[0] | (codes[1] << 16);
+      D.rec[4 * (size_t)q + 2] = codes[2] | (codes[3] << 16);
     }
     std::vector<int> cons_ptr(n + 1, 0), cons_q(push_src.size()), cons_m(push_src.size());
     for (int qj : push_src) cons_ptr[qj + 1]++;
@@ -865,19 +870,24 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
       const int np = cons_ptr[q + 1] - cons_ptr[q];
       if (nx[q] > 255 || np > 255) { derr = "ordered sweep: more than 255 exchanged entries in a row"; return false; }
       if (D.ne[q] > FC_REC_MAX_ENTRIES) { derr = "ordered sweep: more than 8191 entries in a row"; return false; }
-      D.srec[4 * (size_t)q] = D.ne[q] | (np << 8) | (xoff[q] << 16);
-      D.srec[4 * (size_t)q + 1] = poff[q];
+      int* r = D.rec.data() + 4 * (size_t)q;
+      if (checks) {
+        int* const s = D.srec.data() + 4 * (size_t)q;
+        s[0] = D.ne[q] | (np << 8) | (xoff[q] << 16);
+        s[1] = poff[q];
+        s[2] = r[1];
+        s[3] = r[2];
+      }
       {
         const int rw = O.R * O.tile_W[row_tile[O.perm[q]]];
         unsigned place[FC_ELL];
         int mx = 0;
         for (int e = 0; e < FC_ELL; ++e) {
-          const unsigned c1 = ((unsigned)D.srec[4 * (size_t)q + 2 + e / 2] >> (16 * (e & 1))) & 0xFFFFu;
+          const unsigned c1 = ((unsigned)r[1 + e / 2] >> (16 * (e & 1))) & 0xFFFFu;
           if (c1 > 0) place[e] = c1 - 1;
           else if (e < D.ne[q]) place[e] = rw + 1 + xoff[q] + mx++;
           else place[e] = rw;
         }
-        int* r = D.rec.data() + 4 * (size_t)q;
         r[0] = np | (poff[q] << 8);
         r[1] = (int)(place[0] | (place[1] << 16));
         r[2] = (int)(place[2] | (place[3] << 16));
@@ -902,11 +912,11 @@ bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, con
   // ---- DILU transpose slots of the lower entries, diagonal slots, matrix
   O.lo_tslot.assign(E, 0);
   O.lo_ovf_tslot.assign(O.dir[0].ovf_ptr[n], 0);
-  O.dslot.assign(nE, 0);
+  if (checks) O.dslot.assign(nE, 0);
   O.p_ptr.assign(n + 1, 0);
   for (int q = 0; q < n; ++q) {
     const int i = O.perm[q];
-    O.dslot[q] = dg[i];
+    if (checks) O.dslot[q] = dg[i];
     O.p_ptr[q + 1] = O.p_ptr[q] + (ia[i + 1] - ia[i]);
     for (int e = 0; e < O.dir[0].ne[q]; ++e) {
       const int k = ia[i] + e;

@@ -99,21 +99,24 @@ double estimate_sweep_us(const SweepSchedule& S, double tau0, double per_row, do
 
 struct OrderedDir {
   std::vector<int> ne;        // [nE] entries of this triangle in the row
-  std::vector<int> slot;      // [FC_ELL*nE] original CSR slot, -1 past ne (coefficient gather)
-  std::vector<int> col;       // [FC_ELL*nE] new index of the entry's column
-  // [4*nE] packed row record, one 16-byte load per row:
+  // For checks only (the kernels read rec and the slices): the original CSR
+  // slots of the first FC_ELL entries, -1 past ne, the new indices of their
+  // columns, [FC_ELL*nE], and [4*nE] a row record with the codes themselves, for
+  // rows of up to 255 entries:
+  std::vector<int> slot;
+  std::vector<int> col;
   //   [0] ne | np << 8 | xoff << 16   (np: pushes of the row's value; xoff:
   //       first exchange slot of the row in its step's exchange block)
   //   [1] poff: first push target of the row in its step's push block
   //   [2], [3] codes of entries 0..3, 16 bits each, stored as code + 1
   //       (0: the value arrives through the exchange block)
   std::vector<int> srec;
-  // [4*nE] the same record as the kernels read it:
+  // [4*nE] the row record as the kernels read it, one 16-byte load per row:
   //   [0] np | poff << 8
   //   [1], [2] places of the values of entries 0..3, 16 bits each: a ring
   //       index (below R * W of the tile), R * W: a zero (past the row's
   //       entries), R * W + 1 + j: value j of the step's exchange block
-  //   [3] FC_REC_ENTRIES, FC_REC_EXCHANGED, FC_REC_OFFSET below
+  //   [3] FC_REC_ENTRIES, FC_REC_EXCHANGED, FC_REC_OFFSET above
   std::vector<int> rec;
   std::vector<int> xv_ptr;    // [nsteps+1] exchange block of each step
   std::vector<int> push_ptr;  // [nsteps+1] push block of each step (multiples of 4)
@@ -135,7 +138,7 @@ struct OrderedSweep {
   OrderedDir dir[2];               // 0: left of the diagonal (forward), 1: right (backward)
   std::vector<int> lo_tslot;       // [FC_ELL*nE] transpose slot of each lower entry (DILU)
   std::vector<int> lo_ovf_tslot;
-  std::vector<int> dslot;          // [nE] original diagonal slot (0 in the padding)
+  std::vector<int> dslot;          // [nE] original diagonal slot, 0 in the padding (for checks only)
   std::vector<int> p_ptr, p_col, p_slot;  // the matrix in new numbering, entries in original order
 };
 
@@ -144,14 +147,15 @@ struct OrderedSweep {
 int symmetric_levels(int n, const int* ia, const int* ja, const int* dg, std::vector<int>& lev);
 
 // The tile count among cand whose forward schedule has the smallest
-// critical-path estimate (the trials are built concurrently, one thread
-// each; ties go to the earlier candidate, duplicates and counts < 1 are
-// skipped).  best_est (optional) receives that estimate.  With nocut, and
-// where the chains spread along all three axes, every second count is tried
-// with each axis left out of the cuts (and the first two with all of them), and *nocut
-// receives the best one (-1: none): on tetrahedra a cut along one of the axes can separate chains that
-// depend on each other both ways, which makes the tiles wait for each other
-// at every level (750k tetrahedra, 150 tiles: 250 such pairs of tiles and an
+// critical-path estimate, worked out from the tiles alone (large systems: on
+// as many threads as there are cores; ties go to the earlier candidate,
+// duplicates and counts < 1 are skipped).  best_est (optional) receives that
+// estimate.  With nocut, and where the chains spread along all three axes,
+// every second count is tried with each axis left out of the cuts (and the
+// first two with all of them), and *nocut receives the best one (-1: none): on
+// tetrahedra a cut along one of the axes can separate chains that depend on
+// each other both ways, which makes the tiles wait for each other at every
+// level (750k tetrahedra, 150 tiles: 250 such pairs of tiles and an
 // estimate of 152 us with all axes cut, none and 55 us without one of them).
 int pick_sweep_tiles(int n, const int* ia, const int* ja, const int* dg, const double* xyz, const std::vector<int>& cand,
                      double tau0, double per_row, double hop, double* best_est, int* nocut = nullptr);
@@ -160,9 +164,9 @@ int pick_sweep_tiles(int n, const int* ia, const int* ja, const int* dg, const d
 // ntiles the tile target; xyz (optional) row coordinates for the tiling; R
 // the ring depth; wmax > 0 caps the rows of a level in a tile by splitting
 // levels (and cutting the tiles again); chunk > 0 caps the rows of a step as
-// described above; nocut as above.  S receives the underlying tiled schedule (for the
-// critical-path estimate).  Returns false with a message if a consistency
-// check fails.
+// described above; nocut as above; checks fills in the arrays kept for checks
+// alone.  S receives the underlying tiled schedule (for the critical-path
+// estimate).  Returns false with a message if a consistency check fails.
 bool build_ordered_sweep(int n, const int* ia, const int* ja, const int* dg, const int* ts, int ntiles,
                          const double* xyz, int R, OrderedSweep& O, SweepSchedule& S, std::string& err,
-                         int wmax = 0, int chunk = 0, int nocut = -1);
+                         int wmax = 0, int chunk = 0, int nocut = -1, bool checks = true);
