@@ -121,20 +121,21 @@ __device__ __forceinline__ bool mbar_wait_warp(unsigned mb, unsigned parity, vol
   __syncwarp();  // orders what follows in all lanes after lane 0's wait: the shuffle does not
   return ok;
 }
-// The word in which the stager counts the groups whose buffer it has found
-// free: written by one lane at a time, in order; a warp waits until it reaches
-// count (bounded; false also if the block is leaving).  It wraps like the
-// counts it is compared with.
-__device__ __forceinline__ void word_publish(unsigned a, unsigned count) {
+// The word in which the stager counts the groups of a sweep whose buffer it
+// has found free: written by one lane at a time, in order; a warp waits until it
+// reaches count (bounded; false also if the block is leaving).  Sweeps take two
+// words in turn, and the stager clears the other one, which nobody reads then.
+__device__ __forceinline__ void word_publish(unsigned a, int count) {
   asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(a), "r"(count) : "memory");
 }
-__device__ __forceinline__ bool word_wait_warp(unsigned a, unsigned count, volatile int* abort_flag) {
+__device__ __forceinline__ bool word_wait_warp(unsigned a, int count, volatile int* abort_flag) {
   bool ok = true;
   if ((threadIdx.x & 31) == 0) {
-    unsigned v, spins = 0;
+    int v;
+    unsigned spins = 0;
     for (;;) {
       asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-      if ((int)(v - count) >= 0) break;
+      if (v >= count) break;
       if (++spins > FC_MBAR_SPIN_LIMIT || ((spins & 15u) == 0 && *abort_flag)) { ok = false; break; }
       __nanosleep(20);
     }
@@ -264,9 +265,8 @@ struct OsCtx {
   unsigned ring, stage;       // shared addresses
   int W, ncw;                 // the tile's widest step; compute warps of a set
   int s0, ns;                 // the tile's first step, its steps
-  int* abort_flag;            // the stager's word after it
-  unsigned parity;            // bit b: parity of the next use of stage buffer b
-  unsigned groups;            // groups of the sweeps before
+  int* abort_flag;            // the stager's words after it
+  unsigned parity;            // bit b: parity of the next use of stage buffer b; bit 31: of the next sweep
 };
 
 template <class T>
@@ -290,10 +290,9 @@ __device__ __forceinline__ OsCtx osweep_ctx(const OrdView& O, unsigned char* sme
   off += (size_t)O.stage_area;
   X.abort_flag = (int*)(smem + off);
   X.parity = 0;
-  X.groups = 0;
   if (threadIdx.x == 0) {
     *X.abort_flag = 0;
-    X.abort_flag[1] = 0;
+    X.abort_flag[1] = X.abort_flag[2] = 0;
     for (int b = 0; b < FC_MAX_STAGES; ++b) {
       mbar_init(X.full + 8 * b, 1);
       mbar_init(X.empty + 8 * b, O.G * X.ncw);  // every step's warps
@@ -359,7 +358,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
   const int kshift = __ffs(K) - 1, gshift = __ffs(G) - 1;  // both powers of two
   T* const xv = V.xv[dirn];
   volatile int* const abort_flag = X.abort_flag;
-  const unsigned free_word = smem_addr(X.abort_flag + 1);
+  const unsigned free_word = smem_addr(X.abort_flag + 1 + (X.parity >> 31));
   const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5;
   double red[2] = {0.0, 0.0};
   auto step_of = [&](int k) { return dirn ? ns - 1 - k : k; };
@@ -589,7 +588,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
       // group g - ahead is done
       if (ok && g >= ahead)
         ok = by_parity ? mbar_wait_warp(X.empty + 8 * ((g - ahead) & (K - 1)), use_parity(g - ahead), abort_flag)
-                       : word_wait_warp(free_word, X.groups + g + 1, abort_flag);
+                       : word_wait_warp(free_word, g + 1, abort_flag);
       if (ok) release(0);
       for (int c0 = 0; c0 < nx && ok; c0 += 32 * U) {
         unsigned pending = 0, spins = 0;
@@ -637,6 +636,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
     asm volatile("fence.proxy.async;" ::: "memory");
     const int ng = (ns + G - 1) >> gshift;
     const bool by_parity = import_by_parity(K, G);
+    if (lane == 0) X.abort_flag[1 + ((X.parity >> 31) ^ 1u)] = 0;
     int issued = 0;
     bool ok = true;
     for (int g0 = 0; g0 < ng && ok; g0 += 32) {
@@ -669,7 +669,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
             fail();
             ok = false;
           } else {
-            if (!by_parity) word_publish(free_word, X.groups + g + 1);
+            if (!by_parity) word_publish(free_word, g + 1);
             if (tr) tr->staged(k0);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_arrive_tx(mb, bytes);
@@ -701,8 +701,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
   {
     const int ng = (ns + G - 1) >> gshift, rounds = ng >> kshift, rest = ng & (K - 1);
     const unsigned all = (1u << K) - 1u, first = (1u << rest) - 1u;
-    Xr.parity = X.parity ^ first ^ (rounds & 1 ? all : 0u);
-    Xr.groups = X.groups + (unsigned)ng;
+    Xr.parity = X.parity ^ first ^ (rounds & 1 ? all : 0u) ^ 0x80000000u;
   }
   if (MODE == OS_BWD_DOT || kGS) red_out[0] += red[0];
   if (kGS) red_out[1] += red[1];
