@@ -1086,7 +1086,7 @@ def run_gpu(args, rank, world, dist):
                 "inner_iterations": mi.itr_used, "outer_iterations": mi.outer_iterations, "inner_tol": inner_tol,
                 "max_rel_diff_vs_fp64": err}
 
-    if args.mixed_host_loop:  # profiling: the coloured inner kernels launched from the host
+    if args.mixed_host_loop:  # profiling: the coloured inner kernels launched from the host (more than two colours)
         ctx.set_tracing(True)
     mixed = mixed_run(fc.FC_PREC_MIXED_COLOURED, MIXED_INNER_TOL)
     ctx.set_tracing(False)
@@ -1174,7 +1174,8 @@ def main():
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--spmv-calls", type=int, default=20, help="timed fc_spmv calls on device arrays (0: skip)")
     ap.add_argument("--mixed-host-loop", action="store_true",
-                    help="launch the multicolour inner kernels from the host (visible to profilers)")
+                    help="launch the multicolour inner kernels of more than two colours from the host "
+                         "(visible to profilers)")
     ap.add_argument("--simple-n", type=int, default=64, help="cells per side of the SIMPLE cavity (0: skip)")
     ap.add_argument("--simple-big-n", type=int, default=128,
                     help="cells per side of the SIMPLE cavity on the perturbed mesh (0: skip)")

@@ -213,8 +213,8 @@ int fc_set_sweep_cap(fc_ctx* ctx, int rows);
 int fc_set_sweep_tiles(fc_ctx* ctx, int tiles);
 /* Sets the most rows of a sweep step in the pattern analyses that follow, as
  * far as that many fit the shared-memory staging (0 restores the default, one
- * row per compute thread); a level of a tile with more rows takes several
- * consecutive steps.  Results do not depend on it.  Tuning and testing only:
+ * row per compute thread; fewer where exchanged values fill the staging); a
+ * level of a tile with more rows takes several consecutive steps.  Results do not depend on it.  Tuning and testing only:
  * no counterpart in the reference. */
 int fc_set_sweep_stage_rows(fc_ctx* ctx, int rows);
 /* Appends one JSON line per solve to the file at path (NULL or "": stop):
@@ -279,9 +279,10 @@ int fc_batch_tune(fc_batch* b, const char* solver, const double* const* a, const
  * tile's SM), the start of the loads on the global timer, then the set's first
  * thread's loads issued, its release by the previous step, its value computed
  * and its stores issued (clock64).  With
- * tracing on, the multicolour inner solve of FC_PREC_MIXED_COLOURED launches
- * its kernels from the host instead of its CUDA graph, so that a profiler
- * sees each launch. */
+ * tracing on, the multicolour inner solve of FC_PREC_MIXED_COLOURED on more
+ * than two colours launches its kernels from the host instead of its CUDA
+ * graph, so that a profiler sees each launch (on two colours all iterations are
+ * one kernel, with tracing or without). */
 int fc_set_tracing(fc_ctx* ctx, int on);
 int fc_trace_get(fc_ctx* ctx, double* out, unsigned long long* timeline);
 /* ILU(0) factors of ilu_cr (linear_solvers.f90:1267-1385) in the CSR slots. */
