@@ -636,6 +636,8 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
     asm volatile("fence.proxy.async;" ::: "memory");
     const int ng = (ns + G - 1) >> gshift;
     const bool by_parity = import_by_parity(K, G);
+    // also where this sweep does not use its own word: the next one may be of
+    // another mode
     if (lane == 0) X.abort_flag[1 + ((X.parity >> 31) ^ 1u)] = 0;
     int issued = 0;
     bool ok = true;
@@ -684,7 +686,7 @@ __device__ __noinline__ bool osweep_tile(const GridCtl& C, const OrdView& O, con
           }
         }
         ok = __shfl_sync(0xffffffffu, (int)ok, j) != 0;
-        __syncwarp();  // the next lane's word comes after this one's
+        if (!by_parity) __syncwarp();  // the next lane's word comes after this one's
         issued += ok ? 1 : 0;
       }
     }
