@@ -4,7 +4,8 @@
 // plays the hand-over of K stage buffers of G steps between the stager, the
 // importers and the sets of compute warps (csrc/fc_sweep.cuh) in many random
 // orders, one actor or another held up for a while: barriers that are waited
-// for by parity, named barriers of the steps, copies that land late.  rule
+// for by parity, named barriers of the steps, copies that land late; then sweeps
+// of other modes (other K) on the same barriers and words.  rule
 // "code": the importers wait as fc_stage.hpp has it; "parity": always by the
 // parity of `empty`.  Reports buffers written before they were read, read
 // before they were written, named barriers arrived at twice and dead ends.
@@ -40,32 +41,42 @@ struct MBar {  // an mbarrier: completed phases, arrivals still missing
   bool passes(int parity) const { return (done & 1) != parity; }  // of the phase with this parity, or of the one before
 };
 
+struct Shared {  // what the sweeps of a kernel hand on
+  MBar empty[FC_MAX_STAGES], full[FC_MAX_STAGES];
+  unsigned parity = 0;  // bit b: of the next use of buffer b; bit 31: of the next sweep
+  int word[2] = {0, 0};
+  explicit Shared(int G) {
+    for (MBar& b : empty) b.init(G);
+    for (MBar& b : full) b.init(1);
+  }
+};
+
 struct Model {
+  Shared& sh;
   int K, G, ns, ng, ahead;
   bool parity_rule;
   std::mt19937& rng;
-  std::vector<MBar> empty, full;
+  MBar *empty, *full;
   std::vector<int> land;                  // buffers whose copy is under way: its group, else -1
   std::vector<int> copied, imported;      // group whose records / exchanged values a buffer holds
   std::vector<int> read, back;            // per group: steps that have read their values, given their buffer back
   std::vector<char> set_rel, imp_rel, passed;  // named barrier of step k
-  int word = 0;
+  bool cleared = false;
   int set_k[FC_SETS], set_at[FC_SETS], imp_g[FC_IMP_WARPS], imp_rel_k[FC_IMP_WARPS], stag_g = 0;
   bool imp_in[FC_IMP_WARPS];
   std::string bad;
 
-  Model(int K_, int G_, int ns_, bool parity_rule_, std::mt19937& r)
-      : K(K_), G(G_), ns(ns_), ng((ns_ + G_ - 1) / G_), ahead(import_ahead(K_, G_)), parity_rule(parity_rule_), rng(r),
-        empty(K_), full(K_), land(K_, -1), copied(K_, -1), imported(K_, -1), read(ng, 0), back(ng, 0),
+  Model(Shared& s, int K_, int G_, int ns_, bool parity_rule_, std::mt19937& r)
+      : sh(s), K(K_), G(G_), ns(ns_), ng((ns_ + G_ - 1) / G_), ahead(import_ahead(K_, G_)), parity_rule(parity_rule_), rng(r),
+        empty(s.empty), full(s.full), land(K_, -1), copied(K_, -1), imported(K_, -1), read(ng, 0), back(ng, 0),
         set_rel(ns_ + 1, 0), imp_rel(ns_, 0), passed(ns_, 0) {
-    for (MBar& b : empty) b.init(G);
-    for (MBar& b : full) b.init(1);
     for (int s = 0; s < FC_SETS; ++s) { set_k[s] = s; set_at[s] = 0; }
     for (int w = 0; w < FC_IMP_WARPS; ++w) { imp_g[w] = w; imp_in[w] = false; imp_rel_k[w] = 0; }
     set_rel[0] = 1;
   }
   int steps(int g) const { return std::min(G, ns - g * G); }
-  int par(int g) const { return (g / K) & 1; }
+  int par(int g) const { return (int)(((sh.parity >> (g % K)) ^ (unsigned)(g / K)) & 1u); }
+  int& word() { return sh.word[sh.parity >> 31]; }
   void fail(const char* what, int g) {
     if (bad.empty()) bad = std::string(what) + " (group " + std::to_string(g) + ")";
   }
@@ -108,7 +119,7 @@ struct Model {
       if (g >= ahead) {
         if (parity_rule || import_by_parity(K, G)) {
           if (!empty[(g - ahead) % K].passes(par(g - ahead))) return false;
-        } else if (word < g + 1) {
+        } else if (word() < g + 1) {
           return false;
         }
       }
@@ -127,10 +138,14 @@ struct Model {
   bool stager() {
     const int g = stag_g;
     if (g >= ng) return false;
+    if (!cleared) {
+      sh.word[(sh.parity >> 31) ^ 1u] = 0;
+      return cleared = true;
+    }
     const int b = g % K;
     if (g >= K && !empty[b].passes(par(g) ^ 1)) return false;
     if (g >= K && back[g - K] != steps(g - K)) fail("records copied over ones in use", g);
-    word = g + 1;
+    if (!import_by_parity(K, G)) word() = g + 1;
     copied[b] = -1;
     land[b] = g;
     if (steps(g) < G) empty[b].arrive(G - steps(g));
@@ -161,7 +176,11 @@ struct Model {
       idle = moved ? 0 : idle + 1;
       bool over = stag_g >= ng;
       for (int s = 0; s < FC_SETS; ++s) over = over && set_k[s] >= ns;
-      if (over) return true;
+      if (over) {
+        const unsigned first = (1u << (ng % K)) - 1u, all = (1u << K) - 1u;
+        sh.parity ^= first ^ ((ng / K) & 1 ? all : 0u) ^ 0x80000000u;
+        return true;
+      }
       if (idle > 400 * actors) fail("nobody can move", stag_g);
     }
     return false;
@@ -170,11 +189,16 @@ struct Model {
 
 int model(int K, int G, const std::string& rule) {
   std::mt19937 rng(1234);
-  for (int t = 0; t < 4000; ++t) {
-    Model m(K, G, 1 + (int)(rng() % 90), rule == "parity", rng);
-    if (!m.run()) {
-      std::printf("K %d G %d run %d: %s\n", K, G, t, m.bad.c_str());
-      return 1;
+  for (int t = 0; t < 2000; ++t) {
+    Shared sh(G);
+    const int sweeps = 1 + (int)(rng() % 4);
+    for (int s = 0; s < sweeps; ++s) {
+      const int Ks = s == 0 ? K : 4 << (rng() % 3);  // another mode
+      Model m(sh, Ks, G, 1 + (int)(rng() % 90), rule == "parity", rng);
+      if (!m.run()) {
+        std::printf("K %d G %d run %d sweep %d: %s\n", Ks, G, t, s, m.bad.c_str());
+        return 1;
+      }
     }
   }
   std::printf("OK\n");
